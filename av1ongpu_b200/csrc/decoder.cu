@@ -2364,13 +2364,11 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
      * side stream while the picture is reconstructed. The fork point orders
      * them after the previous frame's blend, which read the same state. */
     GrainState* gsd = static_cast<GrainState*>(d->grain_state.p);
-    const size_t tail = offsetof(GrainState, lut);
     CK(cudaEventRecord(d->ev_fork, st), "fork");
     CK(cudaStreamWaitEvent(d->aux, d->ev_fork, 0), "fork wait");
-    CK(cudaMemcpyAsync(reinterpret_cast<uint8_t*>(gsd) + tail, ar + pl->o_gs, sizeof(GrainState) - tail,
-                       cudaMemcpyDeviceToDevice, d->aux), "grain constants");
     CK(timed(d, kStGrainTemplate, [&] {
-         return launch_grain_template(gsd, P.gp, static_cast<const uint16_t*>(d->orbit.p),
+         return launch_grain_template(gsd, reinterpret_cast<const int*>(ar + pl->o_gs), P.gp,
+                                      static_cast<const uint16_t*>(d->orbit.p),
                                       static_cast<const uint16_t*>(d->pos.p), d->aux);
        }, d->aux), "film grain template");
     CK(cudaEventRecord(d->ev_join, d->aux), "join");

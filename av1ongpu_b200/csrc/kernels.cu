@@ -1567,83 +1567,150 @@ __global__ void __launch_bounds__(256) k_lr_tile(const px_t* __restrict__ cdef,
 /* ---- film grain ------------------------------------------------------------------------------- */
 
 /* Generates the three grain templates (7.18.3.3): Gaussian noise from the LFSR
- * (every draw independent through the orbit table), then the auto-regressive
- * filter as a wavefront: sample (x, y) depends on rows above within +-lag
- * columns and on the lag samples to its left, so t = x + 4y orders it
- * (lag <= 3). One block: the Gaussian fill on all its threads, the filters
- * of the three templates on its first warps, luma and chroma in the same
- * steps. */
+ * (every draw independent through the orbit table) on all threads of the
+ * block, then the auto-regressive filters, one warp a template: a sample
+ * reads the samples of its own row to its left and of the rows above within
+ * +-lag columns, so with row y starting LAG + 1 steps after row y - 1 every
+ * step has one sample of each row, and a warp holds the rows of one step in
+ * its lanes. */
 
-/* Luma rows the auto-regressive filter runs (3 .. 72 of the 82x73
- * template), a thread each. */
-constexpr int kGrainLumaRows = 70;
+/* The position stride of the templates in shared memory, all three planes. */
+#define AV1B_GRAIN_W 82
 
-/* The step by which the chroma wavefront trails the luma one: a chroma
- * sample (x, y) of step x + 4y + delay reads the luma samples it averages
- * (columns ((x - 3) << ss_x) + 3 .. + ss_x, rows likewise), whose own step
- * X + 4Y is at most delay - 1 before it; the lag grows with x (y) when
- * ss_x (ss_y) doubles the luma coordinate, largest at the template's last
- * column (row). */
-__host__ __device__ __forceinline__ int grain_chroma_delay(int ss_x, int ss_y, int cw, int ch) {
-  return (ss_x ? cw - 6 : 0) + 4 * (ss_y ? ch - 3 : 0) + 1;
-}
+/* One template's auto-regressive filter by one warp, LAG 2 or 3 (shorter
+ * lags run as LAG 2 with zero taps). Lane l takes rows l, l + 32, ..: at step
+ * t the row's column x = t - S y, S = LAG + 1 (a row is finished before the
+ * lane's next one starts: 82 columns and the lead-in of LAG are fewer than
+ * 32 S steps). The value above at column x + LAG, the newest one a sample
+ * reads, is the output of the lane below's step before, taken by shuffle;
+ * the rows further up were written at least LAG + 2 steps ago and come from
+ * shared memory, loaded a step ahead. Each arriving value is added, weighted,
+ * to the sums of the 2 LAG + 1 positions that read it; the sums rotate
+ * through registers, a block of 2 LAG + 1 steps unrolled so that their
+ * indexes are constants. What bounds it is the chain of one step - shuffle,
+ * multiply-add, round, clip - times 82 + S (rows - 1) steps; a thread a row
+ * with every tap a shared-memory read and a block barrier a step took 0.27 us
+ * a step (150 us a frame's templates). */
+template <int LAG, bool CHROMA>
+struct GrainWave {
+  static constexpr int R = 2 * LAG + 1, S = LAG + 1;
+  int co[LAG + 1][R];        /* taps by rows up, then column; row 0: the left ones */
+  int luma_co;
+  int acc[R];
+  int x, y, prev;
+  int noise, up2, up3;       /* of the coming step, loaded ahead */
 
-/* The auto-regressive filters of the three templates (7.18.3.3) with lag
- * LAG, by wavefront: sample (x, y) reads the LAG rows above within +-LAG
- * columns and the LAG samples to its left, so the steps t = x + 4y order
- * it, and the samples of one step are independent. Thread tid <
- * kGrainLumaRows takes luma row 3 + tid; thread kGrainLumaRows + i takes
- * chroma item i (plane i & 1, row i >> 1), its wavefront `delay` steps
- * behind (grain_chroma_delay) so that every luma sample it reads is final.
- * All `nthreads` threads (a multiple of 32) meet a named barrier after each
- * step. */
+  __device__ __forceinline__ void taps(const int* c, int lag, int lane) {
+#pragma unroll
+    for (int dr = 0; dr <= LAG; ++dr)
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const int dc = k - LAG;
+        const bool in = dr <= lag && dc >= -lag && dc <= lag && (dr > 0 || dc < 0);
+        co[dr][k] = in ? c[(lag - dr) * (2 * lag + 1) + dc + lag] : 0;
+      }
+    luma_co = CHROMA ? c[2 * lag * (lag + 1)] : 0;
+#pragma unroll
+    for (int k = 0; k < R; ++k) acc[k] = 0;
+    y = lane;
+    x = -3 - S * lane;
+    prev = noise = up2 = up3 = 0;
+  }
+
+  /* Template entry (row, col) or, outside the template, any entry: those only
+   * reach positions that keep their noise. */
+  static __device__ __forceinline__ int at(const short* t, int row, int col) {
+    return t[maxi(0, mini(row * AV1B_GRAIN_W + col, AV1B_GRAIN_W * 73 - 1))];
+  }
+
+  /* R steps. gw x gh: the template; luma: its luma template when the chroma
+   * filter reads it. */
+  __device__ __forceinline__ void steps(short* tmpl, int gw, int gh, const short* luma, int sx, int sy,
+                                        int arshift, int gmin, int gmax, int lane) {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int above = __shfl_sync(0xffffffffu, prev, (lane + 31) & 31);
+      int base = acc[q] + ((noise * 2 + 1) << (arshift - 1));
+      if (CHROMA && luma) {
+        const int lx = mini(maxi(((x - 3) << sx) + 3, 0), AV1B_GRAIN_W - 1 - sx);
+        const int ly = mini(maxi(((y - 3) << sy) + 3, 0), 72 - sy);
+        const short* lp = luma + ly * AV1B_GRAIN_W + lx;
+        int v = lp[0];
+        if (sx) v += lp[1];
+        if (sy) v += lp[AV1B_GRAIN_W] + (sx ? lp[AV1B_GRAIN_W + 1] : 0);
+        base += rnd2z(v, sx + sy) * luma_co;
+      }
+      /* this step's sum first: the older rows, the left neighbour, and last
+       * the neighbour above, whose shuffle is the longest wait */
+      base += up2 * co[2][R - 1 - 0] + prev * co[0][LAG - 1];
+      if (LAG == 3) base += up3 * co[LAG][R - 1];
+      const int sum = base + above * co[1][R - 1];
+      const bool keep = x < 3 || x >= gw - 3 || y < 3;
+      const int out = keep ? noise : clampi(sum >> arshift, gmin, gmax);
+      if (!keep && y < gh) tmpl[y * AV1B_GRAIN_W + x] = static_cast<short>(out);
+      /* the positions after this one that read the same values */
+#pragma unroll
+      for (int k = 1; k < R; ++k) {
+        int v = above * co[1][R - 1 - k] + up2 * co[2][R - 1 - k];
+        if (LAG == 3) v += up3 * co[LAG][R - 1 - k];
+        if (k < LAG) v += prev * co[0][LAG - 1 - k];
+        acc[(q + k) % R] += v;
+      }
+      acc[q] = 0;
+      prev = out;
+      if (++x == gw) {
+        x -= 32 * S;
+        y += 32;
+      }
+      noise = at(tmpl, y, x);
+      up2 = at(tmpl, y - 2, x + LAG);
+      if (LAG == 3) up3 = at(tmpl, y - 3, x + LAG);
+      __syncwarp();
+    }
+  }
+};
+
+/* The auto-regressive filters of the three templates (7.18.3.3) by warps 0
+ * (luma), 1 and 2 (chroma) of the block; `tid` < 96. Chroma trails luma: in
+ * iteration k, between two barriers of the three warps, luma runs its steps
+ * 2R k .. 2R (k + 1) - 1 and chroma, from k = 1 on, R (k - 1) .. R k - 1 where
+ * chroma is subsampled (its sample of step s reads luma of step 2s - 5 at
+ * most), 2R (k - 1) .. 2R k - 1 where it is not (step s). */
 template <int LAG>
-__device__ void grain_ar(const GrainParamsDev& prm, short* luma, short* cb, short* cr, int cw, int ch,
-                         bool chroma, int arshift, int gmin, int gmax, int tid, int nthreads) {
-  constexpr int NT = 2 * LAG * (LAG + 1);   /* taps before the sample itself */
-  constexpr int W = 82, H = 73;
+__device__ __forceinline__ void grain_ar(const GrainParamsDev& prm, short* luma, short* cb, short* cr,
+                                         int cw, int ch, bool chroma, int arshift, int gmin, int gmax,
+                                         int tid) {
+  constexpr int R = 2 * LAG + 1, S = LAG + 1;
+  const int warp = tid >> 5, lane = tid & 31, lag = prm.ar_coeff_lag;
   const bool do_luma = prm.num_y_points > 0;
   const int sx = prm.ss_x, sy = prm.ss_y;
-  const int delay = chroma && do_luma ? grain_chroma_delay(sx, sy, cw, ch) : 0;
-  const bool luma_thread = tid < kGrainLumaRows;
-  const int ci = tid - kGrainLumaRows;
-  const int plane = ci & 1;
-  /* this thread's row of its template, and its work */
-  const int y = luma_thread ? 3 + tid : ci >> 1;
-  const bool mine = luma_thread ? do_luma : (chroma && ci >= 0 && ci < 2 * ch && y >= 3);
-  short* gp = luma_thread ? luma : (plane ? cr : cb);
-  const int gw = luma_thread ? W : cw;
-  const int off = luma_thread ? 0 : delay;
-  int co[NT + 1];
-  {
-    const int* cp = luma_thread ? prm.ar_y : (plane ? prm.ar_cr : prm.ar_cb);
-#pragma unroll
-    for (int i = 0; i <= NT; ++i) co[i] = (luma_thread && i == NT) ? 0 : cp[i];
-  }
-  const int tl = do_luma ? (W - 4) + 4 * (H - 1) : 0;
-  const int tc = chroma ? (cw - 4) + 4 * (ch - 1) + delay : 0;
-  const int tmax = tl > tc ? tl : tc;
-  for (int t = 3 + 4 * 3; t <= tmax; ++t) {
-    const int x = t - off - 4 * y;
-    if (mine && x >= 3 && x < gw - 3) {
-      int sum = 0, k = 0;
-#pragma unroll
-      for (int dr = -LAG; dr <= 0; ++dr)
-#pragma unroll
-        for (int dc = -LAG; dc <= LAG; ++dc) {
-          if (dr == 0 && dc == 0) break;
-          sum += gp[(y + dr) * gw + x + dc] * co[k++];
-        }
-      if (!luma_thread && do_luma) {
-        const int lx = ((x - 3) << sx) + 3, ly = ((y - 3) << sy) + 3;
-        int acc = 0;
-        for (int i = 0; i <= sy; ++i)
-          for (int j = 0; j <= sx; ++j) acc += luma[(ly + i) * W + lx + j];
-        sum += rnd2z(acc, sx + sy) * co[NT];
+  const int per = sx || sy ? 1 : 2;   /* chroma's blocks of R steps an iteration */
+  const int luma_it = do_luma ? (3 + AV1B_GRAIN_W + S * 72 + 2 * R - 1) / (2 * R) : 0;
+  const int chroma_it = chroma ? (3 + cw + S * (ch - 1) + per * R - 1) / (per * R) + 1 : 0;
+  const int its = maxi(luma_it, chroma_it);
+  if (warp == 0) {
+    GrainWave<LAG, false> w;
+    w.taps(prm.ar_y, lag, lane);
+    for (int k = 0; k < its; ++k) {
+      if (k < luma_it) {
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r)
+          w.steps(luma, AV1B_GRAIN_W, 73, nullptr, 0, 0, arshift, gmin, gmax, lane);
       }
-      gp[y * gw + x] = (short)clampi(gp[y * gw + x] + rnd2z(sum, arshift), gmin, gmax);
+      if (chroma) asm volatile("bar.sync 1, 96;" ::: "memory");
     }
-    asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+  } else if (chroma) {
+    GrainWave<LAG, true> w;
+    short* t = warp == 1 ? cb : cr;
+    w.taps(warp == 1 ? prm.ar_cb : prm.ar_cr, lag, lane);
+    for (int k = 0; k < its; ++k) {
+      if (k >= 1 && k < chroma_it) {
+#pragma unroll 1
+        for (int r = 0; r < per; ++r)
+          w.steps(t, cw, ch, do_luma ? luma : nullptr, sx, sy, arshift, gmin, gmax, lane);
+      }
+      asm volatile("bar.sync 1, 96;" ::: "memory");
+    }
   }
 }
 
@@ -1654,11 +1721,19 @@ struct GrainTemplateSmem {
   short luma[82 * 73], cb[82 * 73], cr[82 * 73];
 };
 
-/* Every thread of the CTA runs it (the filters on its first five warps);
+/* Every thread of the CTA runs it (the filters on its first three warps);
  * it has no early return. */
-__device__ __forceinline__ void grain_template_body(GrainState* gs, const GrainParamsDev& prm,
-                                                    const uint16_t* orbit, const uint16_t* pos,
-                                                    GrainTemplateSmem& sm) {
+__device__ __forceinline__ void grain_template_body(GrainState* gs, const int* gs_src,
+                                                    const GrainParamsDev& prm, const uint16_t* orbit,
+                                                    const uint16_t* pos, GrainTemplateSmem& sm) {
+  /* the frame's grain constants and scaling tables, from its plan (null: in
+   * place already) */
+  if (gs_src) {
+    constexpr int tail = static_cast<int>(offsetof(GrainState, lut));
+    constexpr int words = static_cast<int>((sizeof(GrainState) - tail) / 4);
+    int* dst = reinterpret_cast<int*>(reinterpret_cast<char*>(gs) + tail);
+    for (int k = threadIdx.x; k < words; k += blockDim.x) dst[k] = gs_src[k];
+  }
   short* s_luma = sm.luma;
   short* s_cb = sm.cb;
   short* s_cr = sm.cr;
@@ -1666,60 +1741,58 @@ __device__ __forceinline__ void grain_template_body(GrainState* gs, const GrainP
   const int bd = prm.bitdepth;
   const int shift = 12 - bd + prm.grain_scale_shift;
   const int gmin = -(128 << (bd - 8)), gmax = (256 << (bd - 8)) - 1 - (128 << (bd - 8));
-  const int cw = gs->chroma_w, ch = gs->chroma_h;
+  const int cw = prm.ss_x ? 44 : AV1B_GRAIN_W, ch = prm.ss_y ? 38 : 73;
   short* luma = s_luma;
   short* cb = s_cb;
   short* cr = s_cr;
-  /* Gaussian fill */
-  for (int k = tid; k < 82 * 73; k += blockDim.x) {
-    int g = 0;
-    if (prm.num_y_points > 0) {
-      const int st = lfsr_after(orbit, pos, (unsigned)prm.seed & 0xffffu, k + 1);
-      g = kGaussianSequence[(st >> 5) & 2047];
-    }
-    luma[k] = (short)rnd2z(g, shift);
+  /* Gaussian fill: draw k is the LFSR's state k + 1 steps after its seed */
+  const auto draw = [&](unsigned seed, unsigned first, int k) {
+    const int st = seed ? orbit[(first + static_cast<unsigned>(k) + 1u) % 65535u] : 0;
+    return rnd2z(kGaussianSequence[(st >> 5) & 2047], shift);
+  };
+  {
+    const bool on = prm.num_y_points > 0;
+    const unsigned seed = (unsigned)prm.seed & 0xffffu, first = pos[seed];
+#pragma unroll 8
+    for (int k = tid; k < 82 * 73; k += blockDim.x)
+      luma[k] = static_cast<short>(on ? draw(seed, first, k) : 0);
   }
   const bool chroma = prm.chroma_scaling_from_luma || prm.num_cb_points > 0 || prm.num_cr_points > 0;
   if (chroma) {
     const bool acb = prm.num_cb_points > 0 || prm.chroma_scaling_from_luma;
     const bool acr = prm.num_cr_points > 0 || prm.chroma_scaling_from_luma;
+    const unsigned sb = ((unsigned)prm.seed ^ 0xb524u) & 0xffffu, sr = ((unsigned)prm.seed ^ 0x49d8u) & 0xffffu;
+    const unsigned fb = pos[sb], fr = pos[sr];
+#pragma unroll 4
     for (int k = tid; k < cw * ch; k += blockDim.x) {
-      int g0 = 0, g1 = 0;
-      if (acb) g0 = kGaussianSequence[(lfsr_after(orbit, pos, ((unsigned)prm.seed ^ 0xb524u) & 0xffffu, k + 1) >> 5) & 2047];
-      if (acr) g1 = kGaussianSequence[(lfsr_after(orbit, pos, ((unsigned)prm.seed ^ 0x49d8u) & 0xffffu, k + 1) >> 5) & 2047];
-      cb[k] = (short)rnd2z(g0, shift);
-      cr[k] = (short)rnd2z(g1, shift);
+      const int y = k / cw, o = y * AV1B_GRAIN_W + k - y * cw;
+      cb[o] = static_cast<short>(acb ? draw(sb, fb, k) : 0);
+      cr[o] = static_cast<short>(acr ? draw(sr, fr, k) : 0);
     }
   }
   __syncthreads();
   const int arshift = prm.ar_coeff_shift_minus_6 + 6;
-  /* the auto-regressive filters on the first warps (a step of a wavefront
-   * has at most 70 luma and 146 chroma samples, one a thread: 96 threads for
-   * luma alone, up to 224 with chroma), a named barrier between steps; the
-   * lag as a constant, so a sample's taps are independent loads */
-  const int ar_threads = ((kGrainLumaRows + (chroma ? 2 * ch : 0)) + 31) & ~31;
-  if (tid < ar_threads) {
-    switch (prm.ar_coeff_lag) {
-      case 0: grain_ar<0>(prm, luma, cb, cr, cw, ch, chroma, arshift, gmin, gmax, tid, ar_threads); break;
-      case 1: grain_ar<1>(prm, luma, cb, cr, cw, ch, chroma, arshift, gmin, gmax, tid, ar_threads); break;
-      case 2: grain_ar<2>(prm, luma, cb, cr, cw, ch, chroma, arshift, gmin, gmax, tid, ar_threads); break;
-      default: grain_ar<3>(prm, luma, cb, cr, cw, ch, chroma, arshift, gmin, gmax, tid, ar_threads); break;
-    }
+  if (tid < 96) {
+    if (prm.ar_coeff_lag >= 3)
+      grain_ar<3>(prm, luma, cb, cr, cw, ch, chroma, arshift, gmin, gmax, tid);
+    else
+      grain_ar<2>(prm, luma, cb, cr, cw, ch, chroma, arshift, gmin, gmax, tid);
   }
   __syncthreads();
   for (int k = tid; k < 82 * 73; k += blockDim.x) gs->luma[k] = luma[k];
   if (chroma)
     for (int k = tid; k < cw * ch; k += blockDim.x) {
-      gs->cb[k] = cb[k];
-      gs->cr[k] = cr[k];
+      const int y = k / cw, o = y * AV1B_GRAIN_W + k - y * cw;
+      gs->cb[k] = cb[o];
+      gs->cr[k] = cr[o];
     }
 }
 
-__global__ void __launch_bounds__(256) k_grain_template(GrainState* gs, GrainParamsDev prm,
-                                                        const uint16_t* orbit,
-                                                        const uint16_t* pos) {
+__global__ void __launch_bounds__(256) k_grain_template(GrainState* gs, const int* gs_src,
+                                                        const __grid_constant__ GrainParamsDev prm,
+                                                        const uint16_t* orbit, const uint16_t* pos) {
   __shared__ GrainTemplateSmem sm;
-  grain_template_body(gs, prm, orbit, pos, sm);
+  grain_template_body(gs, gs_src, prm, orbit, pos, sm);
 }
 
 /* The stripe values of plane `p` (7.18.3.5, the horizontal half: the grain
@@ -2217,9 +2290,9 @@ cudaError_t launch_lr(const px_t* cdef, const px_t* curr, px_t* dst, const Layou
   return cudaGetLastError();
 }
 
-cudaError_t launch_grain_template(GrainState* gs, const GrainParamsDev& prm, const uint16_t* orbit,
-                                  const uint16_t* pos, cudaStream_t s) {
-  k_grain_template<<<1, 256, 0, s>>>(gs, prm, orbit, pos);
+cudaError_t launch_grain_template(GrainState* gs, const int* gs_src, const GrainParamsDev& prm,
+                                  const uint16_t* orbit, const uint16_t* pos, cudaStream_t s) {
+  k_grain_template<<<1, 256, 0, s>>>(gs, gs_src, prm, orbit, pos);
   return cudaGetLastError();
 }
 

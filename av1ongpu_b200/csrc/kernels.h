@@ -138,8 +138,10 @@ cudaError_t launch_upscale(const px_t* src, px_t* dst, const Layout& L, int maxv
                            cudaStream_t s);
 cudaError_t launch_lr(const px_t* cdef, const px_t* curr, px_t* dst, const Layout& L,
                       const LrArgs& r, int maxv, bool copy_rest, cudaStream_t s);
-cudaError_t launch_grain_template(GrainState* gs, const GrainParamsDev& prm, const uint16_t* orbit,
-                                  const uint16_t* pos, cudaStream_t s);
+/* gs_src: the frame's grain constants (GrainState from `lut` on), copied into
+ * `gs` beside the templates; null: `gs` holds them. */
+cudaError_t launch_grain_template(GrainState* gs, const int* gs_src, const GrainParamsDev& prm,
+                                  const uint16_t* orbit, const uint16_t* pos, cudaStream_t s);
 cudaError_t launch_grain_blend(const px_t* src, px_t* dst, const Layout& L, const GrainState* gs,
                                const uint16_t* orbit, const uint16_t* pos, cudaStream_t s);
 cudaError_t launch_nv12(const px_t* pic, uint8_t* out, const Layout& L, int pitch, cudaStream_t s);
