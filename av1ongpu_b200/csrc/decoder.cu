@@ -134,8 +134,9 @@ struct av1b_decoder {
   bool have_last = false;
 
   /* per-frame buffers */
-  DevBuf arena, coef, residual, done, status_q, nv12, rgb;
+  DevBuf arena, coef, residual, done, tags, status_q, nv12, rgb;
   unsigned epoch = 0;
+  unsigned tag = 0;               /* the tag of the last frame's samples, 1 .. 65535 */
 
   /* film grain */
   DevBuf grain_state, orbit, pos;
@@ -888,6 +889,8 @@ struct PlanScratch {
   std::vector<uint64_t> head_key;
   std::vector<int> units_coding, ui_of, udepth, udeps;
   std::vector<uint8_t> is_b;
+  std::vector<uint8_t> flagged;       /* blocks some block waits on by done flag */
+  bool on_grid = false;               /* every block lies on its plane's owner cells */
   std::vector<uint16_t> itx_key;
   std::vector<int> itx_hist;
   std::vector<int2> itx_unsorted;  /* the blocks' transform jobs, before plan_itx sorts them */
@@ -959,6 +962,28 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
         }
     }
   };
+  /* each_cell over one row or one column of cells, for block bi: also the
+   * mask of the cells (bit k: the k-th from (x0, y0)'s, at most 64 of them)
+   * whose owners are phase B blocks before it - the ones it waits for */
+  auto edge_cells = [&](int p, int x0, int x1, int y0, int y1, int bi, auto&& f) {
+    const int s = sh[p], w = cw[p];
+    const int cx0 = std::max(x0 >> s, 0), cx1 = std::min(x1 >> s, w - 1);
+    const int cy0 = std::max(y0 >> s, 0), cy1 = std::min(y1 >> s, ch[p] - 1);
+    const int* o = S.owner[p].data();
+    int last = -1, k = 0;
+    uint64_t mask = 0, in = 0;
+    for (int cy = cy0; cy <= cy1; ++cy)
+      for (int cx = cx0; cx <= cx1; ++cx, ++k) {
+        const int own = o[static_cast<size_t>(cy) * w + cx];
+        if (own != last) {
+          last = own;
+          in = own >= 0 && own < bi && is_b[own] ? 1 : 0;
+          f(own);
+        }
+        if (k < 64) mask |= in << k;
+      }
+    return mask;
+  };
   static const int kAngle[9] = {0, 90, 180, 45, 135, 113, 157, 203, 67};
   const size_t nu = P->R->units.size();
   const int pieces = pieces_for(nu, c, 256);
@@ -969,6 +994,8 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
   std::vector<int>& ui_of = S.ui_of;  /* a phase B block's unit index */
   ui_of.resize(nb);
   std::vector<uint8_t> inter_piece(pieces, 0);
+  S.flagged.assign(nb, 0);
+  uint8_t* flagged = S.flagged.data();
   c.pool->run(pieces, [&](int pi) {
     std::vector<int>& out = pdeps[pi];
     out.clear();
@@ -1015,9 +1042,20 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
           above_x1 = b.x - 1;
           left_y1 = b.y - 1;
         }
-        if (left_y1 >= (b.y & ~(oc - 1))) each_cell(p, b.x - 1, b.x - 1, b.y, left_y1, wait_on);
-        if (above_x1 >= (b.x & ~(oc - 1))) each_cell(p, b.x, above_x1, b.y - 1, b.y - 1, wait_on);
-        if (above_x1 >= b.x || left_y1 >= b.y) each_cell(p, b.x - 1, b.x - 1, b.y - 1, b.y - 1, wait_on);
+        const uint64_t left_cells =
+            left_y1 >= (b.y & ~(oc - 1)) ? edge_cells(p, b.x - 1, b.x - 1, b.y, left_y1, bi, wait_on) : 0;
+        const uint64_t above_cells =
+            above_x1 >= (b.x & ~(oc - 1)) ? edge_cells(p, b.x, above_x1, b.y - 1, b.y - 1, bi, wait_on) : 0;
+        const uint64_t corner = above_x1 >= b.x || left_y1 >= b.y
+                                    ? edge_cells(p, b.x - 1, b.x - 1, b.y - 1, b.y - 1, bi, wait_on)
+                                    : 0;
+        if (b.kind == AV1B_U_INTRA && S.on_grid) {
+          b.sync = static_cast<unsigned char>(AV1B_SYNC_TAGS | (corner ? AV1B_SYNC_CORNER : 0));
+          b.wait_cells[0][0] = static_cast<unsigned>(above_cells);
+          b.wait_cells[0][1] = static_cast<unsigned>(above_cells >> 32);
+          b.wait_cells[1][0] = static_cast<unsigned>(left_cells);
+          b.wait_cells[1][1] = static_cast<unsigned>(left_cells >> 32);
+        }
       }
       if (b.kind == AV1B_U_INTRABC) {
         const int sx_ = p > 0 ? L.ss_x : 0, sy_ = p > 0 ? L.ss_y : 0;
@@ -1027,9 +1065,23 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
         if (x1 > std::max(sx, 0) && y1 > std::max(sy, 0))
           each_cell(p, std::max(sx, 0), x1 - 1, std::max(sy, 0), y1 - 1, wait_on);
       }
-      if (b.kind == AV1B_U_INTRA && b.mode == 13 && !b.palette)
+      if (b.kind == AV1B_U_INTRA && b.mode == 13 && !b.palette) {
+        /* by their tags only where every luma sample is of a block waited
+         * for: another's would never be tagged */
+        const int lx1 = (b.x + b.w) << L.ss_x, ly1 = (b.y + b.h) << L.ss_y;
+        bool all = lx1 <= L.p[0].grid_w && ly1 <= L.p[0].grid_h && b.w * b.h <= 1024;
         each_cell(0, b.x << L.ss_x, (b.x + b.w - 1) << L.ss_x, b.y << L.ss_y,
                   (b.y + b.h - 1) << L.ss_y, wait_on);
+        for (int cy = (b.y << L.ss_y) >> 2; all && cy < (ly1 + 3) >> 2; ++cy)
+          for (int cx = (b.x << L.ss_x) >> 2; cx < (lx1 + 3) >> 2; ++cx) {
+            const int o = S.owner[0][static_cast<size_t>(cy) * cw[0] + cx];
+            all = all && o >= 0 && o < bi && is_b[o];
+          }
+        if (all && b.sync)
+          b.sync |= AV1B_SYNC_LUMA;
+        else
+          b.sync = 0;
+      }
       if (mine.size() > 24) {
         std::sort(mine.begin(), mine.end());
       } else {
@@ -1037,6 +1089,8 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
           for (size_t y = x; y > 0 && mine[y - 1] > mine[y]; --y) std::swap(mine[y - 1], mine[y]);
       }
       mine.erase(std::unique(mine.begin(), mine.end()), mine.end());
+      if (!(b.sync & AV1B_SYNC_TAGS))
+        for (int o : mine) __atomic_store_n(flagged + o, uint8_t(1), __ATOMIC_RELAXED);
       /* prediction and residual fuse when the transforms cover disjoint parts
        * of the block (each sample then gets at most one residual) */
       b.fuse_res = 0;
@@ -1108,6 +1162,7 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
       BlockRec& b = P->R->blocks[P->R->units[ui]];
       b.dep_first = static_cast<int>(first[ui]);
       b.dep_count = dep_count[ui];
+      if (flagged[P->R->units[ui]]) b.sync |= AV1B_SYNC_FLAG;
     }
   });
   /* chains: a warp claims a chain and runs its blocks in order, so a block
@@ -1499,11 +1554,13 @@ int build_plan(av1b_decoder* d, const PlanCtx& c, const av1b_frame_syntax& s, Pl
       if (outs[i].err.code) return fail(d, outs[i].err.code, outs[i].err.msg);
     /* later blocks overwrite earlier ones where cells overlap: a plane whose
      * blocks are not all on the cell grid is filled again, in coding order */
+    S.on_grid = true;
     for (int p = 0; p < 3; ++p) {
       bool aligned = true;
       for (int i = 0; i < pieces; ++i)
         if (outs[i].unaligned[p]) aligned = false;
       if (aligned) continue;
+      S.on_grid = false;
       std::fill(S.owner[p].begin(), S.owner[p].end(), -1);
       const int oc = 1 << cell[p];
       int* o = S.owner[p].data();
@@ -2280,6 +2337,29 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
     CK(cudaMemsetAsync(d->done.p, 0, d->done.cap, st), "done reset");
     d->epoch = 1;
   }
+  /* the tagged samples of phase B; a frame that cannot have them (no memory)
+   * or is traced (a trace follows the done flags) waits on done flags */
+  a.tags = nullptr;
+  if (P.n_units && !d->tracing) {
+    size_t words = 0;
+    for (int p = 0; p < 3; ++p) {
+      a.tag_off[p] = static_cast<int>(words);
+      words += static_cast<size_t>(L.p[p].grid_w) * L.p[p].grid_h;
+    }
+    const size_t bytes = words * sizeof(unsigned);
+    const bool grow = d->tags.cap < bytes;
+    if (dev_ensure(d, d->tags, bytes)) {
+      clear_err(d);
+      cudaGetLastError();
+    } else {
+      if (grow || d->tag == 65535) {
+        CK(cudaMemsetAsync(d->tags.p, 0, d->tags.cap, st), "tag reset");
+        d->tag = 0;
+      }
+      a.tags = static_cast<unsigned*>(d->tags.p);
+      a.tag = ++d->tag << 16;
+    }
+  }
   if (!d->status_q.p) {
     if ((rc = dev_ensure(d, d->status_q, 256))) return rc;
     CK(cudaMemsetAsync(d->status_q.p, 0, 256, st), "status reset");
@@ -2769,7 +2849,7 @@ int av1b_decoder_destroy(av1b_decoder* d) {
   d->packs.clear();
   if (d->copy_stream) cudaStreamDestroy(d->copy_stream);
   DevBuf* bufs[] = {&d->cur, &d->snap, &d->lr_pre_up, &d->lr_cdef, &d->disp,
-                    &d->slot_ptr_dev, &d->arena, &d->coef, &d->residual, &d->done,
+                    &d->slot_ptr_dev, &d->arena, &d->coef, &d->residual, &d->done, &d->tags,
                     &d->status_q, &d->nv12, &d->rgb,
                     &d->grain_state, &d->orbit, &d->pos, &d->cdef_search, &d->pre_res, &d->mask_pool,
                     &d->trace};
@@ -2903,8 +2983,9 @@ size_t av1b_stream_hbm_estimate(int width, int height, int coded_width, int bit_
   auto rounded = [](size_t b) { return align_up(b + b / 8, size_t(1) << 16); };
   /* pictures: the one reconstructed, the snapshot, the display picture, the
    * two loop restoration sources, and the reference slots; per sample: the
-   * phase B residuals (4 B), the done flags (128 B a block, blocks of 16
-   * samples or more) and the difference-weighted luma masks (1 B); per plan:
+   * phase B residuals (4 B), the done flags (32 B a block, blocks of 16
+   * samples or more) with the tagged samples (4 B; 8 B in all is more than
+   * both) and the difference-weighted luma masks (1 B); per plan:
    * its five buffers - records, coefficient pool, residuals, levels, filter
    * lists - at most 10 B a coded sample in all; the grain tables and small
    * buffers, 2 MB */

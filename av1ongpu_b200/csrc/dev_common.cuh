@@ -130,7 +130,13 @@ struct BlockRec {
   int tx_first, tx_count;
   /* inter */
   int ref_slot[2];            /* device slot, -1: the picture being decoded */
-  int mv[2][2];
+  union {
+    int mv[2][2];
+    /* an intra block: which owner cells of its above row and of its left
+     * column, from the block's own column and row on, belong to blocks it
+     * waits for (bit k: the k-th cell; low word, high word) */
+    unsigned wait_cells[2][2];
+  };
   unsigned char filt, filt_v, compound, mask_kind;   /* compound: 0 none 1 avg 2 dist; mask 0/1 wedge/2 diffwtd */
   unsigned char w0, w1, mask_sign, ii_mode;
   unsigned char interintra, ii_wedge, wedge_dir, wedge_flip;
@@ -148,8 +154,19 @@ struct BlockRec {
    * reads that mask instead of predicting the luma itself; 0 - neither */
   int mask_off;
   short mask_w;
-  unsigned char mask_role, pad_mask;
+  unsigned char mask_role;
+  unsigned char sync;         /* AV1B_SYNC_* (phase B) */
 };
+
+/* How a phase B block waits and publishes: it waits on the tagged samples it
+ * reads (otherwise on done flags), the corner above left of it among them;
+ * its chroma-from-luma samples all belong to blocks it waits for, inside the
+ * grid, and are waited on by their tags as well; some block waits on its done
+ * flag. */
+#define AV1B_SYNC_TAGS 1
+#define AV1B_SYNC_CORNER 2
+#define AV1B_SYNC_LUMA 4
+#define AV1B_SYNC_FLAG 8
 
 /* One coded transform of a frame whose coefficients arrive as coded levels:
  * where its raster goes in the coefficient pool, where its levels start, and

@@ -26,6 +26,64 @@ namespace av1b {
 #define AV1B_EDGE_LEN 288
 #define AV1B_EDGE_OFF 16
 
+/* The tagged samples a block reads and writes (FrameArgs::tags): words at its
+ * top-left sample and the luma plane's origin, with the words a row; null
+ * `write`: untagged. `wait`: the edges are read by their tags, the cells (of
+ * 1 << cell samples) of `cells` only - the others are final already; `luma`:
+ * so are the chroma-from-luma samples. Waits give up after limit_ns or once
+ * one has given up (AV1B_STATUS_TIMEOUT, bit 0 of *status). */
+struct TagIo {
+  unsigned* write;
+  const unsigned* at;
+  const unsigned* luma_at;
+  int stride, luma_stride;
+  unsigned tag;               /* in the high half */
+  bool wait, luma, corner;
+  int cell;
+  unsigned long long above, left;
+  int clip_w, clip_h;         /* the block's samples inside the grid */
+  int* status;
+  unsigned long long limit_ns;
+};
+
+__device__ __forceinline__ unsigned ld_tag(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_tag(unsigned* p, unsigned v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+/* Between two rounds of loads of a warp whose samples have not all arrived:
+ * a pause that backs off to 128 ns; every 16th round the status word and the
+ * clock. Returns false when the wait has given up (the same for every lane). */
+struct TagBackoff {
+  unsigned it = 0, pause = 0;
+  unsigned long long t0 = 0;
+  __device__ __forceinline__ bool next(const TagIo& g, int lane) {
+    ++it;
+    if ((it & 15) == 0) {
+      int give_up = 0;
+      if (lane == 0) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (t0 == 0) t0 = now;
+        if (ld_tag(reinterpret_cast<const unsigned*>(g.status)) & 1u) {
+          give_up = 1;
+        } else if (now - t0 > g.limit_ns) {
+          atomicOr(g.status, 1);
+          give_up = 1;
+        }
+      }
+      if (__shfl_sync(0xffffffffu, give_up, 0)) return false;
+    }
+    if (pause) __nanosleep(pause);
+    if (it >= 4) pause = pause < 128 ? (pause ? pause << 1 : 16) : 128;
+    return true;
+  }
+};
+
 /* Everything the intra predictor needs for one block, resolved. */
 struct IntraJob {
   int x, y, w, h;
@@ -82,10 +140,96 @@ AV1B_DEV int upsample_sel(int w, int h, int filter_type, int delta) {
   return filter_type == 0 ? (w + h <= 16) : (w + h <= 8);
 }
 
+/* The gather below for a block that waits on the samples themselves: a
+ * sample of a block it waits for is loaded with its tag until the tag is this
+ * frame's, any other from the picture. The wait and the read are one round
+ * trip; with done flags they were a poll, then the loads, and on the writing
+ * side a fence before the flag. */
+AV1B_DEV void intra_edges_tagged(const IntraJob& j, const px_t* p, int stride, int* above, int* left,
+                                 const TagIo& g, int lane) {
+  const int n = j.w + j.h;
+  const int mid = 1 << (j.bitdepth - 1);
+  const int alimit = mini(j.max_x, j.x + (j.have_ar ? 2 * j.w : j.w) - 1);
+  const int llimit = mini(j.max_y, j.y + (j.have_bl ? 2 * j.h : j.h) - 1);
+  /* entries 2q: above, 2q + 1: left, of sample lane + 32 q; 8: the corner */
+  int v[9], o[9];
+  unsigned pend = 0;
+  auto want = [&](int e, bool have, int dy, int dx, bool tagged, int none) {
+    v[e] = none;
+    o[e] = 0;
+    if (!have) return;
+    if (tagged) {
+      o[e] = dy * g.stride + dx;
+      pend |= 1u << e;
+    } else {
+      v[e] = ldpx(p + dy * stride + dx);
+    }
+  };
+  const bool above0 = g.above & 1, left0 = g.left & 1;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    v[2 * q] = v[2 * q + 1] = o[2 * q] = o[2 * q + 1] = 0;
+    const int i = lane + 32 * q;
+    if (i < n) {
+      if (j.have_above) {
+        const int k = mini(j.x + i, alimit) - j.x;
+        want(2 * q, true, -1, k, (g.above >> (k >> g.cell)) & 1, 0);
+      } else {
+        want(2 * q, j.have_left, 0, -1, left0, mid - 1);
+      }
+      if (j.have_left) {
+        const int k = mini(j.y + i, llimit) - j.y;
+        want(2 * q + 1, true, k, -1, (g.left >> (k >> g.cell)) & 1, 0);
+      } else {
+        want(2 * q + 1, j.have_above, -1, 0, above0, mid + 1);
+      }
+    }
+  }
+  v[8] = mid;
+  o[8] = 0;
+  if (lane == 0) {
+    if (j.have_above && j.have_left) want(8, true, -1, -1, g.corner, 0);
+    else if (j.have_above) want(8, true, -1, 0, above0, 0);
+    else want(8, j.have_left, 0, -1, left0, mid);
+  }
+  TagBackoff back;
+  for (;;) {
+    unsigned w[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e)
+      if (pend >> e & 1) w[e] = ld_tag(g.at + o[e]);
+#pragma unroll
+    for (int e = 0; e < 9; ++e)
+      if ((pend >> e & 1) && (w[e] & 0xffff0000u) == g.tag) {
+        v[e] = static_cast<int>(w[e] & 0xffffu);
+        pend &= ~(1u << e);
+      }
+    if (!__any_sync(0xffffffffu, pend)) break;
+    if (!back.next(g, lane)) break;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = lane + 32 * q;
+    if (i < n) {
+      above[i] = v[2 * q];
+      left[i] = v[2 * q + 1];
+    }
+  }
+  if (lane == 0) {
+    above[-1] = v[8];
+    left[-1] = v[8];
+  }
+  __syncwarp();
+}
+
 /* Gathers AboveRow[-1 .. w+h-1] and LeftCol[-1 .. w+h-1]. `p` is the block's
  * top-left sample in the plane. */
 AV1B_DEV void intra_edges(const IntraJob& j, const px_t* p, int stride, int* above, int* left,
-                          int lane) {
+                          const TagIo& g, int lane) {
+  if (g.wait) {
+    intra_edges_tagged(j, p, stride, above, left, g, lane);
+    return;
+  }
   const int n = j.w + j.h;
   const int mid = 1 << (j.bitdepth - 1);
   const int alimit = mini(j.max_x, j.x + (j.have_ar ? 2 * j.w : j.w) - 1);
@@ -222,6 +366,23 @@ AV1B_DEV int dir_sample(const int* above, const int* left, int w, int h, int pan
  * plane, global memory). `plane` points at the plane origin (for CFL's luma,
  * `luma` at the luma plane origin). `scratch` is warp-private shared memory of
  * 3 * AV1B_EDGE_LEN ints. */
+/* The pause of one lane's chroma-from-luma wait after its `it`-th round;
+ * false when the wait has given up. */
+AV1B_DEV bool luma_backoff(const TagIo& g, unsigned it, unsigned long long* t0) {
+  if ((it & 15) == 15) {
+    unsigned long long now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    if (*t0 == 0) *t0 = now;
+    if (ld_tag(reinterpret_cast<const unsigned*>(g.status)) & 1u) return false;
+    if (now - *t0 > g.limit_ns) {
+      atomicOr(g.status, 1);
+      return false;
+    }
+  }
+  if (it >= 3) __nanosleep(64);
+  return true;
+}
+
 /* Waits for the asynchronous copies this thread issued (cp.async), then
  * for the warp: every lane's copies are in shared memory. */
 AV1B_DEV void async_copies_done() {
@@ -232,7 +393,7 @@ AV1B_DEV void async_copies_done() {
 AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t* luma,
                             int luma_stride, const uint8_t* palette_map,
                             const int* palette_colors, int* scratch, int lane,
-                            const int* res = nullptr, int* fi_pred = nullptr,
+                            const TagIo& g, const int* res = nullptr, int* fi_pred = nullptr,
                             bool res_in_flight = false) {
   /* `res_in_flight`: the caller's residual image is still arriving by
    * asynchronous copies; it is waited for after the edges are read (the two
@@ -245,6 +406,7 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
   auto put = [&](int i, int jj, int v) {
     if (res) v = clampi(v + res[i * w + jj], 0, j.maxv);
     dst[i * stride + jj] = (px_t)v;
+    if (g.write && jj < g.clip_w && i < g.clip_h) st_tag(g.write + i * g.stride + jj, g.tag | v);
   };
   if (j.palette) {
     if (res_in_flight) async_copies_done();
@@ -258,7 +420,7 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
   int* above = scratch + AV1B_EDGE_OFF;
   int* left = scratch + AV1B_EDGE_LEN + AV1B_EDGE_OFF;
   int* tmp = scratch + 2 * AV1B_EDGE_LEN;
-  intra_edges(j, dst, stride, above, left, lane);
+  intra_edges(j, dst, stride, above, left, g, lane);
   if (res_in_flight) async_copies_done();
 
   if (j.mode == 13 && fi_pred && n <= 1024) {
@@ -273,13 +435,37 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
     const int lxl = ((j.x + w) << sx) - (1 << sx);
     const int lyl = ((j.y + h) << sy) - (1 << sy);
     long long sum = 0;
+    unsigned long long luma_t0 = 0;
 #pragma unroll 2
     for (int k = lane; k < n; k += 32) {
       const int i = k >> lw, jj = k & (w - 1);
       const int ly = mini((j.y + i) << sy, lyl), lx = mini((j.x + jj) << sx, lxl);
-      const px_t* p0 = luma + ly * luma_stride + lx;
-      const px_t* p1 = p0 + (sy ? luma_stride : 0);
-      const int v00 = ldpx(p0), v01 = ldpx(p0 + sx), v10 = ldpx(p1), v11 = ldpx(p1 + sx);
+      int v00, v01, v10, v11;
+      if (g.luma) {
+        const unsigned* p0 = g.luma_at + ly * g.luma_stride + lx;
+        const unsigned* p1 = p0 + (sy ? g.luma_stride : 0);
+        unsigned a, b, c, d;
+        /* a lane's own wait: lanes leave the loop as their samples arrive */
+        for (unsigned it = 0;; ++it) {
+          a = ld_tag(p0);
+          b = ld_tag(p0 + sx);
+          c = ld_tag(p1);
+          d = ld_tag(p1 + sx);
+          if ((((a ^ g.tag) | (b ^ g.tag) | (c ^ g.tag) | (d ^ g.tag)) & 0xffff0000u) == 0) break;
+          if (!luma_backoff(g, it, &luma_t0)) break;
+        }
+        v00 = static_cast<int>(a & 0xffffu);
+        v01 = static_cast<int>(b & 0xffffu);
+        v10 = static_cast<int>(c & 0xffffu);
+        v11 = static_cast<int>(d & 0xffffu);
+      } else {
+        const px_t* p0 = luma + ly * luma_stride + lx;
+        const px_t* p1 = p0 + (sy ? luma_stride : 0);
+        v00 = ldpx(p0);
+        v01 = ldpx(p0 + sx);
+        v10 = ldpx(p1);
+        v11 = ldpx(p1 + sx);
+      }
       /* the sum of the 1, 2 or 4 samples the subsampling averages, scaled to 8x */
       int t;
       if (sx && sy) t = (v00 + v01 + v10 + v11) << 1;

@@ -693,7 +693,12 @@ cudaError_t launch_selftest_wait(const unsigned* flag, int* status, unsigned lon
  * blocks its list names - except the one before it in the chain, its own
  * work - and reconstructs. Everything that does not depend on other blocks - the
  * block record, its dependency list, its residual - is loaded before the
- * wait. Shared memory per warp: three edge buffers and a 64x64 scratch (the
+ * wait. An intra block waits on the samples it reads, by their tags
+ * (FrameArgs::tags): a step of the critical path is then one store and one
+ * load through L2 and the prediction, where the done flag added the writer's
+ * fence, its store, the poll and the acquire before the samples could be
+ * loaded (a 4K key frame's phase, 1,372 steps: 6.28 -> 4.18 ms, 4.6 -> 3.0 us
+ * a step; 1080p 3.74 -> 2.51; 720p 2.53 -> 1.67). Shared memory per warp: three edge buffers and a 64x64 scratch (the
  * block's residual image, or the transform scratch). */
 /* Adds a phase B transform's residual - precomputed by k_itx, or the raw
  * residual of a residual-provided block - to the reconstructed prediction
@@ -778,9 +783,11 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
       if (a.trace) t_claim = global_ns();
       /* the block before this one in the chain is this warp's own work, already
        * ordered by the warp barrier that ended it */
-      for (int k = lane; k < b.dep_count; k += 32) {
-        const int o = a.deps[b.dep_first + k];
-        if (o != prev) wait_block(a, o);
+      if (!(a.tags && (b.sync & AV1B_SYNC_TAGS))) {
+        for (int k = lane; k < b.dep_count; k += 32) {
+          const int o = a.deps[b.dep_first + k];
+          if (o != prev) wait_block(a, o);
+        }
       }
       __syncwarp();
       if (a.trace) {
@@ -811,7 +818,27 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
       }
 
       px_t* dst = a.cur + g.off + b.y * g.stride + b.x;
+      /* the tagged samples: written with the prediction where it is final */
+      unsigned* tagged = a.tags ? a.tags + a.tag_off[p] + b.y * g.grid_w + b.x : nullptr;
+      const bool tag_last = tagged && !(b.kind == AV1B_U_INTRA && fused);
       if (b.kind == AV1B_U_INTRA) {
+        TagIo t;
+        t.write = tag_last ? nullptr : tagged;
+        t.at = tagged;
+        t.stride = g.grid_w;
+        t.luma_at = a.tags ? a.tags + a.tag_off[0] : nullptr;
+        t.luma_stride = a.L.p[0].grid_w;
+        t.tag = a.tag;
+        t.wait = a.tags && (b.sync & AV1B_SYNC_TAGS);
+        t.luma = a.tags && (b.sync & AV1B_SYNC_LUMA);
+        t.corner = (b.sync & AV1B_SYNC_CORNER) != 0;
+        t.cell = p == 0 ? 2 : ((p == 1 ? a.L.ss_x : a.L.ss_y) ? 1 : 2);
+        t.above = b.wait_cells[0][0] | (static_cast<unsigned long long>(b.wait_cells[0][1]) << 32);
+        t.left = b.wait_cells[1][0] | (static_cast<unsigned long long>(b.wait_cells[1][1]) << 32);
+        t.clip_w = mini(b.w, g.grid_w - b.x);
+        t.clip_h = mini(b.h, g.grid_h - b.y);
+        t.status = a.status;
+        t.limit_ns = a.wait_ns;
         IntraJob j;
         j.x = b.x;
         j.y = b.y;
@@ -839,7 +866,7 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
         /* filter intra (at most 32x32) keeps its predictions after the
          * residual image: tmp[1024 ..] */
         intra_predict(j, dst, g.stride, a.cur + a.L.p[0].off, a.L.p[0].stride, a.palette_map,
-                      a.palette_colors + 8 * b.palette_color_idx, edges, lane,
+                      a.palette_colors + 8 * b.palette_color_idx, edges, lane, t,
                       fused ? tmp : nullptr, tmp + 1024, fused);
       } else if constexpr (INTER) {
         InterJob j;
@@ -856,13 +883,23 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
       __syncwarp();
       if (!fused)
         for (int t = 0; t < b.tx_count; ++t) add_residual_cg(a, b, a.txs[b.tx_first + t], lane);
+      if (tag_last) {
+        /* a block whose samples are final only now: its tags from the picture */
+        __syncwarp();
+        const int tw = mini(b.w, g.grid_w - b.x), th = mini(b.h, g.grid_h - b.y);
+        for (int y = 0; y < th; ++y)
+          for (int x = lane; x < tw; x += 32)
+            st_tag(tagged + y * g.grid_w + x, a.tag | static_cast<unsigned>(ldpx(dst + y * g.stride + x)));
+      }
 
-      /* publish: the barrier orders every lane's stores before lane 0's
-       * release, whose fence (cumulative) makes them visible at GPU scope to
-       * any warp that acquires the flag */
+      /* publish, for the blocks that wait on the done flag: the barrier
+       * orders every lane's stores before lane 0's release, whose fence
+       * (cumulative) makes them visible at GPU scope to any warp that
+       * acquires the flag */
       __syncwarp();
       if (a.trace && lane == 0) a.trace[4 * (size_t)bi + 2] = global_ns();
-      if (lane == 0) st_release(a.done + (size_t)bi * AV1B_FLAG_STRIDE, a.epoch);
+      if (lane == 0 && (!a.tags || (b.sync & AV1B_SYNC_FLAG)))
+        st_release(a.done + (size_t)bi * AV1B_FLAG_STRIDE, a.epoch);
       prev = bi;
     }
   }

@@ -16,10 +16,9 @@ namespace av1b {
 #define AV1B_STATUS_TIMEOUT 1   /* a dependency wait gave up */
 
 /* Everything the reconstruction kernels read, by value. */
-/* Done flags sit 128 bytes apart: the blocks in flight are neighbours in
- * coding order, and flags sharing lines would pile every poll of the frontier
- * onto a few L2 slices, slowing every other access there. */
-#define AV1B_FLAG_STRIDE 32
+/* Done flags sit 32 bytes apart, a flag a sector (few blocks wait on flags:
+ * most wait on tagged samples, and the memory went to the tags). */
+#define AV1B_FLAG_STRIDE 8
 
 /* Phase B: shared-memory scratch per warp (ints) - the residual image of a
  * block whose prediction and residual fuse (so blocks of up to this many
@@ -58,6 +57,15 @@ struct FrameArgs {
   unsigned* done;               /* per block, AV1B_FLAG_STRIDE apart: == epoch once
                                    reconstructed (phase B) */
   unsigned epoch;
+  /* The tagged samples of phase B: a word a sample of each plane's grid
+   * (grid_w a row), (tag << 16) | sample once the block that owns it has
+   * reconstructed it in the frame of this tag. A word carries its own
+   * validity, so a reader needs no flag and no fence: it loads the samples it
+   * is about to use until their tags match. Null: every wait is on done
+   * flags. */
+  unsigned* tags;
+  unsigned tag;
+  int tag_off[3];
   const int* units;             /* phase B block indices, chain after chain */
   const int* chains;            /* chain c is units[chains[c] .. chains[c + 1]) */
   int n_chains;
