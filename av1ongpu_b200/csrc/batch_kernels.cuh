@@ -40,8 +40,7 @@ __device__ __forceinline__ int warp_claim(unsigned* ctr, int chunk, int lane) {
 template <bool MASK>
 __global__ void __launch_bounds__(128, 5) kb_inter_simple(const StreamStep* __restrict__ st,
                                                        BatchHeader* h, int chunk, int part) {
-  __shared__ McScratch scr[4];
-  __shared__ int pred[4][2][8 * 16];
+  __shared__ McTileBuf buf[4][2];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stage = !MASK ? kBInterSimple : (part ? kBInterMask : kBInterLeanMask);
   const int* pfx = h->pfx[stage];
@@ -55,7 +54,7 @@ __global__ void __launch_bounds__(128, 5) kb_inter_simple(const StreamStep* __re
       s = batch_stream_next(pfx, n, i, s);
       const FrameArgs& a = st[s].a;
       const int t0 = !MASK ? 0 : (part ? a.n_inter_tiles - a.n_inter_cmask : a.n_inter_simple);
-      inter_simple_tile<MASK>(a, t0 + (i - pfx[s]), scr[wib], pred[wib], lane);
+      inter_simple_tile<MASK>(a, t0 + (i - pfx[s]), buf[wib], lane);
       __syncwarp();
     }
   }

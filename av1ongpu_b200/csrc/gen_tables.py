@@ -56,7 +56,8 @@ w('''/*
  * gen_tables.py; do not edit). Flattened, one-dimensional where the kernels
  * index them with computed offsets.
  *
- * AV1B_TABLE is the storage class: __device__ for the CUDA build (global
+ * AV1B_TABLE is the storage class: __device__ for the CUDA build (16-byte
+ * aligned, so that a row of eight filter taps is one load; global
  * memory, read through the L1 so that divergent indices do not serialize the
  * way a __constant__ bank would), plain static const for host code.
  * AV1B_CTABLE: the constant bank, for the small tables a warp reads at one
@@ -67,7 +68,7 @@ w('''/*
 #ifndef AV1B_TABLES_H
 #define AV1B_TABLES_H
 #if defined(__CUDACC__)
-#define AV1B_TABLE static __device__ const
+#define AV1B_TABLE static __device__ const __align__(16)
 #define AV1B_CTABLE static __constant__ const
 #else
 #define AV1B_TABLE static const

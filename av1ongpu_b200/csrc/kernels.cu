@@ -169,6 +169,30 @@ __device__ __forceinline__ int lean_mask(const FrameArgs& a, const LeanMask& k, 
   return n == 1 ? sum : (n == 2 ? (sum + 1) >> 1 : (sum + 2) >> 2);
 }
 
+/* Sample (x, y) of a block's job (a reference, or an OBMC strip, whose own
+ * coordinates these then are), by mc_tap, out of line: the lean kernel's way
+ * for windows that do not fit its buffers, which no reference of a valid
+ * stream has. */
+__device__ __noinline__ int mc_tap_far(const FrameArgs& a, const BlockRec& b, int job, int x, int y) {
+  const int p = b.plane;
+  const PlaneGeom& g = a.L.p[p];
+  InterCtx c;
+  c.sub_x = p > 0 ? a.L.ss_x : 0;
+  c.sub_y = p > 0 ? a.L.ss_y : 0;
+  c.ref_w = g.out_w;
+  c.ref_h = g.out_h;
+  c.bitdepth = a.L.bit_depth;
+  c.scale_x = a.scale_x;
+  c.scale_y = a.scale_y;
+  const int nref = b.compound ? 2 : 1;
+  if (job < nref)
+    return mc_tap(c, ref_plane(a, b.ref_slot[job], p), g.stride, b.x, b.y, b.w, b.h, b.mv[job][0],
+                  b.mv[job][1], b.filt, b.filt_v, x, y, b.compound != 0);
+  const ObmcRec& o = a.obmc[b.obmc_first + job - nref];
+  return mc_tap(c, ref_plane(a, o.ref_slot, p), g.stride, b.x + o.x, b.y + o.y, o.w, o.h, o.mv_x, o.mv_y,
+                o.filt, o.filt_v, x, y, 0);
+}
+
 /* Inter prediction of the phase A blocks but inter-intra ones and chroma
  * blocks of difference-weighted compounds without a luma mask to read (they
  * take the full kernel): one warp per 16x8 tile, each reference through
@@ -181,8 +205,8 @@ __device__ __forceinline__ int lean_mask(const FrameArgs& a, const LeanMask& k, 
  * true: wedge and difference-weighted compounds) - the mask code in the
  * first build slows its tiles by a fifth. */
 template <bool MASK>
-__device__ __forceinline__ void inter_simple_tile(const FrameArgs& a, int tile, McScratch& scr,
-                                                  int (&pred)[2][8 * 16], int lane) {
+__device__ __forceinline__ void inter_simple_tile(const FrameArgs& a, int tile, McTileBuf (&buf)[2],
+                                                  int lane) {
   const int2 t = a.inter_tiles[tile];
   const BlockRec& b = a.blocks[t.x];
   const int p = b.plane;
@@ -195,94 +219,125 @@ __device__ __forceinline__ void inter_simple_tile(const FrameArgs& a, int tile, 
   c.bitdepth = a.L.bit_depth;
   c.scale_x = a.scale_x;
   c.scale_y = a.scale_y;
+  const bool scaled = c.scale_x != AV1B_SCALE_ONE;
   const int x0 = t.y & 0xffff, y0 = t.y >> 16;
   const int tw = mini(16, b.w - x0), th = mini(8, b.h - y0);
-  /* k / tw for the tile's k < 128 as a multiply and a shift (exact there) */
-  const int tmul = (65536 + tw - 1) / tw;
-  const int nref = b.compound ? 2 : 1;
-  for (int r = 0; r < nref; ++r) {
-    int* pr = pred[r];
-    const px_t* ref = ref_plane(a, b.ref_slot[r], p);
-    if (r == 0 ? b.warp0 : b.warp1) {
-      /* one or two whole 8x8 warp blocks (x0 is a multiple of 16, y0 of 8) */
-      const WarpRec& m = a.warps[b.warp_idx[r] >= 0 ? b.warp_idx[r] : 0];
-      for (int bx = 0; bx < tw; bx += 8)
-        warp_block8(c.sub_x, c.sub_y, c.ref_w, c.ref_h, m, ref, g.stride, b.x, b.y, x0 + bx, y0,
-                    c.bitdepth, b.compound != 0, scr, pr + bx, 16, mini(8, tw - bx), th, lane);
-      continue;
-    }
-    if (!mc_rect(c, ref, g.stride, b.x, b.y, b.w, b.h, b.mv[r][0], b.mv[r][1], b.filt, b.filt_v,
-                 b.compound != 0, x0, y0, tw, th, scr, pr, lane)) {
-      for (int k = lane; k < tw * th; k += 32) {
-        const int yy = k / tw, xx = k - yy * tw;
-        pr[yy * 16 + xx] = mc_tap(c, ref, g.stride, b.x, b.y, b.w, b.h, b.mv[r][0], b.mv[r][1],
-                                  b.filt, b.filt_v, x0 + xx, y0 + yy, b.compound != 0);
-      }
-      __syncwarp();
-    }
-  }
-  px_t* dst = a.cur + g.off + (b.y + y0) * g.stride + b.x + x0;
+  /* the lane's samples: columns col, col + 1 of rows row, row + 1 */
+  const int col = (lane & 7) * 2, row = (lane >> 3) * 2;
+  const int compound = b.compound;
+  const int nref = compound ? 2 : 1;
+  const int jobs = nref + b.obmc_count;
   const int post = 7 - (c.bitdepth >= 12 ? 5 : 3);
-  int acc[4];
-  if constexpr (MASK) {
-    const LeanMask mk(b);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k = lane + 32 * q;
-      if (k >= tw * th) continue;
-      const int yy = (k * tmul) >> 16, xx = k - yy * tw;
-      const int v0 = pred[0][yy * 16 + xx], v1 = pred[1][yy * 16 + xx];
-      const int m = lean_mask(a, mk, p, c.sub_x, c.sub_y, c.bitdepth, x0 + xx, y0 + yy, v0, v1);
-      acc[q] = clampi((m * v0 + (64 - m) * v1 + (1 << (5 + post))) >> (6 + post), 0, a.maxv);
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k = lane + 32 * q;
-      if (k >= tw * th) continue;
-      const int yy = (k * tmul) >> 16, xx = k - yy * tw;
-      const int v0 = pred[0][yy * 16 + xx];
-      int out = v0;
-      if (b.compound == 1) {
-        out = (v0 + pred[1][yy * 16 + xx] + (1 << post)) >> (1 + post);
-      } else if (b.compound) {
-        out = (b.w0 * v0 + b.w1 * pred[1][yy * 16 + xx] + (1 << (3 + post))) >> (4 + post);
+  int v0[4] = {0, 0, 0, 0}, acc[4] = {0, 0, 0, 0};
+  McReq cur{}, nxt{};
+  /* what a job is: 0 nothing of the tile, 1 a window on its way, 2 a warped
+   * reference, 3 a translation the window does not fit */
+  int kind = 0, kind_next = 0;
+  /* The references, then the OBMC strips in order, each blended onto the
+   * samples it covers; a job's window is started before the one before it is
+   * filtered. */
+  for (int job = -1; job < jobs; ++job) {
+    kind_next = 0;
+    if (job + 1 < jobs) {
+      const int n = job + 1;
+      McTileBuf& dst = buf[n & 1];
+      if (n < nref) {
+        if (n == 0 ? b.warp0 : b.warp1) {
+          kind_next = 2;
+        } else {
+          kind_next = mc_request(c, ref_plane(a, b.ref_slot[n], p), g.stride, b.x, b.y, b.w, b.h,
+                                 b.mv[n][0], b.mv[n][1], b.filt, b.filt_v, x0, y0, tw, th, 0, 0, dst, nxt, lane)
+                          ? 1
+                          : 3;
+        }
+      } else {
+        const ObmcRec& o = a.obmc[b.obmc_first + n - nref];
+        const int ix0 = maxi(o.x, x0), ix1 = mini(o.x + o.w, x0 + tw);
+        const int iy0 = maxi(o.y, y0), iy1 = mini(o.y + o.h, y0 + th);
+        if (ix0 < ix1 && iy0 < iy1) {
+          const int c0 = (ix0 - x0) & ~1, r0 = (iy0 - y0) & ~1;
+          kind_next = mc_request(c, ref_plane(a, o.ref_slot, p), g.stride, b.x + o.x, b.y + o.y, o.w, o.h,
+                                 o.mv_x, o.mv_y, o.filt, o.filt_v, x0 + c0 - o.x, y0 + r0 - o.y,
+                                 ix1 - x0 - c0, iy1 - y0 - r0, c0, r0, dst, nxt, lane)
+                          ? 1
+                          : 3;
+        }
       }
-      acc[q] = clampi(out, 0, a.maxv);
     }
-  }
-  __syncwarp();
-  /* OBMC: the strips in order, each blended onto the samples it covers */
-  for (int kk = 0; kk < b.obmc_count; ++kk) {
-    const ObmcRec& o = a.obmc[b.obmc_first + kk];
-    const int ix0 = maxi(o.x, x0), ix1 = mini(o.x + o.w, x0 + tw);
-    const int iy0 = maxi(o.y, y0), iy1 = mini(o.y + o.h, y0 + th);
-    if (ix0 >= ix1 || iy0 >= iy1) continue;
-    int* tmp = pred[0];
-    const px_t* oref = ref_plane(a, o.ref_slot, p);
-    const bool ok = mc_rect(c, oref, g.stride, b.x + o.x, b.y + o.y, o.w, o.h, o.mv_x, o.mv_y, o.filt,
-                            o.filt_v, 0, ix0 - o.x, iy0 - o.y, ix1 - ix0, iy1 - iy0, scr, tmp,
-                            lane);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (job >= 0) {
+      McTileBuf& src = buf[job & 1];
+      int out[4] = {0, 0, 0, 0};
+      if (kind == 1) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        mc_filter(cur, scaled, src, c.bitdepth, job < nref ? compound : 0, col, row, out, lane);
+      } else if (kind == 2) {
+        /* one or two whole 8x8 warp blocks (x0 is a multiple of 16, y0 of 8) */
+        const int wi = b.warp_idx[job];
+        const WarpRec& m = a.warps[wi >= 0 ? wi : 0];
+        for (int bx = 0; bx < tw; bx += 8)
+          warp_block8(c.sub_x, c.sub_y, c.ref_w, c.ref_h, m, ref_plane(a, b.ref_slot[job], p), g.stride,
+                      b.x, b.y, x0 + bx, y0, c.bitdepth, compound != 0, src.wwin, src.wmid,
+                      src.wout + bx, 16, mini(8, tw - bx), th, lane);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k = lane + 32 * q;
-      if (k >= tw * th) continue;
-      const int yy = (k * tmul) >> 16, xx = k - yy * tw;
-      const int x = x0 + xx, y = y0 + yy;
-      if (x < ix0 || x >= ix1 || y < iy0 || y >= iy1) continue;
-      const int pv = ok ? tmp[(y - iy0) * 16 + x - ix0]
-                        : mc_tap(c, oref, g.stride, b.x + o.x, b.y + o.y, o.w, o.h, o.mv_x, o.mv_y,
-                                 o.filt, o.filt_v, x - o.x, y - o.y, 0);
-      acc[q] = obmc_blend(o, x - o.x, y - o.y, acc[q], pv, a.maxv);
+        for (int e = 0; e < 4; ++e) out[e] = src.wout[(row + (e >> 1)) * 16 + col + (e & 1)];
+        __syncwarp();
+      }
+      if (job < nref) {
+        if (kind == 3) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int x = col + (e & 1), y = row + (e >> 1);
+            if (x < tw && y < th)
+              out[e] = mc_tap_far(a, b, job, x0 + x, y0 + y);
+          }
+        }
+        if (job + 1 < nref) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v0[e] = out[e];
+        } else if constexpr (MASK) {
+          const LeanMask mk(b);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int x = col + (e & 1), y = row + (e >> 1);
+            if (x >= tw || y >= th) continue;
+            const int m = lean_mask(a, mk, p, c.sub_x, c.sub_y, c.bitdepth, x0 + x, y0 + y, v0[e], out[e]);
+            acc[e] = clampi((m * v0[e] + (64 - m) * out[e] + (1 << (5 + post))) >> (6 + post), 0, a.maxv);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            int v = out[e];
+            if (compound == 1) v = (v0[e] + v + (1 << post)) >> (1 + post);
+            else if (compound) v = (b.w0 * v0[e] + b.w1 * v + (1 << (3 + post))) >> (4 + post);
+            acc[e] = clampi(v, 0, a.maxv);
+          }
+        }
+      } else if (kind) {
+        const ObmcRec& o = a.obmc[b.obmc_first + job - nref];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int x = x0 + col + (e & 1) - o.x, y = y0 + row + (e >> 1) - o.y;
+          if (x < 0 || x >= o.w || y < 0 || y >= o.h || col + (e & 1) >= tw || row + (e >> 1) >= th) continue;
+          const int pv = kind == 1 ? out[e]
+                                   : mc_tap_far(a, b, job, x, y);
+          acc[e] = obmc_blend(o, x, y, acc[e], pv, a.maxv);
+        }
+      }
     }
-    __syncwarp();
+    cur = nxt;
+    kind = kind_next;
   }
+  px_t* dst = a.cur + g.off + (b.y + y0 + row) * g.stride + b.x + x0 + col;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int k = lane + 32 * q;
-    if (k < tw * th) {
-      const int yy = (k * tmul) >> 16, xx = k - yy * tw;
-      dst[yy * g.stride + xx] = (px_t)acc[q];
+  for (int r = 0; r < 2; ++r, dst += g.stride) {
+    if (row + r >= th || col >= tw) continue;
+    if (col + 1 < tw && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+      *reinterpret_cast<unsigned*>(dst) = static_cast<unsigned>(acc[2 * r]) | (static_cast<unsigned>(acc[2 * r + 1]) << 16);
+    } else {
+      dst[0] = static_cast<px_t>(acc[2 * r]);
+      if (col + 1 < tw) dst[1] = static_cast<px_t>(acc[2 * r + 1]);
     }
   }
 }
@@ -292,14 +347,13 @@ __device__ __forceinline__ void inter_simple_tile(const FrameArgs& a, int tile, 
  * next and (a launch of their own, after the luma tiles that write the
  * masks) the chroma tiles that read a luma mask, listed last. */
 template <bool MASK>
-__global__ void __launch_bounds__(128) k_inter_simple(const __grid_constant__ FrameArgs a, int first,
+__global__ void __launch_bounds__(128, 5) k_inter_simple(const __grid_constant__ FrameArgs a, int first,
                                                       int end) {
-  __shared__ McScratch scr[4];
-  __shared__ int pred[4][2][8 * 16];
+  __shared__ McTileBuf buf[4][2];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warp = first + blockIdx.x * 4 + wib;
   if (warp >= end) return;
-  inter_simple_tile<MASK>(a, warp, scr[wib], pred[wib], lane);
+  inter_simple_tile<MASK>(a, warp, buf[wib], lane);
 }
 
 /* Inter prediction of phase A blocks: one warp per 16x8 tile. Translation
@@ -339,8 +393,8 @@ __device__ __forceinline__ void inter_full_tile(const FrameArgs& a, int tile, Mc
        * 16, y0 of 8) */
       for (int bx = 0; bx < tw; bx += 8)
         warp_block8(j.ctx.sub_x, j.ctx.sub_y, j.ctx.ref_w, j.ctx.ref_h, *j.model[r], j.ref[r],
-                    j.ref_stride, j.x, j.y, x0 + bx, y0, j.ctx.bitdepth, j.compound != 0, scr,
-                    pr + bx, 16, mini(8, tw - bx), th, lane);
+                    j.ref_stride, j.x, j.y, x0 + bx, y0, j.ctx.bitdepth, j.compound != 0, scr.win,
+                    scr.mid, pr + bx, 16, mini(8, tw - bx), th, lane);
       continue;
     }
     const bool ok = mc_rect(j.ctx, j.ref[r], j.ref_stride, j.x, j.y, j.w, j.h, j.mv[r][0],
@@ -377,7 +431,7 @@ __device__ __forceinline__ void inter_full_tile(const FrameArgs& a, int tile, Mc
             for (int bx = 0; bx < rw; bx += 8)
               warp_block8(0, 0, j.luma_ref_w, j.luma_ref_h, *j.model[r], j.luma_ref[r],
                           j.luma_stride, j.luma_x, j.luma_y, lx0 + qx + bx, ly0 + qy,
-                          j.ctx.bitdepth, 1, scr, out + bx, 16, mini(8, rw - bx), rh, lane);
+                          j.ctx.bitdepth, 1, scr.win, scr.mid, out + bx, 16, mini(8, rw - bx), rh, lane);
           } else if (!mc_rect(l, j.luma_ref[r], j.luma_stride, j.luma_x, j.luma_y, ew, eh,
                               j.mv[r][0], j.mv[r][1], j.filt, j.filt_v, 1, lx0 + qx, ly0 + qy, rw,
                               rh, scr, out, lane)) {
