@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(128, MINB) kb_inter(const StreamStep* __restri
 }
 
 template <int CLS>
-__global__ void __launch_bounds__(128) kb_itx(const StreamStep* __restrict__ st, BatchHeader* h,
+__global__ void __launch_bounds__(128, kItxCtas[CLS]) kb_itx(const StreamStep* __restrict__ st, BatchHeader* h,
                                               int chunk) {
   extern __shared__ int smem[];
   constexpr int STAGE = kBItx2 + (CLS == 7 ? 5 : CLS - 2);
@@ -398,11 +398,7 @@ cudaError_t set_batch_kernel_attributes() {
       (e = cudaFuncSetAttribute(kb_units<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
       (e = cudaFuncSetAttribute(kb_units<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(kb_itx<6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                4 * 4096 * (int)sizeof(int))) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(kb_itx<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                4 * 4096 * (int)sizeof(int))) != cudaSuccess)
+                                cudaSharedmemCarveoutMaxShared)) != cudaSuccess)
     return e;
   /* load every batched kernel now (lazy loading would load one at its first
    * launch, inside a step, waiting for the kernels running) */

@@ -12,7 +12,8 @@
  *
  * Products are formed in 64 bits and rounded back (Round2(x, 12)), which is
  * what the reference does (av1gpu_kernels.h:495-508) so that an out-of-range
- * coefficient gives the same wrapped result on every backend.
+ * coefficient gives the same wrapped result on every backend - or in 32 bits
+ * where the values' range gives the same integers (mul_rnd12).
  *
  * The 2-D transform of one block is done by one warp: lanes take rows for the
  * first pass (results to shared memory, clamped to the column range) and
@@ -21,6 +22,8 @@
  */
 #ifndef AV1B_DEV_ITX_CUH
 #define AV1B_DEV_ITX_CUH
+
+#include <type_traits>
 
 #include "dev_common.cuh"
 
@@ -41,13 +44,32 @@ AV1B_HD constexpr int brev(int bits, int x) {
   return r;
 }
 
+/* The arithmetic of a 1-D transform's products: 64-bit, or 32-bit (NARROW)
+ * where the inputs and the clips of the transform's range lie within +-2^17.
+ * There no product sum passes 2^31: a rotation's is at most |(a, b)| 2^12,
+ * and its inputs are clipped values or, at most twice rotated since their
+ * clip, 2 x 2^17; the 4-point ADST's is at most (1321 + 2482 + 3344 + 3803)
+ * 2^17. The integers are the same; 64-bit products and shifts took the
+ * transforms twice the multiply issue and the registers of a pair each. */
+template <bool NARROW>
+AV1B_DEV int mul_rnd12(int a, int b) {
+  if constexpr (NARROW) return (a * b + 2048) >> 12;
+  else return rnd2ll((long long)a * b, 12);
+}
+
 /* B(a, b, angle, flip) */
-template <int N>
+template <bool NARROW, int N>
 AV1B_DEV void rot(int (&t)[N], int a, int b, int angle, bool flip) {
-  const long long c = cos128(angle), s = sin128(angle);
-  const long long ta = t[a], tb = t[b];
-  const int x = rnd2ll(ta * c - tb * s, 12);
-  const int y = rnd2ll(ta * s + tb * c, 12);
+  const int c = cos128(angle), s = sin128(angle);
+  const int ta = t[a], tb = t[b];
+  int x, y;
+  if constexpr (NARROW) {
+    x = (ta * c - tb * s + 2048) >> 12;
+    y = (ta * s + tb * c + 2048) >> 12;
+  } else {
+    x = rnd2ll((long long)ta * c - (long long)tb * s, 12);
+    y = rnd2ll((long long)ta * s + (long long)tb * c, 12);
+  }
   t[a] = flip ? y : x;
   t[b] = flip ? x : y;
 }
@@ -64,7 +86,7 @@ AV1B_DEV void had(int (&t)[N], int a, int b, bool flip, int lo, int hi) {
 }
 
 /* Inverse DCT array process for 2^n points, n = 2..6. */
-template <int n, int N>
+template <bool NARROW, int n, int N>
 AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   constexpr int L = 1 << n;
   {
@@ -76,11 +98,11 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   }
   if constexpr (n == 6) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) rot(t, 32 + i, 63 - i, 63 - 4 * brev(4, i), false);
+    for (int i = 0; i < 16; ++i) rot<NARROW>(t, 32 + i, 63 - i, 63 - 4 * brev(4, i), false);
   }
   if constexpr (n >= 5) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) rot(t, 16 + i, 31 - i, 6 + (brev(3, 7 - i) << 3), false);
+    for (int i = 0; i < 8; ++i) rot<NARROW>(t, 16 + i, 31 - i, 6 + (brev(3, 7 - i) << 3), false);
   }
   if constexpr (n == 6) {
 #pragma unroll
@@ -88,7 +110,7 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   }
   if constexpr (n >= 4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) rot(t, 8 + i, 15 - i, 12 + (brev(2, 3 - i) << 4), false);
+    for (int i = 0; i < 4; ++i) rot<NARROW>(t, 8 + i, 15 - i, 12 + (brev(2, 3 - i) << 4), false);
   }
   if constexpr (n >= 5) {
 #pragma unroll
@@ -99,11 +121,11 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j)
-        rot(t, 62 - i * 4 - j, 33 + i * 4 + j, 60 - 16 * brev(2, i) + 64 * j, true);
+        rot<NARROW>(t, 62 - i * 4 - j, 33 + i * 4 + j, 60 - 16 * brev(2, i) + 64 * j, true);
   }
   if constexpr (n >= 3) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) rot(t, 4 + i, 7 - i, 56 - 32 * i, false);
+    for (int i = 0; i < 2; ++i) rot<NARROW>(t, 4 + i, 7 - i, 56 - 32 * i, false);
   }
   if constexpr (n >= 4) {
 #pragma unroll
@@ -114,7 +136,7 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j)
-        rot(t, 30 - 4 * i - j, 17 + 4 * i + j, 24 + (j << 6) + ((1 - i) << 5), true);
+        rot<NARROW>(t, 30 - 4 * i - j, 17 + 4 * i + j, 24 + (j << 6) + ((1 - i) << 5), true);
   }
   if constexpr (n == 6) {
 #pragma unroll
@@ -123,14 +145,14 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
       for (int j = 0; j < 2; ++j) had(t, 32 + i * 4 + j, 35 + i * 4 - j, i & 1, lo, hi);
   }
 #pragma unroll
-  for (int i = 0; i < 2; ++i) rot(t, 2 * i, 2 * i + 1, 32 + 16 * i, i == 0);
+  for (int i = 0; i < 2; ++i) rot<NARROW>(t, 2 * i, 2 * i + 1, 32 + 16 * i, i == 0);
   if constexpr (n >= 3) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) had(t, 4 + 2 * i, 5 + 2 * i, i, lo, hi);
   }
   if constexpr (n >= 4) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) rot(t, 14 - i, 9 + i, 48 + 64 * i, true);
+    for (int i = 0; i < 2; ++i) rot<NARROW>(t, 14 - i, 9 + i, 48 + 64 * i, true);
   }
   if constexpr (n >= 5) {
 #pragma unroll
@@ -143,11 +165,11 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        rot(t, 61 - i * 8 - j, 34 + i * 8 + j, 56 - i * 32 + (j >> 1) * 64, true);
+        rot<NARROW>(t, 61 - i * 8 - j, 34 + i * 8 + j, 56 - i * 32 + (j >> 1) * 64, true);
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i) had(t, i, 3 - i, false, lo, hi);
-  if constexpr (n >= 3) rot(t, 6, 5, 32, true);
+  if constexpr (n >= 3) rot<NARROW>(t, 6, 5, 32, true);
   if constexpr (n >= 4) {
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -156,7 +178,7 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   }
   if constexpr (n >= 5) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) rot(t, 29 - i, 18 + i, 48 + (i >> 1) * 64, true);
+    for (int i = 0; i < 4; ++i) rot<NARROW>(t, 29 - i, 18 + i, 48 + (i >> 1) * 64, true);
   }
   if constexpr (n == 6) {
 #pragma unroll
@@ -170,7 +192,7 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   }
   if constexpr (n >= 4) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) rot(t, 13 - i, 10 + i, 32, true);
+    for (int i = 0; i < 2; ++i) rot<NARROW>(t, 13 - i, 10 + i, 32, true);
   }
   if constexpr (n >= 5) {
 #pragma unroll
@@ -180,7 +202,7 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   }
   if constexpr (n == 6) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) rot(t, 59 - i, 36 + i, i < 4 ? 48 : 112, true);
+    for (int i = 0; i < 8; ++i) rot<NARROW>(t, 59 - i, 36 + i, i < 4 ? 48 : 112, true);
   }
   if constexpr (n >= 4) {
 #pragma unroll
@@ -188,7 +210,7 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   }
   if constexpr (n >= 5) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) rot(t, 27 - i, 20 + i, 32, true);
+    for (int i = 0; i < 4; ++i) rot<NARROW>(t, 27 - i, 20 + i, 32, true);
   }
   if constexpr (n == 6) {
 #pragma unroll
@@ -203,7 +225,7 @@ AV1B_DEV void idct(int (&t)[N], int lo, int hi) {
   }
   if constexpr (n == 6) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) rot(t, 55 - i, 40 + i, 32, true);
+    for (int i = 0; i < 8; ++i) rot<NARROW>(t, 55 - i, 40 + i, 32, true);
 #pragma unroll
     for (int i = 0; i < 32; ++i) had(t, i, 63 - i, false, lo, hi);
   }
@@ -238,56 +260,55 @@ AV1B_DEV void adst_out(int (&t)[N]) {
   }
 }
 
-template <int N>
+template <bool NARROW, int N>
 AV1B_DEV void adst4(int (&t)[N]) {
-  const long long s0a = (long long)AV1B_SINPI_1_9 * t[0];
-  const long long s1a = (long long)AV1B_SINPI_2_9 * t[0];
-  const long long s2a = (long long)AV1B_SINPI_3_9 * t[1];
-  const long long s3a = (long long)AV1B_SINPI_4_9 * t[2];
-  const long long s4 = (long long)AV1B_SINPI_1_9 * t[2];
-  const long long s5 = (long long)AV1B_SINPI_2_9 * t[3];
-  const long long s6 = (long long)AV1B_SINPI_4_9 * t[3];
-  const int a7 = t[0] - t[2];
-  const int b7 = a7 + t[3];
-  const long long s0 = s0a + s3a + s5;
-  const long long s1 = s1a - s4 - s6;
-  const long long s3 = s2a;
-  const long long s2 = (long long)AV1B_SINPI_3_9 * b7;
-  t[0] = rnd2ll(s0 + s3, 12);
-  t[1] = rnd2ll(s1 + s3, 12);
-  t[2] = rnd2ll(s2, 12);
-  t[3] = rnd2ll(s0 + s1 - s3, 12);
+  /* 32-bit sums may pass 2^31 on the way: only the totals have to fit */
+  using acc_t = std::conditional_t<NARROW, unsigned, long long>;
+  const auto mul = [](int k, int v) { return static_cast<acc_t>(k) * static_cast<acc_t>(v); };
+  const auto rnd = [](acc_t v) {
+    if constexpr (NARROW) return static_cast<int>(v + 2048u) >> 12;
+    else return rnd2ll(v, 12);
+  };
+  const int b7 = t[0] - t[2] + t[3];
+  const acc_t s0 = mul(AV1B_SINPI_1_9, t[0]) + mul(AV1B_SINPI_4_9, t[2]) + mul(AV1B_SINPI_2_9, t[3]);
+  const acc_t s1 = mul(AV1B_SINPI_2_9, t[0]) - mul(AV1B_SINPI_1_9, t[2]) - mul(AV1B_SINPI_4_9, t[3]);
+  const acc_t s3 = mul(AV1B_SINPI_3_9, t[1]);
+  const acc_t s2 = mul(AV1B_SINPI_3_9, b7);
+  t[0] = rnd(s0 + s3);
+  t[1] = rnd(s1 + s3);
+  t[2] = rnd(s2);
+  t[3] = rnd(s0 + s1 - s3);
 }
 
-template <int N>
+template <bool NARROW, int N>
 AV1B_DEV void adst8(int (&t)[N], int lo, int hi) {
   adst_in<3>(t);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) rot(t, 2 * i, 2 * i + 1, 60 - 16 * i, true);
+  for (int i = 0; i < 4; ++i) rot<NARROW>(t, 2 * i, 2 * i + 1, 60 - 16 * i, true);
 #pragma unroll
   for (int i = 0; i < 4; ++i) had(t, i, 4 + i, false, lo, hi);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) rot(t, 4 + 3 * i, 5 + i, 48 - 32 * i, true);
+  for (int i = 0; i < 2; ++i) rot<NARROW>(t, 4 + 3 * i, 5 + i, 48 - 32 * i, true);
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j) had(t, 4 * j + i, 2 + 4 * j + i, false, lo, hi);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) rot(t, 2 + 4 * i, 3 + 4 * i, 32, true);
+  for (int i = 0; i < 2; ++i) rot<NARROW>(t, 2 + 4 * i, 3 + 4 * i, 32, true);
   adst_out<3>(t);
 }
 
-template <int N>
+template <bool NARROW, int N>
 AV1B_DEV void adst16(int (&t)[N], int lo, int hi) {
   adst_in<4>(t);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) rot(t, 2 * i, 2 * i + 1, 62 - 8 * i, true);
+  for (int i = 0; i < 8; ++i) rot<NARROW>(t, 2 * i, 2 * i + 1, 62 - 8 * i, true);
 #pragma unroll
   for (int i = 0; i < 8; ++i) had(t, i, 8 + i, false, lo, hi);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    rot(t, 8 + 2 * i, 9 + 2 * i, 56 - 32 * i, true);
-    rot(t, 13 + 2 * i, 12 + 2 * i, 8 + 32 * i, true);
+    rot<NARROW>(t, 8 + 2 * i, 9 + 2 * i, 56 - 32 * i, true);
+    rot<NARROW>(t, 13 + 2 * i, 12 + 2 * i, 8 + 32 * i, true);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -296,25 +317,25 @@ AV1B_DEV void adst16(int (&t)[N], int lo, int hi) {
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) rot(t, 4 + 8 * j + 3 * i, 5 + 8 * j + i, 48 - 32 * i, true);
+    for (int j = 0; j < 2; ++j) rot<NARROW>(t, 4 + 8 * j + 3 * i, 5 + 8 * j + i, 48 - 32 * i, true);
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) had(t, 4 * j + i, 2 + 4 * j + i, false, lo, hi);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) rot(t, 2 + 4 * i, 3 + 4 * i, 32, true);
+  for (int i = 0; i < 4; ++i) rot<NARROW>(t, 2 + 4 * i, 3 + 4 * i, 32, true);
   adst_out<4>(t);
 }
 
 /* The identity transforms rescale to the Q12 convention of the others. */
-template <int n, int N>
+template <bool NARROW, int n, int N>
 AV1B_DEV void iidentity(int (&t)[N]) {
   constexpr int L = 1 << n;
 #pragma unroll
   for (int i = 0; i < L; ++i) {
-    if constexpr (n == 2) t[i] = rnd2ll((long long)t[i] * 5793, 12);
+    if constexpr (n == 2) t[i] = mul_rnd12<NARROW>(t[i], 5793);
     else if constexpr (n == 3) t[i] = t[i] * 2;
-    else if constexpr (n == 4) t[i] = rnd2ll((long long)t[i] * 11586, 12);
+    else if constexpr (n == 4) t[i] = mul_rnd12<NARROW>(t[i], 11586);
     else t[i] = t[i] * 4;
   }
 }
@@ -378,16 +399,16 @@ AV1B_HD int tx_row_shift(int lw, int lh) {
   }
 }
 
-template <int n, int N>
+template <bool NARROW, int n, int N>
 AV1B_DEV void tx1d(int (&t)[N], int kind, int lo, int hi) {
   if (kind == kTxDct) {
-    idct<n>(t, lo, hi);
+    idct<NARROW, n>(t, lo, hi);
   } else if (kind == kTxAdst) {
-    if constexpr (n == 2) adst4(t);
-    else if constexpr (n == 3) adst8(t, lo, hi);
-    else adst16(t, lo, hi); /* the reference runs 16 points for every n >= 4 */
+    if constexpr (n == 2) adst4<NARROW>(t);
+    else if constexpr (n == 3) adst8<NARROW>(t, lo, hi);
+    else adst16<NARROW>(t, lo, hi); /* the reference runs 16 points for every n >= 4 */
   } else {
-    iidentity<n < 5 ? n : 5>(t); /* and scales 32 points by 4 for every n >= 5 */
+    iidentity<NARROW, n < 5 ? n : 5>(t); /* and scales 32 points by 4 for every n >= 5 */
   }
 }
 
@@ -402,20 +423,46 @@ struct ItxParams {
   int bitdepth;
 };
 
-/* Pass 1 for row `y`: coefficients (raster, min(w,32) wide, rows >= 32 are
- * zero) -> tmp[y * w + j], clamped to the column range. */
+/* Ints a row of the intermediate: four more than its width from 8 on, so
+ * that the rows the lanes of pass 1 write, 16 bytes a store, start in
+ * different banks. */
+AV1B_HD constexpr int itx_stride(int lw) { return (1 << lw) + (lw >= 3 ? 4 : 0); }
+
+/* The arithmetic of pass 1 on a row's coefficients, in place: the 2:1
+ * rectangle's scale, the transform, the row shift and the clip to the column
+ * range. */
+template <bool NARROW, int LW>
+AV1B_DEV void itx_row_values(const ItxParams& p, int (&t)[1 << LW]) {
+  constexpr int W = 1 << LW;
+  const int col_bits = maxi(p.bitdepth + 6, 16);
+  const int clo = -(1 << (col_bits - 1)), chi = (1 << (col_bits - 1)) - 1;
+  if (absi(LW - p.lh) == 1) {
+#pragma unroll
+    for (int j = 0; j < W; ++j) t[j] = mul_rnd12<NARROW>(t[j], 2896);
+  }
+  if (p.lossless) {
+    if constexpr (LW == 2) iwht4(t, 2);
+  } else {
+    const int rb = p.bitdepth + 8;
+    tx1d<NARROW, LW>(t, tx_row_kind(p.type), -(1 << (rb - 1)), (1 << (rb - 1)) - 1);
+  }
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const int r = p.lossless ? t[j] : rnd2z(t[j], p.row_shift);
+    t[j] = clampi(r, clo, chi);
+  }
+}
+
+/* Pass 1 for row `y` < 32 (rows from 32 on are zero and pass 2 does not read
+ * them): coefficients (raster, min(w,32) wide) -> tmp[y * itx_stride + j], clamped
+ * to the column range. The 32-bit arithmetic serves the rows whose coefficients
+ * lie within +-2^17, all of them in a valid stream of 8 or 10 bits (the row
+ * range of 12 bits is wider). */
 template <int LW>
 AV1B_DEV void itx_row(const ItxParams& p, const int* __restrict__ coef, int y, int* tmp) {
   constexpr int W = 1 << LW;
   constexpr int CS = W < 32 ? W : 32;
   int t[W];
-  const int col_bits = maxi(p.bitdepth + 6, 16);
-  const int clo = -(1 << (col_bits - 1)), chi = (1 << (col_bits - 1)) - 1;
-  if (y >= 32) {
-#pragma unroll
-    for (int j = 0; j < W; ++j) tmp[y * W + j] = 0;
-    return;
-  }
   const int* row = coef + y * CS;
   if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
     /* a 16-byte aligned row (every row of a raster that starts aligned):
@@ -428,57 +475,72 @@ AV1B_DEV void itx_row(const ItxParams& p, const int* __restrict__ coef, int y, i
       t[j + 2] = v.z;
       t[j + 3] = v.w;
     }
-#pragma unroll
-    for (int j = CS; j < W; ++j) t[j] = 0;
   } else {
 #pragma unroll
-    for (int j = 0; j < W; ++j) t[j] = j < CS ? row[j] : 0;
+    for (int j = 0; j < CS; ++j) t[j] = row[j];
   }
-  if (absi(LW - p.lh) == 1) {
+  unsigned size = 0;
 #pragma unroll
-    for (int j = 0; j < W; ++j) t[j] = rnd2ll((long long)t[j] * 2896, 12);
-  }
-  if (p.lossless) {
-    if constexpr (LW == 2) iwht4(t, 2);
-  } else {
-    const int rb = p.bitdepth + 8;
-    tx1d<LW>(t, tx_row_kind(p.type), -(1 << (rb - 1)), (1 << (rb - 1)) - 1);
-  }
+  for (int j = 0; j < CS; ++j) size |= static_cast<unsigned>(t[j] ^ (t[j] >> 31));
 #pragma unroll
-  for (int j = 0; j < W; ++j) {
-    const int r = p.lossless ? t[j] : rnd2z(t[j], p.row_shift);
-    tmp[y * W + j] = clampi(r, clo, chi);
-  }
+  for (int j = CS; j < W; ++j) t[j] = 0;
+  if (p.bitdepth <= 10 && size < (1u << 17))
+    itx_row_values<true, LW>(p, t);
+  else
+    itx_row_values<false, LW>(p, t);
+#pragma unroll
+  for (int j = 0; j < W; j += 4)
+    *reinterpret_cast<int4*>(tmp + y * itx_stride(LW) + j) = make_int4(t[j], t[j + 1], t[j + 2], t[j + 3]);
 }
 
-/* Pass 2 for column `x`: tmp -> residual, added to dst with the flips. */
+/* Pass 2 for column `x`: tmp -> residual, added to dst with the flips. The
+ * samples it adds to are loaded a chunk at a time, before any is stored (up
+ * to 16 rows: before the transform): the stores go to the picture the loads
+ * read, so the compiler cannot move a load above a store by itself, and a
+ * sample at a time every row waited for its own round trip. */
 template <int LH, bool CG>
 AV1B_DEV void itx_col_add(const ItxParams& p, const int* tmp, int x, px_t* dst, int stride,
                           int maxv, int* res = nullptr) {
-  constexpr int H = 1 << LH;
-  const int W = 1 << p.lw;
+  constexpr int H = 1 << LH, CH = H < 16 ? H : 16;
+  const int W = 1 << p.lw, ts = itx_stride(p.lw);
+  const bool fud = tx_flip_ud(p.type), flr = tx_flip_lr(p.type);
+  const int xx = flr ? W - 1 - x : x;
+  /* row i of the transform is row i, or H - 1 - i, of the block */
+  px_t* q = dst + (fud ? (H - 1) * stride : 0) + xx;
+  const int step = fud ? -stride : stride;
+  int old[CH];
+  const auto load = [&](int c) {
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const px_t* s = q + (c + i) * step;
+      old[i] = CG ? (int)__ldcg(s) : (int)*s;
+    }
+  };
+  if (!res && H <= 16) load(0);
   int t[H];
 #pragma unroll
-  for (int i = 0; i < H; ++i) t[i] = tmp[i * W + x];
+  for (int i = 0; i < H; ++i) t[i] = i < 32 ? tmp[i * ts + x] : 0;
   if (p.lossless) {
     if constexpr (LH == 2) iwht4(t, 0);
   } else {
+    /* pass 1 clipped to at most 18 bits: 32-bit products */
     const int cb = maxi(p.bitdepth + 6, 16);
-    tx1d<LH>(t, tx_col_kind(p.type), -(1 << (cb - 1)), (1 << (cb - 1)) - 1);
+    tx1d<true, LH>(t, tx_col_kind(p.type), -(1 << (cb - 1)), (1 << (cb - 1)) - 1);
   }
-  const bool fud = tx_flip_ud(p.type), flr = tx_flip_lr(p.type);
-  const int xx = flr ? W - 1 - x : x;
 #pragma unroll
-  for (int i = 0; i < H; ++i) {
-    const int r = p.lossless ? t[i] : rnd2(t[i], 4);
-    const int yy = fud ? H - 1 - i : i;
-    if (res) {
-      res[yy * W + xx] = r;
-      continue;
-    }
-    px_t* q = dst + yy * stride + xx;
-    const int old = CG ? (int)__ldcg(q) : (int)*q;
-    *q = (px_t)clampi(old + r, 0, maxv);
+  for (int i = 0; i < H; ++i) t[i] = p.lossless ? t[i] : rnd2(t[i], 4);
+  if (res) {
+    int* o = res + (fud ? (H - 1) * W : 0) + xx;
+    const int rs = fud ? -W : W;
+#pragma unroll
+    for (int i = 0; i < H; ++i) o[i * rs] = t[i];
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < H; c += CH) {
+    if (H > 16) load(c);
+#pragma unroll
+    for (int i = 0; i < CH; ++i) q[(c + i) * step] = (px_t)clampi(old[i] + t[c + i], 0, maxv);
   }
 }
 
@@ -505,14 +567,14 @@ AV1B_DEV void itx_col_dispatch(const ItxParams& p, const int* tmp, int x, px_t* 
 }
 
 /* The whole 2-D transform + add, by one warp. `tmp` is warp-private shared
- * memory of at least w * h ints; `dst` is the block's top-left sample. CG:
+ * memory of at least 32 * itx_stride(6) ints; `dst` is the block's top-left sample. CG:
  * read the prediction back through L2 (the dependency-scheduled kernel, where
  * neighbouring samples are written by other SMs). */
 template <bool CG>
 AV1B_DEV void itx_warp(const ItxParams& p, const int* __restrict__ coef, int* tmp, px_t* dst,
                        int stride, int maxv, int lane) {
   const int w = 1 << p.lw, h = 1 << p.lh;
-  for (int y = lane; y < h; y += 32) itx_row_dispatch(p, coef, y, tmp);
+  for (int y = lane; y < mini(h, 32); y += 32) itx_row_dispatch(p, coef, y, tmp);
   __syncwarp();
   for (int x = lane; x < w; x += 32) itx_col_dispatch<CG>(p, tmp, x, dst, stride, maxv);
   __syncwarp();
@@ -522,20 +584,7 @@ AV1B_DEV void itx_warp(const ItxParams& p, const int* __restrict__ coef, int* tm
  * index in the group), several groups - several transforms of one size class
  * - per warp. Every lane of the warp takes both barriers, active or not.
  * `res` non-null: the residual goes there (w * h, row-major) instead of into
- * the picture. */
-template <bool CG>
-AV1B_DEV void itx_group(const ItxParams& p, const int* __restrict__ coef, int* tmp, px_t* dst,
-                        int stride, int maxv, int* res, int sub, int step, bool active) {
-  const int w = 1 << p.lw, h = 1 << p.lh;
-  if (active)
-    for (int y = sub; y < h; y += step) itx_row_dispatch(p, coef, y, tmp);
-  __syncwarp();
-  if (active)
-    for (int x = sub; x < w; x += step) itx_col_dispatch<CG>(p, tmp, x, dst, stride, maxv, res);
-  __syncwarp();
-}
-
-/* The same for transforms whose longer side is 1 << CLS: only the three
+ * the picture. For transforms whose longer side is 1 << CLS: only the three
  * lengths that class holds (CLS - 2 .. CLS, the 4:1 shapes included) are
  * instantiated, so a kernel for the small classes is not sized for the
  * 64-point transforms' registers. */
@@ -572,21 +621,10 @@ AV1B_DEV void itx_group_cls(const ItxParams& p, const int* __restrict__ coef, in
   constexpr int LO = CLS - 2 > 2 ? CLS - 2 : 2;
   const int w = 1 << p.lw, h = 1 << p.lh;
   if (active)
-    for (int y = sub; y < h; y += step) itx_row_range<LO, CLS>(p, coef, y, tmp);
+    for (int y = sub; y < mini(h, 32); y += step) itx_row_range<LO, CLS>(p, coef, y, tmp);
   __syncwarp();
   if (active)
     for (int x = sub; x < w; x += step) itx_col_range<LO, CLS, CG>(p, tmp, x, dst, stride, maxv, res);
-  __syncwarp();
-}
-
-/* The 2-D transform alone: the residual (before the add and the clip) into
- * `res`, w * h row-major. */
-AV1B_DEV void itx_warp_residual(const ItxParams& p, const int* __restrict__ coef, int* tmp, int* res,
-                                int lane) {
-  const int w = 1 << p.lw, h = 1 << p.lh;
-  for (int y = lane; y < h; y += 32) itx_row_dispatch(p, coef, y, tmp);
-  __syncwarp();
-  for (int x = lane; x < w; x += 32) itx_col_dispatch<false>(p, tmp, x, nullptr, 0, 0, res);
   __syncwarp();
 }
 

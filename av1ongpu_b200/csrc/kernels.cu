@@ -621,7 +621,9 @@ cudaError_t launch_dequant(const DqRec* jobs, int n, const short* levels, const 
 template <int CLS>
 struct ItxScratch {
   static constexpr int S = 1 << (CLS < 7 ? CLS : 5);
-  static constexpr int PER_WARP = CLS >= 6 ? 4096 : 32 * S;
+  /* a transform's intermediate: at most 32 rows of the class's longest */
+  static constexpr int PER_TX = (S < 32 ? S : 32) * itx_stride(CLS < 7 ? CLS : 6);
+  static constexpr int PER_WARP = CLS >= 6 ? PER_TX : 32 / S * PER_TX;
 };
 
 /* One batch of class CLS (`bt`: first job, jobs, class) with the warp's
@@ -645,7 +647,7 @@ __device__ __forceinline__ void itx_batch(const FrameArgs& a, const int4 bt, int
     p.lossless = b.lossless;
     p.row_shift = tx.row_shift;
     p.bitdepth = a.L.bit_depth;
-    int* tmp = wsm + (S <= 32 ? g * S * S : 0);
+    int* tmp = wsm + (S <= 32 ? g * ItxScratch<CLS>::PER_TX : 0);
     const PlaneGeom& gm = a.L.p[b.plane];
     px_t* dst = a.cur + gm.off + (b.y + tx.y) * gm.stride + b.x + tx.x;
     int* res = tx.pre_off >= 0 ? a.pre_res + tx.pre_off : nullptr;
@@ -654,8 +656,13 @@ __device__ __forceinline__ void itx_batch(const FrameArgs& a, const int4 bt, int
   }
 }
 
+/* CTAs an SM of a class's kernels: the registers its transforms need with
+ * little to spare (unbounded, the compiler takes up to twice that for
+ * scheduling, and the small classes live on warps in flight). */
+constexpr int kItxCtas[8] = {0, 0, 10, 8, 5, 4, 3, 3};
+
 template <int CLS>
-__global__ void __launch_bounds__(128) k_itx(const __grid_constant__ FrameArgs a, int first,
+__global__ void __launch_bounds__(128, kItxCtas[CLS]) k_itx(const __grid_constant__ FrameArgs a, int first,
                                              int count) {
   extern __shared__ int smem[];
   const int wib = threadIdx.x >> 5;
@@ -669,7 +676,7 @@ template <int CLS>
 static cudaError_t launch_itx_class(const FrameArgs& a, cudaStream_t s) {
   const int first = a.itx_class_first[CLS], count = a.itx_class_count[CLS];
   if (count <= 0) return cudaSuccess;
-  constexpr int per_warp = CLS == 7 || CLS >= 6 ? 4096 : 32 * (1 << CLS);
+  constexpr int per_warp = ItxScratch<CLS>::PER_WARP;
   k_itx<CLS><<<(count + 3) / 4, 128, 4 * per_warp * sizeof(int), s>>>(a, first, count);
   return cudaGetLastError();
 }
@@ -2463,12 +2470,7 @@ cudaError_t set_kernel_attributes() {
       (e = cudaFuncSetAttribute(k_units<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared)) != cudaSuccess)
     return e;
-  /* the two classes whose scratch passes the 48 KB default */
-  if ((e = cudaFuncSetAttribute(k_itx<6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                4 * 4096 * (int)sizeof(int))) != cudaSuccess)
-    return e;
-  return cudaFuncSetAttribute(k_itx<7>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              4 * 4096 * (int)sizeof(int));
+  return cudaSuccess;
 }
 
 /* ---- batched form: the stage kernels of many streams ------------------------------------- */
