@@ -51,6 +51,8 @@ struct FilterArgs {
   const px_t* cdef_src;
   px_t* cdef_dst;
   const CdefRec* cdef;
+  const unsigned* cdef_cells;     /* non-null: by tiles, cdef_tx x cdef_ty x cdef_tz of them */
+  int cdef_tx, cdef_ty, cdef_tz;
   int n_cdef, cdef_grid_w, cdef_grid_n, cdef_n_grid, n_cdef_extra;
   const unsigned* cdef_extra;
   int* cdef_search;

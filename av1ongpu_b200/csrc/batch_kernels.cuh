@@ -189,10 +189,14 @@ __global__ void __launch_bounds__(128) kb_cdef_search(const StreamStep* __restri
   }
 }
 
-/* CDEF records: eight a CTA item, a half-warp each. */
-__global__ void __launch_bounds__(128) kb_cdef(const StreamStep* __restrict__ st,
+/* CDEF: a tile a CTA item, or (a stream whose blocks are off the cell grid)
+ * sixteen records, a half-warp each. */
+__global__ void __launch_bounds__(256) kb_cdef(const StreamStep* __restrict__ st,
                                                const BatchHeader* __restrict__ h) {
-  __shared__ int sw[8][12 * 12];
+  __shared__ union {
+    CdefTileSmem tile;
+    int sw[16][12 * 12];
+  } sm;
   const int hw = threadIdx.x >> 4, hl = threadIdx.x & 15;
   const unsigned hmask = 0xffffu << (threadIdx.x & 16);
   const int* pfx = h->pfx[kBCdef];
@@ -201,12 +205,20 @@ __global__ void __launch_bounds__(128) kb_cdef(const StreamStep* __restrict__ st
   for (int item = blockIdx.x; item < total; item += gridDim.x) {
     s = batch_stream_next(pfx, n, item, s);
     const FilterArgs& f = st[s].f;
-    const int ri = (item - pfx[s]) * 8 + hw;
-    if (ri < f.n_cdef) {
-      const CdefRec r = f.cdef[ri];
-      cdef_record(f.cdef_src, f.cdef_dst, r, f.cdef_search, st[s].a.L, sw[hw], hl, hmask);
+    int local = item - pfx[s];
+    if (f.cdef_cells) {
+      const int bx = local % f.cdef_tx;
+      local /= f.cdef_tx;
+      cdef_tile_item(f.cdef_src, f.cdef_dst, f.cdef_cells, f.cdef_search, f.cdef_grid_w, st[s].a.L, bx,
+                     local % f.cdef_ty, local / f.cdef_ty, sm.tile);
+    } else {
+      const int ri = local * 16 + hw;
+      if (ri < f.n_cdef) {
+        const CdefRec r = f.cdef[ri];
+        cdef_record(f.cdef_src, f.cdef_dst, r, f.cdef_search, st[s].a.L, sm.sw[hw], hl, hmask);
+      }
     }
-    __syncwarp(hmask);   /* the half-warp's window is reused by its next record */
+    __syncthreads();   /* the window is reused by the next item */
   }
 }
 
@@ -372,7 +384,7 @@ cudaError_t launch_batch_step(const StreamStep* steps, BatchHeader* hdr, const B
   mark(kBCdefSearch);
   kb_cdef_search<<<batch_grid(t, kBCdefSearch, n_sm), 128, 0, s>>>(steps, hdr);
   mark(kBCdef);
-  kb_cdef<<<batch_grid(t, kBCdef, n_sm), 128, 0, s>>>(steps, hdr);
+  kb_cdef<<<batch_grid(t, kBCdef, n_sm), 256, 0, s>>>(steps, hdr);
   mark(kBCopyPost);
   kb_copy<<<batch_grid(t, kBCopyPost, n_sm), 256, 0, s>>>(steps, hdr, 1);
   mark(kBUpscale);
@@ -437,7 +449,7 @@ int batch_stage_max_ctas(int stage) {
     case kBDeblockV: case kBDeblockH: k = reinterpret_cast<const void*>(kb_deblock); threads = 256; break;
     case kBCopySnap: case kBCopyPost: case kBCopyRef: k = reinterpret_cast<const void*>(kb_copy); threads = 256; break;
     case kBCdefSearch: k = reinterpret_cast<const void*>(kb_cdef_search); break;
-    case kBCdef: k = reinterpret_cast<const void*>(kb_cdef); break;
+    case kBCdef: k = reinterpret_cast<const void*>(kb_cdef); threads = 256; break;
     case kBUpscale: k = reinterpret_cast<const void*>(kb_upscale); threads = 128; break;
     case kBLr: k = reinterpret_cast<const void*>(kb_lr); threads = 256; break;
     case kBGrainTemplate: k = reinterpret_cast<const void*>(kb_grain_template); threads = 256; break;

@@ -25,10 +25,6 @@ int fill_filter_args(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
   const size_t pic_bytes = static_cast<size_t>(L.size) * sizeof(px_t);
   const uint8_t* ar = static_cast<const uint8_t*>(pl->arena.p);
   const uint8_t* fl = static_cast<const uint8_t*>(pl->filt.p);
-  px_t* cur = static_cast<px_t*>(d->cur.p);
-  px_t* snap = static_cast<px_t*>(d->snap.p);
-  px_t* lr_cdef = static_cast<px_t*>(d->lr_cdef.p);
-  px_t* lr_pre_up = static_cast<px_t*>(d->lr_pre_up.p);
   f.bd = pl->bit_depth;
   f.maxv = (1 << pl->bit_depth) - 1;
   f.sharpness = pl->sharpness;
@@ -42,12 +38,17 @@ int fill_filter_args(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
     f.copy_bytes[k] = static_cast<long long>(pic_bytes);
     f.copy_items[k] = static_cast<long long>((pic_bytes + AV1B_COPY_ITEM - 1) / AV1B_COPY_ITEM);
   };
-  if (P.n_cdef != 0 || P.use_lr) set_copy(0, cur, snap);
   if (P.n_cdef != 0) {
-    f.cdef_src = snap;
-    f.cdef_dst = cur;
+    if (!P.cdef_tiled) set_copy(0, sp->a.cur, sp->pre);
+    f.cdef_src = sp->pre;
+    f.cdef_dst = sp->post;
     f.cdef = reinterpret_cast<const CdefRec*>(fl + pl->o_cdef);
     f.n_cdef = static_cast<int>(P.n_cdef);
+    if (P.cdef_tiled) {
+      f.cdef_cells = reinterpret_cast<const unsigned*>(fl + pl->o_cdef_cells);
+      cdef_tile_grid(L, &f.cdef_tx, &f.cdef_ty);
+      f.cdef_tz = L.p[1].grid_w > 0 ? 2 : 1;
+    }
     f.cdef_grid_w = P.cdef_grid_w;
     f.cdef_grid_n = P.cdef_grid_n;
     f.cdef_n_grid = P.cdef_search_any ? P.cdef_grid_n : 0;
@@ -55,7 +56,8 @@ int fill_filter_args(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
     f.n_cdef_extra = static_cast<int>(P.n_cdef_search);
     f.cdef_search = static_cast<int*>(d->cdef_search.p);
   }
-  const px_t* lr_curr = snap;
+  const px_t* lr_src = sp->post;
+  const px_t* lr_curr = sp->pre;
   if (P.upscaled) {
     for (int p = 0; p < 3; ++p) superres_params(L.p[p].coded_w, L.p[p].out_w, &f.up.step[p], &f.up.initial[p]);
     auto set_pass = [&](int k, const px_t* src, px_t* dst, bool border) {
@@ -70,29 +72,27 @@ int fill_filter_args(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
       f.up_segs[k] = segs;
       f.up_items[k] = segs * (rows0 + rows1);
     };
+    px_t* up = P.use_lr ? static_cast<px_t*>(d->lr_cdef.p) : sp->out;
     if (P.use_lr) {
-      set_pass(0, snap, lr_pre_up, true);
-      set_pass(1, cur, lr_cdef, false);
-      lr_curr = lr_pre_up;
-    } else {
-      set_copy(1, cur, snap);
-      set_pass(1, snap, cur, false);
+      px_t* border = static_cast<px_t*>(d->lr_pre_up.p);
+      set_pass(0, sp->pre, border, true);
+      lr_curr = border;
+      lr_src = up;
     }
-  } else if (P.use_lr) {
-    set_copy(1, cur, lr_cdef);
+    set_pass(1, sp->post, up, false);
   }
   if (P.use_lr) {
     f.lr = P.lr;
     for (int p = 0; p < 3; ++p) f.lr.units[p] = reinterpret_cast<const LrUnitRec*>(ar + pl->o_lr[p]);
-    f.lr_cdef = lr_cdef;
+    f.lr_cdef = lr_src;
     f.lr_curr = lr_curr;
-    f.lr_dst = cur;
-    f.lr_copy_rest = P.upscaled ? 1 : 0;
+    f.lr_dst = sp->out;
+    f.lr_copy_rest = 1;
     f.lr_tiles = std::max((L.p[0].out_w + AV1B_LR_TW - 1) / AV1B_LR_TW,
                           2 * ((L.p[1].out_w + AV1B_LR_TW - 1) / AV1B_LR_TW));
     f.lr_stripes = (L.p[0].out_h + 8 + 63) / 64;
   }
-  if (sp->keep) set_copy(2, cur, static_cast<px_t*>(d->slot_buf[sp->slot].p));
+  if (sp->store) set_copy(2, sp->out, static_cast<px_t*>(d->slot_buf[sp->slot].p));
   d->disp_is_cur = true;
   d->disp_pending = false;
   if (P.grain) {
@@ -104,7 +104,7 @@ int fill_filter_args(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
     f.gp = P.gp;
     f.orbit = static_cast<const uint16_t*>(d->orbit.p);
     f.pos = static_cast<const uint16_t*>(d->pos.p);
-    f.grain_src = cur;
+    f.grain_src = sp->out;
     f.grain_dst = static_cast<px_t*>(d->disp.p);
     const int groups = std::max((L.p[0].out_w + 3) / 4, 2 * ((L.p[1].out_w + 3) / 4));
     f.grain_xblocks = (groups + 127) / 128;
@@ -282,8 +282,7 @@ int batch_step(av1b_batch* b, int n, av1b_decoder* const* decs, av1b_plan* const
       f.nv12_xblocks = static_cast<int>((pitch[i] + 8 * 128 - 1) / (8 * 128));
       f.nv12_rows = d->L.p[0].out_h + (d->L.p[0].out_h + 1) / 2;
       f.fuse_grain = f.grain && b->tuning.fuse_grain_nv12 ? 1 : 0;
-      f.nv12_src = f.fuse_grain || !f.grain ? static_cast<const px_t*>(d->cur.p)
-                                            : static_cast<const px_t*>(d->disp.p);
+      f.nv12_src = f.fuse_grain || !f.grain ? sp[i].out : static_cast<const px_t*>(d->disp.p);
       if (f.fuse_grain) d->disp_pending = true;
     }
     units_inter = units_inter || P.units_inter;
@@ -333,7 +332,7 @@ int batch_step(av1b_batch* b, int n, av1b_decoder* const* decs, av1b_plan* const
     items[kBCopyPost] = f.copy_items[1];
     items[kBCopyRef] = f.copy_items[2];
     items[kBCdefSearch] = f.n_cdef > 0 ? (f.cdef_n_grid + f.n_cdef_extra + 127) / 128 : 0;
-    items[kBCdef] = (f.n_cdef + 7) / 8;
+    items[kBCdef] = f.cdef_cells ? static_cast<long long>(f.cdef_tx) * f.cdef_ty * f.cdef_tz : (f.n_cdef + 15) / 16;
     items[kBUpscale] = f.up_items[0] + f.up_items[1];
     items[kBLr] = f.lr_tiles ? static_cast<long long>(f.lr_tiles) * f.lr_stripes * 2 : 0;
     items[kBGrainTemplate] = f.grain ? 1 : 0;

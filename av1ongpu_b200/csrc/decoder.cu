@@ -115,9 +115,12 @@ struct av1b_decoder {
   DevBuf cdef_search;             /* CDEF direction search results */
   DevBuf pre_res;                 /* phase B residuals computed ahead */
   DevBuf mask_pool;               /* difference-weighted luma masks chroma tiles read */
+  /* the last frame's picture before grain: its slot's buffer, or one of the
+   * above; its display picture is the same one (disp_is_cur) or disp */
+  const px_t* last_pic = nullptr;
   bool disp_is_cur = true;
   /* a batched step applied the last frame's film grain inside its NV12 pack:
-   * the display picture is made from cur when an output call asks for it */
+   * the display picture is made from last_pic when an output call asks for it */
   bool disp_pending = false;
   cudaEvent_t ev_batch = nullptr;   /* a batched step's wait on this decoder's stream */
   /* a batched step ran this decoder's frame on the batch's stream: the
@@ -464,6 +467,7 @@ struct Plan {
   int itx_class_first[8] = {0}, itx_class_count[8] = {0};  /* batches per class */
   int cdef_grid_w = 0, cdef_grid_n = 0;  /* the grid of 8x8 luma searches */
   bool cdef_search_any = false;          /* some record reads the grid */
+  bool cdef_tiled = false;               /* the cells describe every CDEF block */
   LrArgs lr{};
   bool use_lr = false;
   size_t coef_pool = 0, residual_pool = 0;
@@ -1895,7 +1899,7 @@ struct av1b_plan {
   size_t o_blocks = 0, o_txs = 0, o_obmc = 0, o_warps = 0, o_pal = 0, o_units = 0, o_deps = 0;
   size_t o_chains = 0;
   size_t o_tiles = 0, o_itx = 0, o_itxb = 0, o_dbv = 0, o_dbh = 0, o_cdef = 0, o_lr[3] = {0, 0, 0};
-  size_t o_map = 0, o_cdef_search = 0, o_dq = 0, o_de_raw = 0, o_cb_raw = 0, o_prep = 0;
+  size_t o_map = 0, o_cdef_search = 0, o_cdef_cells = 0, o_dq = 0, o_de_raw = 0, o_cb_raw = 0, o_prep = 0;
   size_t o_gs = 0;                /* the film grain constants and scaling tables */
   int slots_read[kSlots + 1];     /* the reference slots the frame reads, -1 ended */
   int n_blocks = 0;
@@ -2042,6 +2046,8 @@ int plan_frame(av1b_decoder* d, const av1b_frame_syntax& s, av1b_plan* pl) {
     pl->o_dbh = room(nde * sizeof(DeblockRec));
     pl->o_cdef = room(ncb * sizeof(CdefRec));
     pl->o_cdef_search = room(ncb * sizeof(unsigned));
+    const size_t cell_bytes = ncb ? 3 * static_cast<size_t>(cdef_cells(c.L)) * sizeof(unsigned) : 0;
+    pl->o_cdef_cells = room(cell_bytes);
     pl->o_prep = room(sizeof(PrepOut));
     if ((rc = dev_ensure(d, pl->filt, fo, fo + fo / 2))) {
       cudaStreamSynchronize(st);
@@ -2058,7 +2064,9 @@ int plan_frame(av1b_decoder* d, const av1b_frame_syntax& s, av1b_plan* pl) {
     if (ncb)
       CK(cudaMemcpyAsync(fl + pl->o_cb_raw, s.cdef, ncb * sizeof(av1b_cdef_block),
                          cudaMemcpyHostToDevice, st), "CDEF block upload");
-    CK(cudaMemsetAsync(fl + pl->o_prep, 0, sizeof(PrepOut), st), "count reset");
+    /* the cells lie right before the counts: one reset for both */
+    CK(cudaMemsetAsync(fl + pl->o_cdef_cells, 0, pl->o_prep + sizeof(PrepOut) - pl->o_cdef_cells, st),
+       "count reset");
     const int grid_w = c.L.p[0].stride >> 3;
     CK(launch_prep_filters(reinterpret_cast<const av1b_deblock_edge*>(fl + pl->o_de_raw),
                            static_cast<int>(nde),
@@ -2067,6 +2075,7 @@ int plan_frame(av1b_decoder* d, const av1b_frame_syntax& s, av1b_plan* pl) {
                            reinterpret_cast<DeblockRec*>(fl + pl->o_dbv),
                            reinterpret_cast<DeblockRec*>(fl + pl->o_dbh),
                            reinterpret_cast<CdefRec*>(fl + pl->o_cdef),
+                           reinterpret_cast<unsigned*>(fl + pl->o_cdef_cells),
                            reinterpret_cast<unsigned*>(fl + pl->o_cdef_search),
                            reinterpret_cast<PrepOut*>(fl + pl->o_prep), st),
        "filter record launch");
@@ -2221,6 +2230,7 @@ int plan_frame(av1b_decoder* d, const av1b_frame_syntax& s, av1b_plan* pl) {
   P.n_cdef = s.n_cdef;
   P.n_cdef_search = po.n_extra;
   P.cdef_search_any = po.any_grid != 0;
+  P.cdef_tiled = s.n_cdef > 0 && !po.irregular;
   P.R = nullptr;
   return AV1B_OK;
 }
@@ -2240,6 +2250,17 @@ struct StepPrep {
    * decode reads nothing back): the NV12 pack of the frame then applies it
    * while packing, and no display picture is written */
   bool defer_grain = false;
+  /* The pictures of the step. It is reconstructed and deblocked in a.cur;
+   * `pre` is the deblocked picture CDEF and the restoration's stripe borders
+   * read (a.cur, or its snapshot when CDEF filters a.cur in place), `post` the
+   * picture after CDEF and `out` the finished one: the destination slot's own
+   * buffer whenever a filter writes out of place, or when no block of the
+   * frame predicts from the slot's old picture; otherwise (`store`) it is
+   * copied there. */
+  px_t* pre = nullptr;
+  px_t* post = nullptr;
+  px_t* out = nullptr;
+  bool store = false;
   FrameArgs a{};
   FilterArgs f{};
 };
@@ -2299,11 +2320,10 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
   if ((P.cdef_search_any || (P.n_cdef_search != 0)) &&
       (rc = dev_ensure(d, d->cdef_search, (P.cdef_grid_n + P.n_cdef_search) * sizeof(int))))
     return rc;
-  if (P.use_lr) {
-    if ((rc = dev_ensure(d, d->lr_cdef, pic_bytes)) ||
-        (P.upscaled && (rc = dev_ensure(d, d->lr_pre_up, pic_bytes))))
-      return rc;
-  }
+  /* superres then restoration needs two pictures between them; restoration
+   * alone one more than cur and snap when the frame is not kept */
+  if (P.use_lr && (P.upscaled || !keep) && (rc = dev_ensure(d, d->lr_cdef, pic_bytes))) return rc;
+  if (P.use_lr && P.upscaled && (rc = dev_ensure(d, d->lr_pre_up, pic_bytes))) return rc;
   if (P.grain && (rc = init_grain_tables(d))) return rc;
 
   /* the plan's uploads (done when plan_frame returned; the wait orders them
@@ -2369,7 +2389,30 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
   if (!batched)   /* a batched step claims chains from its own counter */
     CK(cudaMemsetAsync(d->status_q.p, 0, sizeof(unsigned), st), "queue reset");
 
-  a.cur = static_cast<px_t*>(d->cur.p);
+  {
+    px_t* const cur = static_cast<px_t*>(d->cur.p);
+    px_t* const snap = static_cast<px_t*>(d->snap.p);
+    px_t* const kept = keep ? static_cast<px_t*>(d->slot_buf[slot].p) : nullptr;
+    bool reads_dst = false;
+    for (int i = 0; pl->slots_read[i] >= 0; ++i) reads_dst |= pl->slots_read[i] == slot;
+    const bool in_place = P.n_cdef != 0 && !P.cdef_tiled;
+    if (!P.cdef_tiled && !P.upscaled && !P.use_lr) {
+      /* nothing writes out of place: reconstructed where it stays */
+      a.cur = kept && !reads_dst ? kept : cur;
+      sp->post = sp->out = a.cur;
+      sp->store = kept && reads_dst;
+    } else {
+      a.cur = cur;
+      sp->post = in_place || P.n_cdef == 0 ? cur : (P.upscaled || P.use_lr ? snap : nullptr);
+      if (kept) sp->out = kept;
+      else if (P.upscaled) sp->out = P.use_lr || sp->post == snap ? cur : snap;
+      else if (P.use_lr) sp->out = P.n_cdef == 0 ? snap : static_cast<px_t*>(d->lr_cdef.p);
+      else sp->out = snap;
+      if (!sp->post) sp->post = sp->out;
+      sp->store = false;
+    }
+    sp->pre = in_place ? snap : a.cur;
+  }
   a.slot_ptr = static_cast<px_t* const*>(d->slot_ptr_dev.p);
   a.blocks = reinterpret_cast<const BlockRec*>(ar + pl->o_blocks);
   a.n_blocks = static_cast<int>(P.n_blocks);
@@ -2435,7 +2478,7 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
   cudaStream_t st = d->stream;
   cudaEvent_t* ev = d->ev;
   const FrameArgs& a = sp->a;
-  const int keep = sp->keep, slot = sp->slot;
+  const int slot = sp->slot;
   const size_t pic_bytes = static_cast<size_t>(L.size) * sizeof(px_t);
   uint8_t* ar = static_cast<uint8_t*>(pl->arena.p);
   int launches = 0;
@@ -2492,65 +2535,58 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
                                maxv, st);
        }), "deblock H");
   launches += ((P.n_dbv != 0)) + ((P.n_dbh != 0));
-  /* One snapshot of the deblocked picture serves CDEF (its source, CDEF
-   * writes the picture) and loop restoration (the pre-CDEF rows of its
-   * stripe boundaries); with superres the upscaled picture goes out of place
-   * into the restoration's source buffer, so it needs no snapshot of its own */
-  px_t* snap = static_cast<px_t*>(d->snap.p);
-  if ((P.n_cdef != 0) || P.use_lr)
-    CK(timed(d, kStCopy, [&] {
-         return cudaMemcpyAsync(snap, cur, pic_bytes, cudaMemcpyDeviceToDevice, st);
-       }), "deblocked snapshot");
-  if ((P.n_cdef != 0)) {
-    CK(timed(d, kStCdef, [&] {
-         return launch_cdef(snap, cur, reinterpret_cast<const CdefRec*>(fl + pl->o_cdef),
-                            static_cast<int>(P.n_cdef), P.cdef_grid_w, P.cdef_grid_n,
-                            P.cdef_search_any,
-                            reinterpret_cast<const unsigned*>(fl + pl->o_cdef_search),
-                            static_cast<int>(P.n_cdef_search),
-                            static_cast<int*>(d->cdef_search.p), L, st);
-       }), "CDEF");
+  /* CDEF by tiles filters out of place; blocks off the cell grid are
+   * filtered in place from a snapshot of the deblocked picture, which the
+   * restoration then reads the stripe borders from */
+  if (P.n_cdef != 0) {
+    int* search = static_cast<int*>(d->cdef_search.p);
+    if (P.cdef_tiled) {
+      CK(timed(d, kStCdef, [&] {
+           return launch_cdef_tiles(sp->pre, sp->post, reinterpret_cast<const unsigned*>(fl + pl->o_cdef_cells),
+                                    P.cdef_grid_w, P.cdef_grid_n, P.cdef_search_any, search, L, st);
+         }), "CDEF");
+    } else {
+      CK(timed(d, kStCopy, [&] {
+           return cudaMemcpyAsync(sp->pre, cur, pic_bytes, cudaMemcpyDeviceToDevice, st);
+         }), "deblocked snapshot");
+      CK(timed(d, kStCdef, [&] {
+           return launch_cdef(sp->pre, sp->post, reinterpret_cast<const CdefRec*>(fl + pl->o_cdef),
+                              static_cast<int>(P.n_cdef), P.cdef_grid_w, P.cdef_grid_n,
+                              P.cdef_search_any,
+                              reinterpret_cast<const unsigned*>(fl + pl->o_cdef_search),
+                              static_cast<int>(P.n_cdef_search), search, L, st);
+         }), "CDEF");
+    }
     /* the direction searches, when any record reads them, then the filter */
     launches += 1 + ((P.cdef_search_any ? P.cdef_grid_n : 0) + static_cast<int>(P.n_cdef_search) > 0);
   }
-  px_t* lr_cdef = static_cast<px_t*>(d->lr_cdef.p);
-  const px_t* lr_curr = snap;
+  const px_t* lr_src = sp->post;
+  const px_t* lr_curr = sp->pre;
   if (P.upscaled) {
+    px_t* up = P.use_lr ? static_cast<px_t*>(d->lr_cdef.p) : sp->out;
     if (P.use_lr) {
-      CK(timed(d, kStUpscale, [&] {
-           return launch_upscale(snap, static_cast<px_t*>(d->lr_pre_up.p), L, maxv, true, st);
-         }), "superres (pre-CDEF)");
-      CK(timed(d, kStUpscale, [&] { return launch_upscale(cur, lr_cdef, L, maxv, false, st); }),
-         "superres");
-      launches += 2;
-      lr_curr = static_cast<px_t*>(d->lr_pre_up.p);
-    } else {
-      CK(timed(d, kStCopy, [&] {
-           return cudaMemcpyAsync(snap, cur, pic_bytes, cudaMemcpyDeviceToDevice, st);
-         }), "superres snapshot");
-      CK(timed(d, kStUpscale, [&] { return launch_upscale(snap, cur, L, maxv, false, st); }),
-         "superres");
+      px_t* border = static_cast<px_t*>(d->lr_pre_up.p);
+      CK(timed(d, kStUpscale, [&] { return launch_upscale(sp->pre, border, L, maxv, true, st); }),
+         "superres (pre-CDEF)");
       ++launches;
+      lr_curr = border;
+      lr_src = up;
     }
-  } else if (P.use_lr) {
-    CK(timed(d, kStCopy, [&] {
-         return cudaMemcpyAsync(lr_cdef, cur, pic_bytes, cudaMemcpyDeviceToDevice, st);
-       }), "LR snapshot");
+    CK(timed(d, kStUpscale, [&] { return launch_upscale(sp->post, up, L, maxv, false, st); }), "superres");
+    ++launches;
   }
   if (P.use_lr) {
     LrArgs lr = P.lr;
     for (int p = 0; p < 3; ++p) lr.units[p] = reinterpret_cast<const LrUnitRec*>(ar + pl->o_lr[p]);
-    /* with superres the restoration's source is the upscaled picture, not
-     * the picture's own content: tiles it does not restore pass through */
-    CK(timed(d, kStLr, [&] { return launch_lr(lr_cdef, lr_curr, cur, L, lr, maxv, P.upscaled, st); }),
+    /* out of place: tiles it does not restore pass through */
+    CK(timed(d, kStLr, [&] { return launch_lr(lr_src, lr_curr, sp->out, L, lr, maxv, true, st); }),
        "loop restoration");
     ++launches;
   }
-  if (keep)
+  if (sp->store)
     CK(timed(d, kStCopy, [&] {
-         return cudaMemcpyAsync(d->slot_buf[slot].p, cur, pic_bytes, cudaMemcpyDeviceToDevice, st);
+         return cudaMemcpyAsync(d->slot_buf[slot].p, sp->out, pic_bytes, cudaMemcpyDeviceToDevice, st);
        }), "reference store");
-  const px_t* display = cur;
   d->disp_is_cur = true;
   d->disp_pending = false;
   if (P.grain) {
@@ -2560,13 +2596,12 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
       d->disp_pending = true;
     } else {
       CK(timed(d, kStGrainBlend, [&] {
-           return launch_grain_blend(cur, static_cast<px_t*>(d->disp.p), L, gsd,
+           return launch_grain_blend(sp->out, static_cast<px_t*>(d->disp.p), L, gsd,
                                      static_cast<const uint16_t*>(d->orbit.p),
                                      static_cast<const uint16_t*>(d->pos.p), st);
          }), "film grain blend");
       launches += 1;
     }
-    display = static_cast<px_t*>(d->disp.p);
     d->disp_is_cur = false;
   }
   CK(cudaEventRecord(ev[2], st), "event");
@@ -2586,8 +2621,8 @@ int commit_step(av1b_decoder* d, av1b_plan* pl, StepPrep* sp, const av1b_planes*
   const FrameArgs& a = sp->a;
   const int keep = sp->keep, slot = sp->slot;
   const int launches = sp->launches;
-  const px_t* display = d->disp_is_cur ? static_cast<const px_t*>(d->cur.p)
-                                       : static_cast<const px_t*>(d->disp.p);
+  d->last_pic = sp->out;
+  const px_t* display = d->disp_is_cur ? sp->out : static_cast<const px_t*>(d->disp.p);
 
   /* ---- read back ---------------------------------------------------------------------------- */
   if (out) {
@@ -2705,14 +2740,14 @@ int picture_of(av1b_decoder* d, int slot, const px_t** pic) {
     if (d->disp_pending) {
       /* the output picture of a frame whose grain a batched step applied
        * inside its NV12 pack: the blend from the frame's own grain state */
-      CK(launch_grain_blend(static_cast<const px_t*>(d->cur.p), static_cast<px_t*>(d->disp.p), d->L,
+      CK(launch_grain_blend(d->last_pic, static_cast<px_t*>(d->disp.p), d->L,
                             static_cast<const GrainState*>(d->grain_state.p),
                             static_cast<const uint16_t*>(d->orbit.p),
                             static_cast<const uint16_t*>(d->pos.p), d->stream),
          "film grain blend");
       d->disp_pending = false;
     }
-    *pic = d->disp_is_cur ? static_cast<const px_t*>(d->cur.p) : static_cast<const px_t*>(d->disp.p);
+    *pic = d->disp_is_cur ? d->last_pic : static_cast<const px_t*>(d->disp.p);
     return AV1B_OK;
   }
   if (slot >= kSlots || !d->slot_used[slot] || !d->slot_valid[slot])
@@ -3058,7 +3093,7 @@ size_t av1b_nv12_size(int width, int height, int ss_x, int ss_y, size_t pitch) {
 int launch_pack(av1b_decoder* d, int slot, uint8_t* target, size_t pitch) {
   if ((slot < 0 || slot == d->last_slot) && d->have_last && d->disp_pending) {
     CK(timed(d, kStNv12, [&] {
-         return launch_nv12_grain(static_cast<const px_t*>(d->cur.p), target, d->L,
+         return launch_nv12_grain(d->last_pic, target, d->L,
                                   static_cast<int>(pitch),
                                   static_cast<const GrainState*>(d->grain_state.p),
                                   static_cast<const uint16_t*>(d->orbit.p),

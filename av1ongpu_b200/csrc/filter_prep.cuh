@@ -107,10 +107,22 @@ AV1B_HD int prep_cdef(const Layout& L, const av1b_cdef_block& c, int grid_w, Cde
 /* What k_prep_filters reports back: the V and H edge counts, the searches
  * off the grid, whether any block reads the grid, and whether some record
  * was invalid. */
+/* irregular: some CDEF block is off its plane's cell grid or filters a cell
+ * another one filters too, so the cells do not describe the frame. */
 struct PrepOut {
-  unsigned n_v, n_h, n_extra, any_grid, bad;
-  unsigned pad[3];
+  unsigned n_v, n_h, n_extra, any_grid, bad, irregular;
+  unsigned pad[2];
 };
+
+/* A CDEF block as its cell's word: strengths, damping and direction (+ 2, so
+ * that 1 is a searched one); 0 is a cell no block filters. */
+AV1B_HD unsigned cdef_cell_word(const CdefRec& r) {
+  return r.pri | (r.sec << 8) | (static_cast<unsigned>(r.damping) << 16) |
+         (static_cast<unsigned>(r.dir + 2) << 24);
+}
+/* Cells of a plane: the 8x8 luma grid's, a cell being the 8x8 block, or the
+ * chroma samples it covers. */
+AV1B_HD int cdef_cells(const Layout& L) { return (L.p[0].grid_w >> 3) * (L.p[0].grid_h >> 3); }
 
 }  // namespace av1b
 

@@ -33,6 +33,9 @@ namespace av1b {
  * columns of a tile */
 #define AV1B_UP_OUT 512
 #define AV1B_LR_TW 32
+/* CDEF: samples of a plane a CTA filters */
+#define AV1B_CDEF_TW 64
+#define AV1B_CDEF_TH 32
 #define AV1B_UNIT_CTAS_PER_SM 2
 /* deblocking: the edge records a warp takes at once in the batched form and
  * in a single stream's launch */
@@ -128,8 +131,8 @@ cudaError_t launch_selftest_wait(const unsigned* flag, int* status, unsigned lon
 cudaError_t launch_recon_stage(int stage, const FrameArgs& a, int n_sm, cudaStream_t s);
 cudaError_t launch_prep_filters(const av1b_deblock_edge* edges, int n_edges, const av1b_cdef_block* cdef,
                                 int n_cdef, const Layout& L, int grid_w, int grid_n, DeblockRec* v,
-                                DeblockRec* h, CdefRec* cdef_out, unsigned* extra, PrepOut* out,
-                                cudaStream_t s);
+                                DeblockRec* h, CdefRec* cdef_out, unsigned* cells, unsigned* extra,
+                                PrepOut* out, cudaStream_t s);
 cudaError_t launch_dequant(const DqRec* jobs, int n, const short* levels, const unsigned char* qm,
                            int* coef, int bit_depth, cudaStream_t s);
 cudaError_t launch_deblock(px_t* pic, const DeblockRec* recs, int n, int sharpness, int bd,
@@ -140,6 +143,21 @@ cudaError_t launch_deblock(px_t* pic, const DeblockRec* recs, int n, int sharpne
 cudaError_t launch_cdef(const px_t* src, px_t* dst, const CdefRec* recs, int n, int grid_w,
                         int grid_n, bool grid, const unsigned* extra_pos, int n_extra, int* search,
                         const Layout& L, cudaStream_t s);
+/* CDEF by tiles, from `src` into `dst`, every sample of the planes' grids:
+ * the blocks of `cells` filtered (cdef_cell_word; three planes of cdef_cells),
+ * the rest copied. The direction searches as launch_cdef's. */
+cudaError_t launch_cdef_tiles(const px_t* src, px_t* dst, const unsigned* cells, int grid_w, int grid_n,
+                              bool grid, int* search, const Layout& L, cudaStream_t s);
+/* Tiles a picture has in a grid row of launch_cdef_tiles, and its rows: the
+ * luma plane's (z 0), or planes 1 and 2 side by side (z 1). */
+AV1B_HD void cdef_tile_grid(const Layout& L, int* tx, int* ty) {
+  const int t0 = (L.p[0].grid_w + AV1B_CDEF_TW - 1) / AV1B_CDEF_TW;
+  const int t1 = 2 * ((L.p[1].grid_w + AV1B_CDEF_TW - 1) / AV1B_CDEF_TW);
+  const int r0 = (L.p[0].grid_h + AV1B_CDEF_TH - 1) / AV1B_CDEF_TH;
+  const int r1 = (L.p[1].grid_h + AV1B_CDEF_TH - 1) / AV1B_CDEF_TH;
+  *tx = t0 > t1 ? t0 : t1;
+  *ty = r0 > r1 ? r0 : r1;
+}
 /* border_rows: only the rows within two of a loop restoration stripe
  * boundary (for the pre-CDEF picture loop restoration reads). */
 cudaError_t launch_upscale(const px_t* src, px_t* dst, const Layout& L, int maxv, bool border_rows,
