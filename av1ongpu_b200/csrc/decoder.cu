@@ -139,6 +139,7 @@ struct av1b_decoder {
   /* per-frame buffers */
   DevBuf arena, coef, residual, done, tags, status_q, nv12, rgb;
   unsigned epoch = 0;
+  unsigned queue_base = 0;        /* claims the plain phase B queue has counted */
   unsigned tag = 0;               /* the tag of the last frame's samples, 1 .. 65535 */
 
   /* film grain */
@@ -464,6 +465,7 @@ struct Plan {
    * streams' chains by it) */
   std::vector<int> depth_first;
   bool units_inter = false;       /* some phase B block is an inter kind */
+  bool itx_overlap = false;       /* some block's transforms share samples */
   int itx_class_first[8] = {0}, itx_class_count[8] = {0};  /* batches per class */
   int cdef_grid_w = 0, cdef_grid_n = 0;  /* the grid of 8x8 luma searches */
   bool cdef_search_any = false;          /* some record reads the grid */
@@ -556,9 +558,11 @@ struct BlockOut {
   int* owner[3] = {nullptr, nullptr, nullptr};
   int owner_w[3] = {0, 0, 0}, owner_h[3] = {0, 0, 0}, cell[3] = {2, 2, 2};
   uint8_t unaligned[3] = {0, 0, 0};  /* a block of the plane off its owner-cell grid */
+  bool tx_overlap = false;        /* some block's transforms share samples */
   PlanErr err;
   void clear() {
     unaligned[0] = unaligned[1] = unaligned[2] = 0;
+    tx_overlap = false;
     txs.clear();
     dq.clear();
     obmc.clear();
@@ -795,6 +799,11 @@ int plan_block(const PlanCtx& ctx, const av1b_frame_syntax& s, size_t bi, BlockR
   if (b.tx_count > 0) {
     if (b.tx_first < 0 || static_cast<size_t>(b.tx_first) + b.tx_count > s.n_transforms)
       return O->err.set(AV1B_ERR_SYNTAX, "transform range outside the frame's list");
+    /* 4x4 cells its transforms cover (rows of up to 32), where they add to
+     * the picture as they come: the size classes run side by side only in
+     * frames where no two of them write the same sample */
+    uint32_t covered[32];
+    if (!r.phase_b) std::fill(covered, covered + std::min(32, (b.h + 3) >> 2), 0u);
     for (int k = 0; k < b.tx_count; ++k) {
       const av1b_transform& t = s.transforms[b.tx_first + k];
       if (t.eob <= 0) continue;
@@ -824,6 +833,17 @@ int plan_block(const PlanCtx& ctx, const av1b_frame_syntax& s, size_t bi, BlockR
         if (ctx.levels) {
           int rc;
           if ((rc = plan_dequant(ctx, t, x, O))) return rc;
+        }
+      }
+      if (!r.phase_b && !O->tx_overlap) {
+        if (((t.x | t.y | t.w | t.h) & 3) || t.x + t.w > b.w || t.y + t.h > b.h) {
+          O->tx_overlap = true;
+        } else {
+          const uint32_t m = static_cast<uint32_t>(((1ull << (t.w >> 2)) - 1) << (t.x >> 2));
+          for (int cy = t.y >> 2; cy < (t.y + t.h) >> 2; ++cy) {
+            if (covered[cy] & m) O->tx_overlap = true;
+            covered[cy] |= m;
+          }
         }
       }
       x.pre_off = -1;
@@ -1556,6 +1576,8 @@ int build_plan(av1b_decoder* d, const PlanCtx& c, const av1b_frame_syntax& s, Pl
     });
     for (int i = 0; i < pieces; ++i)
       if (outs[i].err.code) return fail(d, outs[i].err.code, outs[i].err.msg);
+    P->itx_overlap = false;
+    for (int i = 0; i < pieces; ++i) P->itx_overlap |= outs[i].tx_overlap;
     /* later blocks overwrite earlier ones where cells overlap: a plane whose
      * blocks are not all on the cell grid is filled again, in coding order */
     S.on_grid = true;
@@ -2326,9 +2348,7 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
   if (P.use_lr && P.upscaled && (rc = dev_ensure(d, d->lr_pre_up, pic_bytes))) return rc;
   if (P.grain && (rc = init_grain_tables(d))) return rc;
 
-  /* the plan's uploads (done when plan_frame returned; the wait orders them
-   * on this stream) */
-  CK(cudaStreamWaitEvent(st, pl->ready, 0), "upload order");
+  /* the plan's uploads were done when plan_frame returned */
 
   /* slot pointer table, uploaded when a slot buffer moved */
   {
@@ -2384,10 +2404,8 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
     if ((rc = dev_ensure(d, d->status_q, 256))) return rc;
     CK(cudaMemsetAsync(d->status_q.p, 0, 256, st), "status reset");
   }
-  /* the claim counter restarts every frame; the status word is sticky until
-   * finish_frame has read it, so frames queued without a wait are covered */
-  if (!batched)   /* a batched step claims chains from its own counter */
-    CK(cudaMemsetAsync(d->status_q.p, 0, sizeof(unsigned), st), "queue reset");
+  /* the status word is sticky until finish_frame has read it, so frames
+   * queued without a wait are covered */
 
   {
     px_t* const cur = static_cast<px_t*>(d->cur.p);
@@ -2432,6 +2450,7 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
   a.deps = reinterpret_cast<const int*>(ar + pl->o_deps);
   a.units_inter = P.units_inter ? 1 : 0;
   a.queue = static_cast<unsigned*>(d->status_q.p);
+  a.queue_base = d->queue_base;   /* a batched step claims chains from its own counter */
   a.trace = nullptr;
   if (d->tracing) {
     const size_t bytes = static_cast<size_t>(pl->n_blocks) * 4 * sizeof(unsigned long long) + 64;
@@ -2441,6 +2460,8 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
     d->trace_n = static_cast<size_t>(pl->n_blocks) * 4;
   }
   a.status = reinterpret_cast<int*>(static_cast<uint8_t*>(d->status_q.p) + 64);
+  a.status_host = d->status_host;
+  a.itx_overlap = P.itx_overlap ? 1 : 0;
   a.inter_tiles = reinterpret_cast<const int2*>(ar + pl->o_tiles);
   a.n_inter_tiles = static_cast<int>(P.n_tiles);
   a.n_inter_simple = static_cast<int>(P.n_tiles_simple);
@@ -2482,21 +2503,18 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
   const size_t pic_bytes = static_cast<size_t>(L.size) * sizeof(px_t);
   uint8_t* ar = static_cast<uint8_t*>(pl->arena.p);
   int launches = 0;
-  if (P.grain) {
-    /* the grain templates depend only on the parameters: build them on the
-     * side stream while the picture is reconstructed. The fork point orders
-     * them after the previous frame's blend, which read the same state. */
-    GrainState* gsd = static_cast<GrainState*>(d->grain_state.p);
-    CK(cudaEventRecord(d->ev_fork, st), "fork");
-    CK(cudaStreamWaitEvent(d->aux, d->ev_fork, 0), "fork wait");
-    CK(timed(d, kStGrainTemplate, [&] {
-         return launch_grain_template(gsd, reinterpret_cast<const int*>(ar + pl->o_gs), P.gp,
-                                      static_cast<const uint16_t*>(d->orbit.p),
-                                      static_cast<const uint16_t*>(d->pos.p), d->aux);
-       }, d->aux), "film grain template");
-    CK(cudaEventRecord(d->ev_join, d->aux), "join");
-    ++launches;
-  }
+  /* the grain templates depend only on the parameters: one CTA beside the
+   * dependency-scheduled phase (or the last stage before it), whose kernel
+   * has let the next start. What read the state last, the previous frame's
+   * output, was complete before this frame's first kernel began. */
+  auto grain_template = [&](bool early) {
+    return timed(d, kStGrainTemplate, [&] {
+      return launch_grain_template(static_cast<GrainState*>(d->grain_state.p),
+                                   reinterpret_cast<const int*>(ar + pl->o_gs), P.gp,
+                                   static_cast<const uint16_t*>(d->orbit.p),
+                                   static_cast<const uint16_t*>(d->pos.p), early, st);
+    });
+  };
   CK(cudaEventRecord(ev[0], st), "event");
   for (int stage = 1; stage < 4; ++stage) {
     const bool any =
@@ -2510,30 +2528,43 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
      * a size class present, one dependency-scheduled kernel */
     if (stage == 1) {
       const int lm_end = a.n_inter_simple + a.n_inter_lmask, cm_first = a.n_inter_tiles - a.n_inter_cmask;
-      launches += (a.n_inter_simple > 0) + (a.n_inter_lmask > 0) + (cm_first > lm_end) + (a.n_inter_cmask > 0);
+      launches += (inter_one_launch(a, d->n_sm) ? 1 : (a.n_inter_simple > 0) + (a.n_inter_lmask > 0)) +
+                  (cm_first > lm_end) + (a.n_inter_cmask > 0);
     } else if (stage == 2) {
-      for (int c = 2; c <= 7; ++c) launches += a.itx_class_count[c] > 0;
+      if (itx_one_launch(a, d->n_sm)) ++launches;
+      else
+        for (int c = 2; c <= 7; ++c) launches += a.itx_class_count[c] > 0;
     } else {
       ++launches;
+      d->queue_base += static_cast<unsigned>(a.n_chains) + 4u * AV1B_UNIT_CTAS_PER_SM * d->n_sm;
     }
+  }
+  if (P.grain) {
+    CK(grain_template(a.n_units > 0), "film grain template");
+    ++launches;
   }
   CK(cudaEventRecord(ev[1], st), "event");
 
   /* ---- filters --------------------------------------------------------------------------- */
+  /* the first one waits for everything before it; each one after it starts
+   * early and itself waits for the one before */
+  bool early = false;
   px_t* cur = a.cur;
   const uint8_t* fl = static_cast<const uint8_t*>(pl->filt.p);
   if ((P.n_dbv != 0))
     CK(timed(d, kStDeblockV, [&] {
          return launch_deblock(cur, reinterpret_cast<const DeblockRec*>(fl + pl->o_dbv),
                                static_cast<int>(P.n_dbv), pl->sharpness, pl->bit_depth,
-                               maxv, st);
+                               maxv, early, st);
        }), "deblock V");
+  early |= P.n_dbv != 0;
   if ((P.n_dbh != 0))
     CK(timed(d, kStDeblockH, [&] {
          return launch_deblock(cur, reinterpret_cast<const DeblockRec*>(fl + pl->o_dbh),
                                static_cast<int>(P.n_dbh), pl->sharpness, pl->bit_depth,
-                               maxv, st);
+                               maxv, early, st);
        }), "deblock H");
+  early |= P.n_dbh != 0;
   launches += ((P.n_dbv != 0)) + ((P.n_dbh != 0));
   /* CDEF by tiles filters out of place; blocks off the cell grid are
    * filtered in place from a snapshot of the deblocked picture, which the
@@ -2543,7 +2574,7 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
     if (P.cdef_tiled) {
       CK(timed(d, kStCdef, [&] {
            return launch_cdef_tiles(sp->pre, sp->post, reinterpret_cast<const unsigned*>(fl + pl->o_cdef_cells),
-                                    P.cdef_grid_w, P.cdef_grid_n, P.cdef_search_any, search, L, st);
+                                    P.cdef_grid_w, P.cdef_grid_n, P.cdef_search_any, search, L, early, st);
          }), "CDEF");
     } else {
       CK(timed(d, kStCopy, [&] {
@@ -2557,6 +2588,7 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
                               static_cast<int>(P.n_cdef_search), search, L, st);
          }), "CDEF");
     }
+    early = true;
     /* the direction searches, when any record reads them, then the filter */
     launches += 1 + ((P.cdef_search_any ? P.cdef_grid_n : 0) + static_cast<int>(P.n_cdef_search) > 0);
   }
@@ -2566,20 +2598,22 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
     px_t* up = P.use_lr ? static_cast<px_t*>(d->lr_cdef.p) : sp->out;
     if (P.use_lr) {
       px_t* border = static_cast<px_t*>(d->lr_pre_up.p);
-      CK(timed(d, kStUpscale, [&] { return launch_upscale(sp->pre, border, L, maxv, true, st); }),
+      CK(timed(d, kStUpscale, [&] { return launch_upscale(sp->pre, border, L, maxv, true, early, st); }),
          "superres (pre-CDEF)");
       ++launches;
+      early = true;
       lr_curr = border;
       lr_src = up;
     }
-    CK(timed(d, kStUpscale, [&] { return launch_upscale(sp->post, up, L, maxv, false, st); }), "superres");
+    CK(timed(d, kStUpscale, [&] { return launch_upscale(sp->post, up, L, maxv, false, early, st); }), "superres");
+    early = true;
     ++launches;
   }
   if (P.use_lr) {
     LrArgs lr = P.lr;
     for (int p = 0; p < 3; ++p) lr.units[p] = reinterpret_cast<const LrUnitRec*>(ar + pl->o_lr[p]);
     /* out of place: tiles it does not restore pass through */
-    CK(timed(d, kStLr, [&] { return launch_lr(lr_src, lr_curr, sp->out, L, lr, maxv, true, st); }),
+    CK(timed(d, kStLr, [&] { return launch_lr(lr_src, lr_curr, sp->out, L, lr, maxv, true, early, st); }),
        "loop restoration");
     ++launches;
   }
@@ -2590,13 +2624,12 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
   d->disp_is_cur = true;
   d->disp_pending = false;
   if (P.grain) {
-    GrainState* gsd = static_cast<GrainState*>(d->grain_state.p);
-    CK(cudaStreamWaitEvent(st, d->ev_join, 0), "join wait");
     if (sp->defer_grain) {
       d->disp_pending = true;
     } else {
       CK(timed(d, kStGrainBlend, [&] {
-           return launch_grain_blend(sp->out, static_cast<px_t*>(d->disp.p), L, gsd,
+           return launch_grain_blend(sp->out, static_cast<px_t*>(d->disp.p), L,
+                                   static_cast<const GrainState*>(d->grain_state.p),
                                      static_cast<const uint16_t*>(d->orbit.p),
                                      static_cast<const uint16_t*>(d->pos.p), st);
          }), "film grain blend");
@@ -2618,7 +2651,6 @@ int commit_step(av1b_decoder* d, av1b_plan* pl, StepPrep* sp, const av1b_planes*
   const Layout& L = d->L;
   /* a batched step's status copy and plan event go on the batch's stream */
   cudaStream_t st = batch_stream ? batch_stream : d->stream;
-  const FrameArgs& a = sp->a;
   const int keep = sp->keep, slot = sp->slot;
   const int launches = sp->launches;
   d->last_pic = sp->out;
@@ -2636,7 +2668,6 @@ int commit_step(av1b_decoder* d, av1b_plan* pl, StepPrep* sp, const av1b_planes*
                            cudaMemcpyDeviceToHost, st), "read back");
     }
   }
-  CK(cudaMemcpyAsync(d->status_host, a.status, sizeof(int), cudaMemcpyDeviceToHost, st), "status read");
   d->stats.blocks = pl->n_blocks;
   d->stats.waves = 0;
   d->stats.kernel_launches = launches;

@@ -43,8 +43,19 @@ struct TagIo {
   unsigned long long above, left;
   int clip_w, clip_h;         /* the block's samples inside the grid */
   int* status;
+  int* status_host;           /* page-locked; null: none */
   unsigned long long limit_ns;
 };
+
+/* A wait has given up: in the status word the other waits read, and in the
+ * host's copy. */
+__device__ __forceinline__ void wait_failed(int* status, int* status_host) {
+  atomicOr(status, 1);
+  if (status_host) {
+    *reinterpret_cast<volatile int*>(status_host) = 1;
+    __threadfence_system();
+  }
+}
 
 __device__ __forceinline__ unsigned ld_tag(const unsigned* p) {
   unsigned v;
@@ -72,7 +83,7 @@ struct TagBackoff {
         if (ld_tag(reinterpret_cast<const unsigned*>(g.status)) & 1u) {
           give_up = 1;
         } else if (now - t0 > g.limit_ns) {
-          atomicOr(g.status, 1);
+          wait_failed(g.status, g.status_host);
           give_up = 1;
         }
       }
@@ -375,7 +386,7 @@ AV1B_DEV bool luma_backoff(const TagIo& g, unsigned it, unsigned long long* t0) 
     if (*t0 == 0) *t0 = now;
     if (ld_tag(reinterpret_cast<const unsigned*>(g.status)) & 1u) return false;
     if (now - *t0 > g.limit_ns) {
-      atomicOr(g.status, 1);
+      wait_failed(g.status, g.status_host);
       return false;
     }
   }

@@ -22,6 +22,8 @@
  */
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "dev_common.cuh"
 #include "dev_filters.cuh"
 #include "dev_inter.cuh"
@@ -52,6 +54,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+
+/* Programmatic dependent launch: `deps_may_start` lets the next kernel of the
+ * stream, launched with that attribute, take the SMs this one leaves;
+ * `deps_done` waits there for the kernels before it (a no-op in a kernel
+ * launched without). */
+__device__ __forceinline__ void deps_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void deps_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ const px_t* ref_plane(const FrameArgs& a, int slot, int plane) {
   const px_t* base = slot >= 0 ? a.slot_ptr[slot] : a.cur;
@@ -350,10 +359,26 @@ template <bool MASK>
 __global__ void __launch_bounds__(128, 5) k_inter_simple(const __grid_constant__ FrameArgs a, int first,
                                                       int end) {
   __shared__ McTileBuf buf[4][2];
+  deps_may_start();
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warp = first + blockIdx.x * 4 + wib;
   if (warp >= end) return;
   inter_simple_tile<MASK>(a, warp, buf[wib], lane);
+}
+
+/* Both of the lean kernel's luma-side ranges in one launch, for frames with
+ * few tiles: there the launches, not the tiles, take the time (240x136: 41 ->
+ * 27 us a frame for the stage; 360p, above the rule's line, 54 -> 39 by
+ * running the two launches side by side). */
+__global__ void __launch_bounds__(128, 5) k_inter_lean(const __grid_constant__ FrameArgs a, int n_unmasked,
+                                                       int end) {
+  __shared__ McTileBuf buf[4][2];
+  deps_may_start();
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = blockIdx.x * 4 + wib;
+  if (warp >= end) return;
+  if (warp < n_unmasked) inter_simple_tile<false>(a, warp, buf[wib], lane);
+  else inter_simple_tile<true>(a, warp, buf[wib], lane);
 }
 
 /* Inter prediction of phase A blocks: one warp per 16x8 tile. Translation
@@ -665,6 +690,7 @@ template <int CLS>
 __global__ void __launch_bounds__(128, kItxCtas[CLS]) k_itx(const __grid_constant__ FrameArgs a, int first,
                                              int count) {
   extern __shared__ int smem[];
+  deps_may_start();
   const int wib = threadIdx.x >> 5;
   const int bi = blockIdx.x * (blockDim.x >> 5) + wib;
   const int lane = threadIdx.x & 31;
@@ -672,13 +698,62 @@ __global__ void __launch_bounds__(128, kItxCtas[CLS]) k_itx(const __grid_constan
   itx_batch<CLS>(a, a.itx_batches[first + bi], smem + wib * ItxScratch<CLS>::PER_WARP, lane);
 }
 
+/* Every class in one launch, the longest transforms first (they take the
+ * longest): for frames whose batches all fit the GPU at once at this kernel's
+ * registers, the largest class's, so that the stage takes as long as its
+ * longest class instead of the sum of six launches (a 240x136 frame 37 -> 19
+ * us, 360p 47 -> 26). Larger frames launch a kernel a class, each with its own
+ * registers, side by side where no two transforms of a block share samples
+ * (1080p 65 -> 37 us, 4K 100 -> 64). */
+__global__ void __launch_bounds__(128, AV1B_ITX_ALL_CTAS) k_itx_all(const __grid_constant__ FrameArgs a, int n) {
+  extern __shared__ int smem[];
+  deps_may_start();
+  const int wib = threadIdx.x >> 5;
+  const int bi = blockIdx.x * 4 + wib;
+  const int lane = threadIdx.x & 31;
+  if (bi >= n) return;
+  const int4 bt = a.itx_batches[n - 1 - bi];
+  int* wsm = smem + wib * ItxScratch<6>::PER_WARP;
+  switch (bt.z) {
+    case 2: itx_batch<2>(a, bt, wsm, lane); break;
+    case 3: itx_batch<3>(a, bt, wsm, lane); break;
+    case 4: itx_batch<4>(a, bt, wsm, lane); break;
+    case 5: itx_batch<5>(a, bt, wsm, lane); break;
+    case 6: itx_batch<6>(a, bt, wsm, lane); break;
+    default: itx_batch<7>(a, bt, wsm, lane); break;
+  }
+}
+
+static inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
+
+/* Launches a kernel that may start once the one before it in the stream lets
+ * it (deps_may_start): one that waits for it itself (deps_done), or one that
+ * does not read what it writes. */
+template <class... P, class... A>
+static cudaError_t launch_chained(bool early, void (*k)(P...), dim3 grid, int block, size_t smem,
+                                  cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
+/* `early`: beside the class launched before it (they write other samples). */
 template <int CLS>
-static cudaError_t launch_itx_class(const FrameArgs& a, cudaStream_t s) {
+static cudaError_t launch_itx_class(const FrameArgs& a, bool* early, cudaStream_t s) {
   const int first = a.itx_class_first[CLS], count = a.itx_class_count[CLS];
   if (count <= 0) return cudaSuccess;
-  constexpr int per_warp = ItxScratch<CLS>::PER_WARP;
-  k_itx<CLS><<<(count + 3) / 4, 128, 4 * per_warp * sizeof(int), s>>>(a, first, count);
-  return cudaGetLastError();
+  constexpr size_t smem = 4 * ItxScratch<CLS>::PER_WARP * sizeof(int);
+  const cudaError_t e = launch_chained(*early, k_itx<CLS>, (count + 3) / 4, 128, smem, s, a, first, count);
+  *early = !a.itx_overlap;
+  return e;
 }
 
 /* ---- phase B -------------------------------------------------------------------------- */
@@ -713,7 +788,7 @@ __device__ __forceinline__ bool flag_seen(const unsigned* flag, unsigned want) {
  * wait has given up (AV1B_STATUS_TIMEOUT in *status), nothing waits any more:
  * the frame has failed and the kernel only has to run to its end. The status
  * word and the clock are read every 16th poll. */
-__device__ bool bounded_wait(const unsigned* flag, unsigned want, int* status,
+__device__ bool bounded_wait(const unsigned* flag, unsigned want, int* status, int* status_host,
                              unsigned long long limit_ns) {
   if (flag_seen(flag, want)) return true;
   const unsigned long long t0 = global_ns();
@@ -723,7 +798,7 @@ __device__ bool bounded_wait(const unsigned* flag, unsigned want, int* status,
     if ((it & 15) == 0) {
       if (ld_relaxed(reinterpret_cast<const unsigned*>(status)) & AV1B_STATUS_TIMEOUT) return false;
       if (global_ns() - t0 > limit_ns) {
-        atomicOr(status, AV1B_STATUS_TIMEOUT);
+        wait_failed(status, status_host);
         return false;
       }
     }
@@ -734,12 +809,12 @@ __device__ bool bounded_wait(const unsigned* flag, unsigned want, int* status,
 
 /* Waits until block `o` is reconstructed. Returns false on timeout. */
 __device__ bool wait_block(const FrameArgs& a, int o) {
-  return bounded_wait(a.done + (size_t)o * AV1B_FLAG_STRIDE, a.epoch, a.status, a.wait_ns);
+  return bounded_wait(a.done + (size_t)o * AV1B_FLAG_STRIDE, a.epoch, a.status, a.status_host, a.wait_ns);
 }
 
 /* A wait on a flag nothing sets: the failure-detection self test. */
 __global__ void k_selftest_wait(const unsigned* flag, int* status, unsigned long long limit_ns) {
-  if (threadIdx.x == 0) bounded_wait(flag, 1u, status, limit_ns);
+  if (threadIdx.x == 0) bounded_wait(flag, 1u, status, nullptr, limit_ns);
 }
 
 cudaError_t launch_selftest_wait(const unsigned* flag, int* status, unsigned long long limit_ns,
@@ -899,6 +974,7 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
         t.clip_w = mini(b.w, g.grid_w - b.x);
         t.clip_h = mini(b.h, g.grid_h - b.y);
         t.status = a.status;
+        t.status_host = a.status_host;
         t.limit_ns = a.wait_ns;
         IntraJob j;
         j.x = b.x;
@@ -969,13 +1045,16 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
 template <bool INTER>
 __global__ void __launch_bounds__(128, AV1B_UNIT_CTAS_PER_SM) k_units(const __grid_constant__ FrameArgs a) {
   extern __shared__ int smem[];
+  deps_may_start();
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int* edges = smem + wib * (3 * AV1B_EDGE_LEN + AV1B_UNIT_SCRATCH);
   int* tmp = edges + 3 * AV1B_EDGE_LEN;
   for (;;) {
     int c = 0;
-    if (lane == 0) c = atomicAdd(a.queue, 1);
+    /* every warp makes one claim past the last chain and ends: a frame adds
+     * its chains and its warps to the counter, which is never reset */
+    if (lane == 0) c = static_cast<int>(atomicAdd(a.queue, 1u) - a.queue_base);
     c = __shfl_sync(0xffffffffu, c, 0);
     if (c >= a.n_chains) break;
     run_chain<INTER>(a, c, edges, tmp, lane);
@@ -1029,6 +1108,8 @@ __device__ __forceinline__ void deblock_group(px_t* pic, const DeblockRec* recs,
 template <int G>
 __global__ void k_deblock(px_t* pic, const DeblockRec* recs, int n, int sharpness, int bd,
                           int maxv) {
+  deps_may_start();
+  deps_done();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long r0 = static_cast<long long>(warp) * G;
@@ -1138,6 +1219,8 @@ __global__ void __launch_bounds__(128) k_cdef_search(const px_t* __restrict__ sr
                                                      int grid_n, int n_grid,
                                                      const unsigned* __restrict__ pos, int n_extra,
                                                      int* out, const __grid_constant__ Layout L) {
+  deps_may_start();
+  deps_done();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n_grid + n_extra) return;
   cdef_search_one(src, grid_w, grid_n, n_grid, pos, out, L, t);
@@ -1508,6 +1591,8 @@ __global__ void __launch_bounds__(256) k_cdef_tile(const px_t* __restrict__ src,
                                                    const int* __restrict__ search, int search_w,
                                                    const __grid_constant__ Layout L) {
   __shared__ CdefTileSmem sm;
+  deps_may_start();
+  deps_done();
   cdef_tile_item(src, dst, cells, search, search_w, L, blockIdx.x, blockIdx.y, blockIdx.z, sm);
 }
 
@@ -1603,7 +1688,9 @@ __global__ void __launch_bounds__(128) k_upscale(const px_t* __restrict__ src, p
                                                 int border_rows, int rows0) {
   __shared__ __align__(16) short taps[512];
   __shared__ px_t span[AV1B_UP_SPAN];
+  deps_may_start();
   for (int i = threadIdx.x; i < 512; i += blockDim.x) taps[i] = kUpscaleFilter[i];
+  deps_done();
   upscale_item(src, dst, L, u, maxv, border_rows, rows0, blockIdx.x, blockIdx.y, taps, span);
 }
 
@@ -1884,6 +1971,8 @@ __global__ void __launch_bounds__(256) k_lr_tile(const px_t* __restrict__ cdef,
                                                  const __grid_constant__ LrArgs r, int maxv,
                                                  int copy_rest) {
   __shared__ LrSmem sm;
+  deps_may_start();
+  deps_done();
   lr_tile_item(cdef, curr, dst, L, r, maxv, copy_rest, blockIdx.x, blockIdx.y, blockIdx.z, sm);
 }
 
@@ -2459,21 +2548,31 @@ __global__ void k_rgb(const px_t* __restrict__ pic, uint8_t* out, const __grid_c
 }
 
 /* ---- launchers ------------------------------------------------------------------------------------ */
-static inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 cudaError_t launch_recon_stage(int stage, const FrameArgs& a, int n_sm, cudaStream_t s) {
   switch (stage) {
     case 1:
-      if (a.n_inter_tiles > 0)
-      {
-        if (a.n_inter_simple > 0)
-          k_inter_simple<false><<<cdiv(a.n_inter_simple, 4), 128, 0, s>>>(a, 0, a.n_inter_simple);
+      if (a.n_inter_tiles > 0) {
         const int lm_end = a.n_inter_simple + a.n_inter_lmask;
-        if (a.n_inter_lmask > 0)
-          k_inter_simple<true><<<cdiv(a.n_inter_lmask, 4), 128, 0, s>>>(a, a.n_inter_simple, lm_end);
+        const int cm_first = a.n_inter_tiles - a.n_inter_cmask;
+        /* the ranges before the last one write different samples and read
+         * only other pictures: they run side by side */
+        cudaError_t e = cudaSuccess;
+        bool early = false;
+        if (inter_one_launch(a, n_sm)) {
+          k_inter_lean<<<cdiv(lm_end, 4), 128, 0, s>>>(a, a.n_inter_simple, lm_end);
+        } else {
+          if (a.n_inter_simple > 0) {
+            k_inter_simple<false><<<cdiv(a.n_inter_simple, 4), 128, 0, s>>>(a, 0, a.n_inter_simple);
+            early = true;
+          }
+          if (a.n_inter_lmask > 0)
+            e = launch_chained(early, k_inter_simple<true>, cdiv(a.n_inter_lmask, 4), 128, 0, s, a,
+                               a.n_inter_simple, lm_end);
+        }
+        if (e != cudaSuccess) return e;
         /* the full kernel's tiles, then the chroma tiles that read the masks
          * the luma tiles wrote */
-        const int cm_first = a.n_inter_tiles - a.n_inter_cmask;
         if (cm_first > lm_end) k_inter<<<cdiv(cm_first - lm_end, 4), 128, 0, s>>>(a, lm_end, cm_first);
         if (a.n_inter_cmask > 0)
           k_inter_simple<true><<<cdiv(a.n_inter_cmask, 4), 128, 0, s>>>(a, cm_first, a.n_inter_tiles);
@@ -2481,10 +2580,19 @@ cudaError_t launch_recon_stage(int stage, const FrameArgs& a, int n_sm, cudaStre
       break;
     case 2:
       if (a.n_itx_batches > 0) {
+        if (itx_one_launch(a, n_sm)) {
+          k_itx_all<<<cdiv(a.n_itx_batches, 4), 128, 4 * ItxScratch<6>::PER_WARP * sizeof(int), s>>>(
+              a, a.n_itx_batches);
+          break;
+        }
         cudaError_t e;
-        if ((e = launch_itx_class<2>(a, s)) != cudaSuccess || (e = launch_itx_class<3>(a, s)) != cudaSuccess ||
-            (e = launch_itx_class<4>(a, s)) != cudaSuccess || (e = launch_itx_class<5>(a, s)) != cudaSuccess ||
-            (e = launch_itx_class<6>(a, s)) != cudaSuccess || (e = launch_itx_class<7>(a, s)) != cudaSuccess)
+        bool early = false;
+        if ((e = launch_itx_class<6>(a, &early, s)) != cudaSuccess ||
+            (e = launch_itx_class<5>(a, &early, s)) != cudaSuccess ||
+            (e = launch_itx_class<4>(a, &early, s)) != cudaSuccess ||
+            (e = launch_itx_class<3>(a, &early, s)) != cudaSuccess ||
+            (e = launch_itx_class<2>(a, &early, s)) != cudaSuccess ||
+            (e = launch_itx_class<7>(a, &early, s)) != cudaSuccess)
           return e;
       }
       break;
@@ -2587,11 +2695,10 @@ cudaError_t launch_prep_filters(const av1b_deblock_edge* edges, int n_edges, con
 }
 
 cudaError_t launch_deblock(px_t* pic, const DeblockRec* recs, int n, int sharpness, int bd, int maxv,
-                           cudaStream_t s) {
+                           bool early, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_deblock<AV1B_DB_PLAIN><<<cdiv(cdiv(n, AV1B_DB_PLAIN) * 32, 256), 256, 0, s>>>(pic, recs, n, sharpness, bd,
-                                                                                  maxv);
-  return cudaGetLastError();
+  const unsigned grid = cdiv(cdiv(n, AV1B_DB_PLAIN) * 32, 256);
+  return launch_chained(early, k_deblock<AV1B_DB_PLAIN>, grid, 256, 0, s, pic, recs, n, sharpness, bd, maxv);
 }
 
 cudaError_t launch_cdef(const px_t* src, px_t* dst, const CdefRec* recs, int n, int grid_w,
@@ -2607,38 +2714,41 @@ cudaError_t launch_cdef(const px_t* src, px_t* dst, const CdefRec* recs, int n, 
 }
 
 cudaError_t launch_cdef_tiles(const px_t* src, px_t* dst, const unsigned* cells, int grid_w, int grid_n,
-                              bool grid, int* search, const Layout& L, cudaStream_t s) {
-  if (grid) k_cdef_search<<<cdiv(grid_n, 128), 128, 0, s>>>(src, grid_w, grid_n, grid_n, nullptr, 0, search, L);
+                              bool grid, int* search, const Layout& L, bool early, cudaStream_t s) {
+  if (grid) {
+    const cudaError_t e = launch_chained(early, k_cdef_search, cdiv(grid_n, 128), 128, 0, s, src, grid_w, grid_n,
+                                         grid_n, nullptr, 0, search, L);
+    if (e != cudaSuccess) return e;
+    early = true;
+  }
   int tx, ty;
   cdef_tile_grid(L, &tx, &ty);
-  k_cdef_tile<<<dim3(tx, ty, L.p[1].grid_w > 0 ? 2 : 1), 256, 0, s>>>(src, dst, cells, search, grid_w, L);
-  return cudaGetLastError();
+  return launch_chained(early, k_cdef_tile, dim3(tx, ty, L.p[1].grid_w > 0 ? 2 : 1), 256, 0, s, src, dst, cells, search,
+                      grid_w, L);
 }
 
 cudaError_t launch_upscale(const px_t* src, px_t* dst, const Layout& L, int maxv, bool border_rows,
-                           cudaStream_t s) {
+                           bool early, cudaStream_t s) {
   UpscaleArgs u;
   for (int p = 0; p < 3; ++p) superres_params(L.p[p].coded_w, L.p[p].out_w, &u.step[p], &u.initial[p]);
   /* grid rows: the luma rows, then the chroma rows (planes 1 and 2 side by side) */
   const int rows0 = border_rows ? 4 * ((L.p[0].out_h + 8) / 64 + 1) : L.p[0].out_h;
   const int rows1 = L.p[1].out_h > 0 ? (border_rows ? rows0 : L.p[1].out_h) : 0;
   const int segs = maxi(cdiv(L.p[0].out_w, AV1B_UP_OUT), 2 * cdiv(L.p[1].out_w, AV1B_UP_OUT));
-  k_upscale<<<dim3(segs, rows0 + rows1), 128, 0, s>>>(src, dst, L, u, maxv, border_rows ? 1 : 0, rows0);
-  return cudaGetLastError();
+  return launch_chained(early, k_upscale, dim3(segs, rows0 + rows1), 128, 0, s, src, dst, L, u, maxv, border_rows ? 1 : 0,
+                      rows0);
 }
 
 cudaError_t launch_lr(const px_t* cdef, const px_t* curr, px_t* dst, const Layout& L,
-                      const LrArgs& r, int maxv, bool copy_rest, cudaStream_t s) {
+                      const LrArgs& r, int maxv, bool copy_rest, bool early, cudaStream_t s) {
   const int stripes = (L.p[0].out_h + 8 + 63) / 64;
   const int tiles = maxi(cdiv(L.p[0].out_w, AV1B_LR_TW), 2 * cdiv(L.p[1].out_w, AV1B_LR_TW));
-  k_lr_tile<<<dim3(tiles, stripes, 2), 256, 0, s>>>(cdef, curr, dst, L, r, maxv, copy_rest ? 1 : 0);
-  return cudaGetLastError();
+  return launch_chained(early, k_lr_tile, dim3(tiles, stripes, 2), 256, 0, s, cdef, curr, dst, L, r, maxv, copy_rest ? 1 : 0);
 }
 
 cudaError_t launch_grain_template(GrainState* gs, const int* gs_src, const GrainParamsDev& prm,
-                                  const uint16_t* orbit, const uint16_t* pos, cudaStream_t s) {
-  k_grain_template<<<1, 256, 0, s>>>(gs, gs_src, prm, orbit, pos);
-  return cudaGetLastError();
+                                  const uint16_t* orbit, const uint16_t* pos, bool early, cudaStream_t s) {
+  return launch_chained(early, k_grain_template, 1, 256, 0, s, gs, gs_src, prm, orbit, pos);
 }
 
 cudaError_t launch_grain_blend(const px_t* src, px_t* dst, const Layout& L, const GrainState* gs,
@@ -2684,6 +2794,7 @@ static cudaError_t load_all_kernels() {
   cudaError_t e;
   if ((e = load_kernel(k_inter_simple<false>)) != cudaSuccess ||
       (e = load_kernel(k_inter_simple<true>)) != cudaSuccess || (e = load_kernel(k_inter)) != cudaSuccess ||
+      (e = load_kernel(k_inter_lean)) != cudaSuccess || (e = load_kernel(k_itx_all)) != cudaSuccess ||
       (e = load_kernel(k_itx<2>)) != cudaSuccess || (e = load_kernel(k_itx<3>)) != cudaSuccess ||
       (e = load_kernel(k_itx<4>)) != cudaSuccess || (e = load_kernel(k_itx<5>)) != cudaSuccess ||
       (e = load_kernel(k_itx<6>)) != cudaSuccess || (e = load_kernel(k_itx<7>)) != cudaSuccess ||

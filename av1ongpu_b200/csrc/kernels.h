@@ -37,6 +37,11 @@ namespace av1b {
 #define AV1B_CDEF_TW 64
 #define AV1B_CDEF_TH 32
 #define AV1B_UNIT_CTAS_PER_SM 2
+/* prediction: up to this many tiles an SM, unmasked and masked ones go in one
+ * launch (16 warps an SM run at once) */
+#define AV1B_LEAN_ONE_LAUNCH 20
+/* the inverse transforms' one-launch kernel: CTAs of four warps an SM */
+#define AV1B_ITX_ALL_CTAS 3
 /* deblocking: the edge records a warp takes at once in the batched form and
  * in a single stream's launch */
 #define AV1B_DB_GROUP 8
@@ -75,7 +80,8 @@ struct FrameArgs {
   const int* deps;              /* the phase B blocks each phase B block waits for */
   int units_inter;              /* some phase B block is an inter kind */
   int n_units;
-  unsigned* queue;
+  unsigned* queue;              /* counts every claim: chain = count - queue_base */
+  unsigned queue_base;
   const int2* inter_tiles;      /* phase A: (block, x0 | y0 << 16) */
   int n_inter_tiles;
   int n_inter_simple;           /* the first ones: unmasked blocks (the lean kernel) */
@@ -89,8 +95,10 @@ struct FrameArgs {
   const int4* itx_batches;      /* (first job, jobs, log2 size class or 7 raw) */
   int n_itx_batches;
   int itx_class_first[8], itx_class_count[8];   /* the batches of each class */
+  int itx_overlap;              /* some block's transforms share samples: the classes run in order */
   int* pre_res;                 /* residuals computed ahead (TxRec::pre_off) */
   int* status;
+  int* status_host;             /* page-locked copy, set with it */
   int maxv;
   int scale_x, scale_y;
   unsigned long long wait_ns;   /* limit of one dependency wait */
@@ -125,10 +133,24 @@ struct RgbArgs {
 cudaError_t set_kernel_attributes();
 cudaError_t launch_selftest_wait(const unsigned* flag, int* status, unsigned long long limit_ns,
                                  cudaStream_t s);
+/* Whether stage 1's unmasked and masked tiles, and stage 2's classes, go in
+ * one launch. */
+inline bool inter_one_launch(const FrameArgs& a, int n_sm) {
+  const int n = a.n_inter_simple + a.n_inter_lmask;
+  return n > 0 && n <= AV1B_LEAN_ONE_LAUNCH * n_sm;
+}
+inline bool itx_one_launch(const FrameArgs& a, int n_sm) {
+  return !a.itx_overlap && a.n_itx_batches <= 4 * AV1B_ITX_ALL_CTAS * n_sm;
+}
 /* stage 1: phase A prediction; 2: the inverse transforms (phase A residual
  * added, phase B residual computed ahead); 3: the dependency-scheduled
  * phase B. */
 cudaError_t launch_recon_stage(int stage, const FrameArgs& a, int n_sm, cudaStream_t s);
+/* `early` (here and below): the kernel starts as the one launched before it
+ * drains, and waits for it to end before it reads anything. Only for a kernel
+ * that follows one which waited itself, or was launched without: the kernels
+ * before that one are then complete too. (The grain templates' kernel does not
+ * wait: it reads nothing a kernel of the frame writes.) */
 cudaError_t launch_prep_filters(const av1b_deblock_edge* edges, int n_edges, const av1b_cdef_block* cdef,
                                 int n_cdef, const Layout& L, int grid_w, int grid_n, DeblockRec* v,
                                 DeblockRec* h, CdefRec* cdef_out, unsigned* cells, unsigned* extra,
@@ -136,7 +158,7 @@ cudaError_t launch_prep_filters(const av1b_deblock_edge* edges, int n_edges, con
 cudaError_t launch_dequant(const DqRec* jobs, int n, const short* levels, const unsigned char* qm,
                            int* coef, int bit_depth, cudaStream_t s);
 cudaError_t launch_deblock(px_t* pic, const DeblockRec* recs, int n, int sharpness, int bd,
-                           int maxv, cudaStream_t s);
+                           int maxv, bool early, cudaStream_t s);
 /* CDEF: the direction searches - every 8x8 luma block of a grid_w-wide grid
  * (grid_n cells) when `grid`, then the n_extra positions off the grid (x | y
  * << 16, results after the grid's) - then the filter of every record. */
@@ -147,7 +169,7 @@ cudaError_t launch_cdef(const px_t* src, px_t* dst, const CdefRec* recs, int n, 
  * the blocks of `cells` filtered (cdef_cell_word; three planes of cdef_cells),
  * the rest copied. The direction searches as launch_cdef's. */
 cudaError_t launch_cdef_tiles(const px_t* src, px_t* dst, const unsigned* cells, int grid_w, int grid_n,
-                              bool grid, int* search, const Layout& L, cudaStream_t s);
+                              bool grid, int* search, const Layout& L, bool early, cudaStream_t s);
 /* Tiles a picture has in a grid row of launch_cdef_tiles, and its rows: the
  * luma plane's (z 0), or planes 1 and 2 side by side (z 1). */
 AV1B_HD void cdef_tile_grid(const Layout& L, int* tx, int* ty) {
@@ -161,13 +183,13 @@ AV1B_HD void cdef_tile_grid(const Layout& L, int* tx, int* ty) {
 /* border_rows: only the rows within two of a loop restoration stripe
  * boundary (for the pre-CDEF picture loop restoration reads). */
 cudaError_t launch_upscale(const px_t* src, px_t* dst, const Layout& L, int maxv, bool border_rows,
-                           cudaStream_t s);
+                           bool early, cudaStream_t s);
 cudaError_t launch_lr(const px_t* cdef, const px_t* curr, px_t* dst, const Layout& L,
-                      const LrArgs& r, int maxv, bool copy_rest, cudaStream_t s);
+                      const LrArgs& r, int maxv, bool copy_rest, bool early, cudaStream_t s);
 /* gs_src: the frame's grain constants (GrainState from `lut` on), copied into
  * `gs` beside the templates; null: `gs` holds them. */
 cudaError_t launch_grain_template(GrainState* gs, const int* gs_src, const GrainParamsDev& prm,
-                                  const uint16_t* orbit, const uint16_t* pos, cudaStream_t s);
+                                  const uint16_t* orbit, const uint16_t* pos, bool early, cudaStream_t s);
 cudaError_t launch_grain_blend(const px_t* src, px_t* dst, const Layout& L, const GrainState* gs,
                                const uint16_t* orbit, const uint16_t* pos, cudaStream_t s);
 cudaError_t launch_nv12(const px_t* pic, uint8_t* out, const Layout& L, int pitch, cudaStream_t s);
