@@ -65,17 +65,25 @@ AV1B_HD int rnd2s(int x, int n) {
  * reference uses in its scaled prediction path, av1gpu_kernels.h:81-84). */
 AV1B_HD int rnd2s_shift(int x, int n) { return (x + (1 << (n - 1)) + (x < 0 ? -1 : 0)) >> n; }
 AV1B_HD int ilog2(int v) {
+#ifdef __CUDA_ARCH__
+  return v <= 1 ? 0 : 32 - __clz(v - 1);
+#else
   int n = 0;
   while ((1 << n) < v) ++n;
   return n;
+#endif
 }
 AV1B_HD int floor_log2(int v) {
+#ifdef __CUDA_ARCH__
+  return v <= 1 ? 0 : 31 - __clz(v);
+#else
   int n = 0;
   while (v > 1) {
     v >>= 1;
     ++n;
   }
   return n;
+#endif
 }
 
 /* A sample of the picture being reconstructed, read through L2: another SM

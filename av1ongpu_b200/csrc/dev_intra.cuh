@@ -335,7 +335,8 @@ AV1B_DEV int intra_dc(const IntraJob& j, const int* above, const int* left, int 
   if (j.have_left)
     for (int k = lane; k < j.h; k += 32) s += left[k];
   s = warp_sum(s);
-  if (j.have_above && j.have_left) return (s + ((j.w + j.h) >> 1)) / (j.w + j.h);
+  if (j.have_above && j.have_left)
+    return static_cast<int>(static_cast<unsigned>(s + ((j.w + j.h) >> 1)) / static_cast<unsigned>(j.w + j.h));
   if (j.have_left) return (s + (j.h >> 1)) >> ilog2(j.h);
   if (j.have_above) return (s + (j.w >> 1)) >> ilog2(j.w);
   return 1 << (j.bitdepth - 1);
@@ -401,14 +402,16 @@ AV1B_DEV void async_copies_done() {
   __syncwarp();
 }
 
+template <class Ahead>
 AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t* luma,
                             int luma_stride, const uint8_t* palette_map,
                             const int* palette_colors, int* scratch, int lane,
-                            const TagIo& g, const int* res = nullptr, int* fi_pred = nullptr,
-                            bool res_in_flight = false) {
+                            const TagIo& g, const int* res, int* fi_pred, bool res_in_flight,
+                            Ahead&& ahead) {
   /* `res_in_flight`: the caller's residual image is still arriving by
    * asynchronous copies; it is waited for after the edges are read (the two
-   * fetches overlap), before the first sample is written */
+   * fetches overlap), before the first sample is written. `ahead`: called
+   * once the edges are there, to start loads for what comes after */
   const int w = j.w, h = j.h, n = w * h;
   const int lw = ilog2(w);
   /* the reconstructed sample: the prediction plus, when the caller fused the
@@ -420,6 +423,7 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
     if (g.write && jj < g.clip_w && i < g.clip_h) st_tag(g.write + i * g.stride + jj, g.tag | v);
   };
   if (j.palette) {
+    ahead();
     if (res_in_flight) async_copies_done();
     const uint8_t* map = palette_map + j.palette_off;
     for (int k = lane; k < n; k += 32) {
@@ -432,6 +436,7 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
   int* left = scratch + AV1B_EDGE_LEN + AV1B_EDGE_OFF;
   int* tmp = scratch + 2 * AV1B_EDGE_LEN;
   intra_edges(j, dst, stride, above, left, g, lane);
+  ahead();
   if (res_in_flight) async_copies_done();
 
   if (j.mode == 13 && fi_pred && n <= 1024) {
