@@ -413,6 +413,8 @@ struct PlanLists {
   pvec<int> chains;               /* where each chain starts in `units`, and the end */
   pvec<int> deps;                 /* per phase B block (dep_first, dep_count): the
                                      phase B blocks it waits for */
+  pvec<int4> regions;             /* FrameArgs::regions */
+  pvec<int> items;                /* the phase B blocks (their parts), region after region */
   pvec<int2> inter_tiles;
   pvec<int2> itx_jobs;            /* sorted by size class, then shape and type */
   pvec<int4> itx_batches;         /* (first job, jobs, log2 class or 7 = raw) */
@@ -437,6 +439,8 @@ void each_list(PlanLists& R, F&& f) {
   f(i++, R.itx_batches);
   for (int p = 0; p < 3; ++p) f(i++, R.lr_units[p]);
   f(i++, R.dq);
+  f(i++, R.regions);
+  f(i++, R.items);
 }
 
 /* One planned frame's constants and record counts (its records live in
@@ -465,6 +469,7 @@ struct Plan {
    * streams' chains by it) */
   std::vector<int> depth_first;
   bool units_inter = false;       /* some phase B block is an inter kind */
+  int region_log2 = 6;            /* the side of its regions */
   bool itx_overlap = false;       /* some block's transforms share samples */
   int itx_class_first[8] = {0}, itx_class_count[8] = {0};  /* batches per class */
   int cdef_grid_w = 0, cdef_grid_n = 0;  /* the grid of 8x8 luma searches */
@@ -913,6 +918,7 @@ struct PlanScratch {
   std::vector<uint64_t> head_key;
   std::vector<int> units_coding, ui_of, udepth, udeps;
   std::vector<uint8_t> is_b;
+  std::vector<int> region_of, region_level, region_count, by_depth;
   std::vector<uint8_t> flagged;       /* blocks some block waits on by done flag */
   bool on_grid = false;               /* every block lies on its plane's owner cells */
   std::vector<uint16_t> itx_key;
@@ -927,6 +933,141 @@ int pieces_for(size_t n, const PlanCtx& c, size_t min_piece) {
   return static_cast<int>(std::max<size_t>(1, std::min(most, n / min_piece)));
 }
 inline size_t piece_begin(size_t n, int pieces, int i) { return n * i / pieces; }
+
+/* The phase B blocks by regions of 1 << log2 luma samples square, for the
+ * kernel that runs a region a CTA: U, the blocks in coding order, with their dependency
+ * lists (unit indices) and depths. Regions are listed by level - one more
+ * than the deepest region a block of theirs waits for - so every region comes
+ * after those it waits for, and a region's blocks by depth, for the same
+ * reason. A large block whose samples can be predicted apart is several items
+ * of some rows each, and items in each region where several share it. Returns
+ * false, and the frame runs by larger regions or by chains, where a block that
+ * cannot be does not lie in one region, or is off the cell grid (no tagged
+ * samples), regions wait on each other in a circle, inter blocks are among
+ * them, or a palette colour could be the tiles' empty mark. */
+bool plan_regions(const PlanCtx& c, int log2, Plan* P, const std::vector<int>& U,
+                  const std::vector<int>& first, const std::vector<int>& udeps, const std::vector<int>& depth) {
+  PlanScratch& S = *c.scratch;
+  const Layout& L = c.L;
+  auto& B = P->R->blocks;
+  const size_t nu = U.size();
+  if (!S.on_grid || P->units_inter || B.size() >= (size_t(1) << AV1B_ITEM_SHIFT)) return false;
+  if (log2 > 6 && !(L.ss_x && L.ss_y)) return false;  /* the tiles would not fit an SM */
+  for (int v : P->R->palette_colors)
+    if (v < 0 || v > 4095) return false;
+  const int rw = (L.p[0].grid_w + (1 << log2) - 1) >> log2, rh = (L.p[0].grid_h + (1 << log2) - 1) >> log2;
+  std::vector<int>& of = S.region_of;  /* a block's region; -1: several */
+  std::vector<int>& level = S.region_level;
+  std::vector<int>& count = S.region_count;
+  of.resize(nu);
+  level.assign(static_cast<size_t>(rw) * rh, 0);
+  count.assign(static_cast<size_t>(rw) * rh, 0);
+  /* the regions of block u's parts, each `f(region, part)` */
+  auto each_part = [&](size_t u, auto&& f) {
+    const BlockRec& b = B[U[u]];
+    if (of[u] >= 0) {
+      for (int k = 0; k < b.parts; ++k) f(of[u], k);
+      return;
+    }
+    const int bx = log2 - (b.plane ? L.ss_x : 0), by = log2 - (b.plane ? L.ss_y : 0);
+    const int cols = std::min<int>(b.w, 1 << bx), across = b.w / cols, rows = b.h / (b.parts / across);
+    for (int k = 0; k < b.parts; ++k)
+      f(((b.y + k / across * rows) >> by) * rw + ((b.x + k % across * cols) >> bx), k);
+  };
+  for (size_t u = 0; u < nu; ++u) {
+    BlockRec& b = B[U[u]];
+    const int bx = log2 - (b.plane ? L.ss_x : 0), by = log2 - (b.plane ? L.ss_y : 0);
+    const int rx = b.x >> bx, ry = b.y >> by;
+    const int n = b.w * b.h;
+    const int rx1 = (b.x + b.w - 1) >> bx, ry1 = (b.y + b.h - 1) >> by;
+    if (b.x < 0 || b.y < 0 || rx1 >= rw || ry1 >= rh || (b.fi_mode >= 0 && n > 1024)) return false;
+    of[u] = rx1 == rx && ry1 == ry ? ry * rw + rx : -1;
+    /* in parts: not the recursive filter, nor chroma from luma (one average),
+     * nor a block that others wait for as a whole */
+    const bool apart = pow2_in(b.w, 4, 64) && pow2_in(b.h, 4, 64) && b.fuse_res &&
+                       (b.tx_count == 0 || b.res_one) && (b.palette || (b.mode != 13 && b.fi_mode < 0)) &&
+                       !(b.sync & AV1B_SYNC_FLAG);
+    int down = 1, across = 1;
+    if (apart) {
+      const int cols = std::min<int>(b.w, 1 << bx);
+      across = b.w / cols;
+      while (b.h / down > (1 << by) || b.h / down * cols > AV1B_ITEM_SAMPLES) down *= 2;
+    }
+    if (of[u] < 0 && (!apart || (across > 1 && b.x & ((1 << bx) - 1)) || b.y & (b.h / down - 1) ||
+                      (across == 1 && rx1 != rx)))
+      return false;
+    b.parts = static_cast<short>(down * across);
+    bool full = false;
+    each_part(u, [&](int r, int) { full |= ++count[r] > region_items(L, log2); });
+    if (full) return false;
+  }
+  /* one sweep in coding order gives the levels where regions are coded one
+   * after another; where they interleave, a few */
+  bool changed = true;
+  for (int sweep = 0; changed; ++sweep) {
+    if (sweep == 8) return false;
+    changed = false;
+    for (size_t u = 0; u < nu; ++u) {
+      auto raise = [&](int r, int) {
+        int l = level[r];
+        for (int j = first[u]; j < first[u + 1]; ++j) {
+          auto wait = [&](int o, int) {
+            if (o != r && level[o] >= l) l = level[o] + 1;
+          };
+          const int o = udeps[j];
+          if (of[o] >= 0) wait(of[o], 0);
+          else each_part(o, wait);
+        }
+        if (l > level[r]) {
+          level[r] = l;
+          changed = true;
+        }
+      };
+      if (of[u] >= 0) raise(of[u], 0);
+      else each_part(u, raise);
+    }
+  }
+  std::vector<int>& order = S.by_depth;
+  const size_t nr = level.size();
+  int most = 0;
+  size_t items = 0, used = 0;
+  for (size_t r = 0; r < nr; ++r) {
+    most = std::max(most, level[r]);
+    items += static_cast<size_t>(count[r]);
+    used += count[r] > 0;
+  }
+  /* the regions by level (a counting sort), their items' places */
+  std::vector<int> at(most + 2, 0);
+  for (size_t r = 0; r < nr; ++r)
+    if (count[r]) ++at[level[r] + 1];
+  for (int k = 0; k <= most; ++k) at[k + 1] += at[k];
+  sized(P->R->regions, used);
+  sized(P->R->items, items);
+  for (size_t r = 0; r < nr; ++r)
+    if (count[r])
+      P->R->regions[at[level[r]]++] = make_int4(0, count[r], static_cast<int>(r % rw), static_cast<int>(r / rw));
+  int place = 0;
+  for (int4& g : P->R->regions) {
+    g.x = place;
+    level[static_cast<size_t>(g.w) * rw + g.z] = place;
+    place += g.y;
+  }
+  /* the blocks by depth (a counting sort), into their regions */
+  int deep = 0;
+  for (size_t u = 0; u < nu; ++u) deep = std::max(deep, depth[u]);
+  at.assign(deep + 2, 0);
+  for (size_t u = 0; u < nu; ++u) ++at[depth[u] + 1];
+  for (int k = 0; k <= deep; ++k) at[k + 1] += at[k];
+  order.resize(nu);
+  for (size_t u = 0; u < nu; ++u) order[at[depth[u]]++] = static_cast<int>(u);
+  for (size_t k = 0; k < nu; ++k) {
+    const int bi = U[order[k]];
+    each_part(order[k],
+              [&](int r, int part) { P->R->items[level[r]++] = bi | part << AV1B_ITEM_SHIFT; });
+  }
+  P->region_log2 = log2;
+  return true;
+}
 
 /* The dependency-scheduled (phase B) blocks: what each waits for, and the
  * order the device claims them in.
@@ -954,6 +1095,8 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
   P->n_chains = 0;
   P->depth_first.clear();
   P->R->chains.clear();
+  P->R->regions.clear();
+  P->R->items.clear();
   if (P->R->units.empty()) return AV1B_OK;
   PlanScratch& S = *c.scratch;
   int sh[3], cw[3], ch[3];
@@ -1160,6 +1303,16 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
         }
         b.fuse_res = ok ? 1 : 0;
       }
+      if (b.kind == AV1B_U_INTRA) {
+        b.res_off = b.res_one = 0;
+        if (b.fuse_res && b.tx_count == 1) {
+          const TxRec& x = P->R->txs[b.tx_first];
+          if (x.w == b.w && x.h == b.h) {
+            b.res_one = 1;
+            b.res_off = b.residual_provided ? x.coef_off : x.pre_off;
+          }
+        }
+      }
       dep_count[ui] = static_cast<int>(mine.size());
       out.insert(out.end(), mine.begin(), mine.end());
     }
@@ -1282,6 +1435,7 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
   P->units_inter = false;
   for (int pi = 0; pi < pieces; ++pi)
     if (inter_piece[pi]) P->units_inter = true;
+  if (!plan_regions(c, 6, P, U, first, udeps, ud)) plan_regions(c, 7, P, U, first, udeps, ud);
   return AV1B_OK;
 }
 
@@ -1919,7 +2073,8 @@ struct av1b_plan {
   cudaEvent_t ready = nullptr, done = nullptr;
   bool in_flight = false;
   size_t o_blocks = 0, o_txs = 0, o_obmc = 0, o_warps = 0, o_pal = 0, o_units = 0, o_deps = 0;
-  size_t o_chains = 0;
+  size_t o_chains = 0, o_regions = 0, o_items = 0;
+  int n_regions = 0;
   size_t o_tiles = 0, o_itx = 0, o_itxb = 0, o_dbv = 0, o_dbh = 0, o_cdef = 0, o_lr[3] = {0, 0, 0};
   size_t o_map = 0, o_cdef_search = 0, o_cdef_cells = 0, o_dq = 0, o_de_raw = 0, o_cb_raw = 0, o_prep = 0;
   size_t o_gs = 0;                /* the film grain constants and scaling tables */
@@ -2157,6 +2312,9 @@ int plan_frame(av1b_decoder* d, const av1b_frame_syntax& s, av1b_plan* pl) {
   pl->o_pal = stage_put(&off, P.R->palette_colors);
   pl->o_units = stage_put(&off, P.R->units);
   pl->o_chains = stage_put(&off, P.R->chains);
+  pl->o_regions = stage_put(&off, P.R->regions);
+  pl->o_items = stage_put(&off, P.R->items);
+  pl->n_regions = static_cast<int>(P.R->regions.size());
   pl->o_deps = stage_put(&off, P.R->deps);
   pl->o_tiles = stage_put(&off, P.R->inter_tiles);
   pl->o_itx = stage_put(&off, P.R->itx_jobs);
@@ -2191,6 +2349,8 @@ int plan_frame(av1b_decoder* d, const av1b_frame_syntax& s, av1b_plan* pl) {
   CK(put(pl->o_pal, P.R->palette_colors), "record upload");
   CK(put(pl->o_units, P.R->units), "record upload");
   CK(put(pl->o_chains, P.R->chains), "record upload");
+  CK(put(pl->o_regions, P.R->regions), "record upload");
+  CK(put(pl->o_items, P.R->items), "record upload");
   CK(put(pl->o_deps, P.R->deps), "record upload");
   CK(put(pl->o_tiles, P.R->inter_tiles), "record upload");
   CK(put(pl->o_itx, P.R->itx_jobs), "record upload");
@@ -2447,6 +2607,10 @@ int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool
   a.n_units = static_cast<int>(P.n_units);
   a.chains = reinterpret_cast<const int*>(ar + pl->o_chains);
   a.n_chains = static_cast<int>(P.n_chains);
+  a.regions = reinterpret_cast<const int4*>(ar + pl->o_regions);
+  a.items = reinterpret_cast<const int*>(ar + pl->o_items);
+  a.n_regions = d->tracing ? 0 : pl->n_regions;
+  a.region_log2 = P.region_log2;
   a.deps = reinterpret_cast<const int*>(ar + pl->o_deps);
   a.units_inter = P.units_inter ? 1 : 0;
   a.queue = static_cast<unsigned*>(d->status_q.p);
@@ -2536,7 +2700,7 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
         for (int c = 2; c <= 7; ++c) launches += a.itx_class_count[c] > 0;
     } else {
       ++launches;
-      d->queue_base += static_cast<unsigned>(a.n_chains) + 4u * AV1B_UNIT_CTAS_PER_SM * d->n_sm;
+      d->queue_base += unit_claims(a, d->n_sm);
     }
   }
   if (P.grain) {

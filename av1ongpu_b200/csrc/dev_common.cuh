@@ -127,7 +127,7 @@ struct Layout {
 #define AV1B_U_INTRABC 2        /* kind: intra block copy */
 
 /* The per block record every reconstruction kernel reads. Fields a kind does
- * not use are zero. 128 bytes. */
+ * not use are zero. 120 bytes. */
 struct BlockRec {
   short x, y, w, h;           /* plane samples */
   unsigned char plane, kind, is_inter, mode;
@@ -153,7 +153,16 @@ struct BlockRec {
   unsigned char fuse_res;     /* phase B: the transforms tile disjoint parts of the
                                  block, so prediction and residual add fuse */
   int warp_idx[2];            /* into the frame's warp model table, -1 none */
-  int obmc_first, obmc_count;
+  /* an intra block of one transform of its size (phase B): res_one 1, and
+   * where its residual starts */
+  union {
+    int obmc_first;
+    int res_off;
+  };
+  union {
+    int obmc_count;
+    int res_one;
+  };
   int palette_color_idx;      /* into the palette colour table */
   int dep_first, dep_count;   /* phase B: the blocks it waits for (frame's dep list) */
   /* a difference-weighted compound: 1 - a luma block that writes its blend
@@ -161,7 +170,10 @@ struct BlockRec {
    * pool; 2 - a chroma block whose luma block is the same prediction, which
    * reads that mask instead of predicting the luma itself; 0 - neither */
   int mask_off;
-  short mask_w;
+  union {
+    short mask_w;
+    short parts;              /* phase B, an intra block: the items it is */
+  };
   unsigned char mask_role;
   unsigned char sync;         /* AV1B_SYNC_* (phase B) */
 };

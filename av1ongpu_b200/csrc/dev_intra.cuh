@@ -32,6 +32,7 @@ namespace av1b {
  * 1 << cell samples) of `cells` only - the others are final already; `luma`:
  * so are the chroma-from-luma samples. Waits give up after limit_ns or once
  * one has given up (AV1B_STATUS_TIMEOUT, bit 0 of *status). */
+#define AV1B_TILE_EMPTY 0xffffu
 struct TagIo {
   unsigned* write;
   const unsigned* at;
@@ -42,6 +43,16 @@ struct TagIo {
   int cell;
   unsigned long long above, left;
   int clip_w, clip_h;         /* the block's samples inside the grid */
+  /* The region form: the samples of the region's phase B blocks, in shared
+   * memory, tile_w a row (AV1B_TILE_EMPTY until reconstructed); tile_x and
+   * tile_y are the block's place in it. What a block waits for inside its
+   * region it reads there; the tagged words then serve other regions, which
+   * read the last row and column only. Null: no region. */
+  volatile unsigned short* tile;
+  volatile const unsigned short* luma_tile;   /* at the block's first luma sample */
+  int tile_x, tile_y, tile_w, tile_h, luma_tile_w;
+  int row0, row1;             /* the rows and columns of the block this warp */
+  int col0, cols;             /* predicts (a power of two of columns) */
   int* status;
   int* status_host;           /* page-locked; null: none */
   unsigned long long limit_ns;
@@ -66,15 +77,23 @@ __device__ __forceinline__ void st_tag(unsigned* p, unsigned v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+/* Four consecutive tagged words (16-byte aligned): one access, but each word
+ * is valid by its own tag. */
+__device__ __forceinline__ void st_tag4(unsigned* p, unsigned a, unsigned b, unsigned c, unsigned d) {
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+
 /* Between two rounds of loads of a warp whose samples have not all arrived:
- * a pause that backs off to 128 ns; every 16th round the status word and the
- * clock. Returns false when the wait has given up (the same for every lane). */
+ * a pause that backs off to `most` ns; every 128th round the status word and
+ * the clock. Returns false when the wait has given up (the same for every
+ * lane). */
 struct TagBackoff {
   unsigned it = 0, pause = 0;
   unsigned long long t0 = 0;
-  __device__ __forceinline__ bool next(const TagIo& g, int lane) {
+  __device__ __forceinline__ bool next(const TagIo& g, int lane, unsigned most) {
     ++it;
-    if ((it & 15) == 0) {
+    if ((it & 127) == 0) {
       int give_up = 0;
       if (lane == 0) {
         unsigned long long now;
@@ -90,7 +109,7 @@ struct TagBackoff {
       if (__shfl_sync(0xffffffffu, give_up, 0)) return false;
     }
     if (pause) __nanosleep(pause);
-    if (it >= 4) pause = pause < 128 ? (pause ? pause << 1 : 16) : 128;
+    if (it >= 4) pause = mini(pause ? pause << 1 : 16, most);
     return true;
   }
 };
@@ -155,30 +174,43 @@ AV1B_DEV int upsample_sel(int w, int h, int filter_type, int delta) {
  * sample of a block it waits for is loaded with its tag until the tag is this
  * frame's, any other from the picture. The wait and the read are one round
  * trip; with done flags they were a poll, then the loads, and on the writing
- * side a fence before the flag. */
+ * side a fence before the flag. A sample of the block's own region is read
+ * from the region's tile in shared memory instead. NQ: samples of each edge
+ * a lane takes (edges of up to 32 * NQ). */
+template <int NQ>
 AV1B_DEV void intra_edges_tagged(const IntraJob& j, const px_t* p, int stride, int* above, int* left,
                                  const TagIo& g, int lane) {
+  constexpr int E = 2 * NQ + 1;
   const int n = j.w + j.h;
   const int mid = 1 << (j.bitdepth - 1);
   const int alimit = mini(j.max_x, j.x + (j.have_ar ? 2 * j.w : j.w) - 1);
   const int llimit = mini(j.max_y, j.y + (j.have_bl ? 2 * j.h : j.h) - 1);
-  /* entries 2q: above, 2q + 1: left, of sample lane + 32 q; 8: the corner */
-  int v[9], o[9];
-  unsigned pend = 0;
+  /* entries 2q: above, 2q + 1: left, of sample lane + 32 q; last: the corner */
+  int v[E], o[E];
+  unsigned pend = 0, in_tile = 0;
   auto want = [&](int e, bool have, int dy, int dx, bool tagged, int none) {
     v[e] = none;
     o[e] = 0;
     if (!have) return;
-    if (tagged) {
-      o[e] = dy * g.stride + dx;
-      pend |= 1u << e;
-    } else {
+    if (!tagged) {
       v[e] = ldpx(p + dy * stride + dx);
+      return;
     }
+    pend |= 1u << e;
+    if (g.tile) {
+      const int ty = g.tile_y + dy, tx = g.tile_x + dx;
+      if (static_cast<unsigned>(ty) < static_cast<unsigned>(g.tile_h) &&
+          static_cast<unsigned>(tx) < static_cast<unsigned>(g.tile_w)) {
+        in_tile |= 1u << e;
+        o[e] = ty * g.tile_w + tx;
+        return;
+      }
+    }
+    o[e] = dy * g.stride + dx;
   };
   const bool above0 = g.above & 1, left0 = g.left & 1;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < NQ; ++q) {
     v[2 * q] = v[2 * q + 1] = o[2 * q] = o[2 * q + 1] = 0;
     const int i = lane + 32 * q;
     if (i < n) {
@@ -196,30 +228,39 @@ AV1B_DEV void intra_edges_tagged(const IntraJob& j, const px_t* p, int stride, i
       }
     }
   }
-  v[8] = mid;
-  o[8] = 0;
+  v[E - 1] = mid;
+  o[E - 1] = 0;
   if (lane == 0) {
-    if (j.have_above && j.have_left) want(8, true, -1, -1, g.corner, 0);
-    else if (j.have_above) want(8, true, -1, 0, above0, 0);
-    else want(8, j.have_left, 0, -1, left0, mid);
+    if (j.have_above && j.have_left) want(E - 1, true, -1, -1, g.corner, 0);
+    else if (j.have_above) want(E - 1, true, -1, 0, above0, 0);
+    else want(E - 1, j.have_left, 0, -1, left0, mid);
   }
   TagBackoff back;
   for (;;) {
-    unsigned w[9];
+    unsigned w[E];
 #pragma unroll
-    for (int e = 0; e < 9; ++e)
-      if (pend >> e & 1) w[e] = ld_tag(g.at + o[e]);
+    for (int e = 0; e < E; ++e)
+      if (pend >> e & 1) {
+        if (in_tile >> e & 1) {
+          const unsigned t = g.tile[o[e]];
+          w[e] = t == AV1B_TILE_EMPTY ? 0 : g.tag | t;
+        } else {
+          w[e] = ld_tag(g.at + o[e]);
+        }
+      }
 #pragma unroll
-    for (int e = 0; e < 9; ++e)
+    for (int e = 0; e < E; ++e)
       if ((pend >> e & 1) && (w[e] & 0xffff0000u) == g.tag) {
         v[e] = static_cast<int>(w[e] & 0xffffu);
         pend &= ~(1u << e);
       }
     if (!__any_sync(0xffffffffu, pend)) break;
-    if (!back.next(g, lane)) break;
+    /* short pauses once only the tile is waited for: its reads are cheap */
+    const unsigned most = __any_sync(0xffffffffu, pend & ~in_tile) ? 128 : 32;
+    if (!back.next(g, lane, most)) break;
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < NQ; ++q) {
     const int i = lane + 32 * q;
     if (i < n) {
       above[i] = v[2 * q];
@@ -227,8 +268,8 @@ AV1B_DEV void intra_edges_tagged(const IntraJob& j, const px_t* p, int stride, i
     }
   }
   if (lane == 0) {
-    above[-1] = v[8];
-    left[-1] = v[8];
+    above[-1] = v[E - 1];
+    left[-1] = v[E - 1];
   }
   __syncwarp();
 }
@@ -238,7 +279,8 @@ AV1B_DEV void intra_edges_tagged(const IntraJob& j, const px_t* p, int stride, i
 AV1B_DEV void intra_edges(const IntraJob& j, const px_t* p, int stride, int* above, int* left,
                           const TagIo& g, int lane) {
   if (g.wait) {
-    intra_edges_tagged(j, p, stride, above, left, g, lane);
+    if (j.w + j.h <= 32) intra_edges_tagged<1>(j, p, stride, above, left, g, lane);
+    else intra_edges_tagged<4>(j, p, stride, above, left, g, lane);
     return;
   }
   const int n = j.w + j.h;
@@ -281,38 +323,48 @@ AV1B_DEV void intra_edges(const IntraJob& j, const px_t* p, int stride, int* abo
 }
 
 /* The 5-tap intra edge filter over buf[-1 .. sz-2] (entry i-1 is edge sample
- * i; sample 0, the corner, is read but not written). */
-AV1B_DEV void edge_filter(int* buf, int sz, int strength, int* tmp, int lane) {
-  if (strength <= 0) return;
-  for (int i = lane; i < sz; i += 32) tmp[i] = buf[i - 1];
+ * i; sample 0, the corner, is read but not written), of both edges at once: a
+ * warp barrier serves both. Strength 0: the edge stays. */
+#define AV1B_EDGE_TMP 144
+AV1B_DEV void edge_filter(int* above, int asz, int astrength, int* left, int lsz, int lstrength, int* tmp,
+                          int lane) {
+  if ((astrength | lstrength) == 0) return;
+  if (astrength)
+    for (int i = lane; i < asz; i += 32) tmp[i] = above[i - 1];
+  if (lstrength)
+    for (int i = lane; i < lsz; i += 32) tmp[AV1B_EDGE_TMP + i] = left[i - 1];
   __syncwarp();
-  const short* k = kEdgeKernel + (strength - 1) * 5;
-  for (int i = 1 + lane; i < sz; i += 32) {
-    int s = 0;
-#pragma unroll
-    for (int t = 0; t < 5; ++t) s += k[t] * tmp[clampi(i - 2 + t, 0, sz - 1)];
-    buf[i - 1] = (s + 8) >> 4;
-  }
+  auto run = [&](int* buf, int sz, int strength, const int* t) {
+    /* kernels (0 4 8 4 0), (0 5 6 5 0), (2 4 4 4 2) */
+    const int k1 = strength == 2 ? 5 : 4, k2 = strength == 1 ? 8 : (strength == 2 ? 6 : 4);
+    const int k0 = strength == 3 ? 2 : 0;
+    for (int i = 1 + lane; i < sz; i += 32) {
+      const int s = k0 * (t[maxi(i - 2, 0)] + t[mini(i + 2, sz - 1)]) +
+                    k1 * (t[i - 1] + t[mini(i + 1, sz - 1)]) + k2 * t[i];
+      buf[i - 1] = (s + 8) >> 4;
+    }
+  };
+  if (astrength) run(above, asz, astrength, tmp);
+  if (lstrength) run(left, lsz, lstrength, tmp + AV1B_EDGE_TMP);
   __syncwarp();
 }
 
-/* Doubles the edge resolution: buf[-2 .. 2*num-2]. */
-AV1B_DEV void edge_upsample(int* buf, int num, int maxv, int* dup, int lane) {
-  /* dup[k] = buf[k-2] for k = 1..num+1, with both ends repeated */
-  for (int k = lane; k < num + 3; k += 32) {
-    int v;
-    if (k == 0) v = buf[-1];
-    else if (k == num + 2) v = buf[num - 1];
-    else v = buf[k - 2];
-    dup[k] = v;
-  }
+/* Doubles the resolution of an edge of at most 16 samples: buf[-2 .. 2*num-2].
+ * The samples pass between lanes (lane i: sample i - 1), no scratch. */
+AV1B_DEV void edge_upsample(int* buf, int num, int maxv, int lane) {
+  const int at = mini(lane, num) - 1;
+  const int v = buf[at];
+  /* of the samples -1, -1, 0, .., num - 1, num - 1: lane i has the four from
+   * its own on */
+  const int d0 = __shfl_up_sync(0xffffffffu, v, 1), d2 = __shfl_down_sync(0xffffffffu, v, 1);
+  const int d3 = __shfl_down_sync(0xffffffffu, v, 2);
   __syncwarp();
-  if (lane == 0) buf[-2] = dup[0];
-  for (int i = lane; i < num; i += 32) {
-    int s = -dup[i] + 9 * dup[i + 1] + 9 * dup[i + 2] - dup[i + 3];
-    buf[2 * i - 1] = clampi(rnd2(s, 4), 0, maxv);
-    buf[2 * i] = dup[i + 2];
+  if (lane < num) {
+    const int s = -(lane == 0 ? v : d0) + 9 * v + 9 * d2 - d3;
+    buf[2 * lane - 1] = clampi(rnd2(s, 4), 0, maxv);
+    buf[2 * lane] = d2;
   }
+  if (lane == 0) buf[-2] = v;
   __syncwarp();
 }
 
@@ -381,7 +433,7 @@ AV1B_DEV int dir_sample(const int* above, const int* left, int w, int h, int pan
 /* The pause of one lane's chroma-from-luma wait after its `it`-th round;
  * false when the wait has given up. */
 AV1B_DEV bool luma_backoff(const TagIo& g, unsigned it, unsigned long long* t0) {
-  if ((it & 15) == 15) {
+  if ((it & 127) == 127) {
     unsigned long long now;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
     if (*t0 == 0) *t0 = now;
@@ -391,7 +443,7 @@ AV1B_DEV bool luma_backoff(const TagIo& g, unsigned it, unsigned long long* t0) 
       return false;
     }
   }
-  if (it >= 3) __nanosleep(64);
+  if (it >= 3) __nanosleep(g.tile ? 32 : 64);
   return true;
 }
 
@@ -406,7 +458,7 @@ template <class Ahead>
 AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t* luma,
                             int luma_stride, const uint8_t* palette_map,
                             const int* palette_colors, int* scratch, int lane,
-                            const TagIo& g, const int* res, int* fi_pred, bool res_in_flight,
+                            const TagIo& g, const int* res, short* fi_pred, bool res_in_flight,
                             Ahead&& ahead) {
   /* `res_in_flight`: the caller's residual image is still arriving by
    * asynchronous copies; it is waited for after the edges are read (the two
@@ -417,19 +469,72 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
   /* the reconstructed sample: the prediction plus, when the caller fused the
    * residual in (`res`, the block's residual, w x h row-major), that residual,
    * clipped - what adding the transforms afterwards gives */
+  const int row0 = g.row0, col0 = g.col0, cols = g.cols, lc = ilog2(cols);
+  const int n_rows = (g.row1 - g.row0) << lc;
   auto put = [&](int i, int jj, int v) {
-    if (res) v = clampi(v + res[i * w + jj], 0, j.maxv);
+    if (res) v = clampi(v + res[(i - row0) * cols + jj - col0], 0, j.maxv);
     dst[i * stride + jj] = (px_t)v;
-    if (g.write && jj < g.clip_w && i < g.clip_h) st_tag(g.write + i * g.stride + jj, g.tag | v);
+    if (g.write && jj < g.clip_w && i < g.clip_h) {
+      if (g.tile) {
+        const int ty = g.tile_y + i, tx = g.tile_x + jj;
+        g.tile[ty * g.tile_w + tx] = static_cast<unsigned short>(v);
+        if (ty != g.tile_h - 1 && tx != g.tile_w - 1) return;
+      }
+      st_tag(g.write + i * g.stride + jj, g.tag | v);
+    }
+  };
+  /* four samples of a row at once where everything they are stored to is
+   * aligned for it (blocks lie on a grid of 4 samples; odd callers' may not) */
+  const bool vec = n_rows > 32 && cols >= 4 &&
+                   ((static_cast<unsigned>(reinterpret_cast<uintptr_t>(dst)) & 7) | (stride & 3)) == 0 &&
+                   (!g.write || ((static_cast<unsigned>(reinterpret_cast<uintptr_t>(g.write)) & 15) |
+                                 (g.stride & 3) | (g.clip_w & 3) | (g.tile ? g.tile_x & 3 : 0)) == 0);
+  auto put4 = [&](int i, int jj, int v0, int v1, int v2, int v3) {
+    if (res) {
+      const int4 r = *reinterpret_cast<const int4*>(res + (i - row0) * cols + jj - col0);
+      v0 = clampi(v0 + r.x, 0, j.maxv);
+      v1 = clampi(v1 + r.y, 0, j.maxv);
+      v2 = clampi(v2 + r.z, 0, j.maxv);
+      v3 = clampi(v3 + r.w, 0, j.maxv);
+    }
+    const uint2 two = make_uint2(static_cast<unsigned>(v0 | (v1 << 16)), static_cast<unsigned>(v2 | (v3 << 16)));
+    *reinterpret_cast<uint2*>(dst + i * stride + jj) = two;
+    if (g.write && jj < g.clip_w && i < g.clip_h) {
+      if (g.tile) {
+        const int ty = g.tile_y + i, tx = g.tile_x + jj;
+        volatile unsigned* t = reinterpret_cast<volatile unsigned*>(g.tile + ty * g.tile_w + tx);
+        t[0] = two.x;
+        t[1] = two.y;
+        if (ty != g.tile_h - 1) {
+          if (tx + 3 == g.tile_w - 1) st_tag(g.write + i * g.stride + jj + 3, g.tag | v3);
+          return;
+        }
+      }
+      st_tag4(g.write + i * g.stride + jj, g.tag | v0, g.tag | v1, g.tag | v2, g.tag | v3);
+    }
+  };
+  /* every sample the warp predicts from pred(row, column): four a lane (their
+   * loads all before the first store, which no load can be moved across) or,
+   * of up to 32 samples, one */
+  auto each = [&](auto&& pred) {
+    if (vec) {
+      for (int k = lane * 4; k < n_rows; k += 128) {
+        const int i = row0 + (k >> lc), jj = col0 + (k & (cols - 1));
+        const int v0 = pred(i, jj), v1 = pred(i, jj + 1), v2 = pred(i, jj + 2), v3 = pred(i, jj + 3);
+        put4(i, jj, v0, v1, v2, v3);
+      }
+    } else {
+      for (int k = lane; k < n_rows; k += 32) {
+        const int i = row0 + (k >> lc), jj = col0 + (k & (cols - 1));
+        put(i, jj, pred(i, jj));
+      }
+    }
   };
   if (j.palette) {
     ahead();
     if (res_in_flight) async_copies_done();
     const uint8_t* map = palette_map + j.palette_off;
-    for (int k = lane; k < n; k += 32) {
-      const int i = k >> lw, jj = k & (w - 1);
-      put(i, jj, palette_colors[map[i * j.palette_stride + jj]]);
-    }
+    each([&](int i, int jj) { return palette_colors[map[i * j.palette_stride + jj]]; });
     return;
   }
   int* above = scratch + AV1B_EDGE_OFF;
@@ -457,7 +562,19 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
       const int i = k >> lw, jj = k & (w - 1);
       const int ly = mini((j.y + i) << sy, lyl), lx = mini((j.x + jj) << sx, lxl);
       int v00, v01, v10, v11;
-      if (g.luma) {
+      if (g.luma && g.tile) {
+        volatile const unsigned short* p0 =
+            g.luma_tile + (ly - (j.y << sy)) * g.luma_tile_w + lx - (j.x << sx);
+        volatile const unsigned short* p1 = p0 + (sy ? g.luma_tile_w : 0);
+        for (unsigned it = 0;; ++it) {
+          v00 = p0[0];
+          v01 = p0[sx];
+          v10 = p1[0];
+          v11 = p1[sx];
+          if (maxi(maxi(v00, v01), maxi(v10, v11)) != static_cast<int>(AV1B_TILE_EMPTY)) break;
+          if (!luma_backoff(g, it, &luma_t0)) break;
+        }
+      } else if (g.luma) {
         const unsigned* p0 = g.luma_at + ly * g.luma_stride + lx;
         const unsigned* p1 = p0 + (sy ? g.luma_stride : 0);
         unsigned a, b, c, d;
@@ -488,17 +605,16 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
       else if (sx) t = (v00 + v01) << 2;
       else if (sy) t = (v00 + v10) << 2;
       else t = v00 << 3;
-      fi_pred[k] = t;
+      fi_pred[k] = static_cast<short>(t);   /* at most 8 * 4095 */
       sum += t;
     }
     sum = warp_sum64(sum);
     const int shift = lw + ilog2(h);
     const int avg = (int)((sum + (1LL << (shift - 1))) >> shift);
     __syncwarp();
-    for (int k = lane; k < n; k += 32) {
-      const int i = k >> lw, jj = k & (w - 1);
-      put(i, jj, clampi(dc + rnd2s(j.cfl_alpha * (fi_pred[k] - avg), 6), 0, j.maxv));
-    }
+    each([&](int i, int jj) {
+      return clampi(dc + rnd2s(j.cfl_alpha * (fi_pred[(i << lw) + jj] - avg), 6), 0, j.maxv);
+    });
     return;
   }
   if (j.mode == 13) { /* chroma from luma */
@@ -556,14 +672,11 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
         }
         int pr = 0;
         for (int t = 0; t < 7; ++t) pr += taps[pos * 7 + t] * pv[t];
-        fi_pred[((i2 << 1) + i1) * w + (j4 << 2) + j1] = clampi(rnd2(pr, 4), 0, j.maxv);
+        fi_pred[((i2 << 1) + i1) * w + (j4 << 2) + j1] = static_cast<short>(clampi(rnd2(pr, 4), 0, j.maxv));
       }
       __syncwarp();
     }
-    for (int k = lane; k < n; k += 32) {
-      const int i = k >> lw, jj = k & (w - 1);
-      put(i, jj, fi_pred[k]);
-    }
+    each([&](int i, int jj) { return static_cast<int>(fi_pred[(i << lw) + jj]); });
     return;
   }
 
@@ -580,90 +693,55 @@ AV1B_DEV void intra_predict(const IntraJob& j, px_t* dst, int stride, const px_t
         }
         __syncwarp();
       }
-      if (j.have_above) {
-        const int s = edge_strength(w, h, j.filter_type, pangle - 90);
-        const int num = mini(w, j.max_x - j.x + 1) + (pangle < 90 ? h : 0) + 1;
-        edge_filter(above, num, s, tmp, lane);
-      }
-      if (j.have_left) {
-        const int s = edge_strength(w, h, j.filter_type, pangle - 180);
-        const int num = mini(h, j.max_y - j.y + 1) + (pangle > 180 ? w : 0) + 1;
-        edge_filter(left, num, s, tmp, lane);
-      }
+      const int as = j.have_above ? edge_strength(w, h, j.filter_type, pangle - 90) : 0;
+      const int ls = j.have_left ? edge_strength(w, h, j.filter_type, pangle - 180) : 0;
+      edge_filter(above, mini(w, j.max_x - j.x + 1) + (pangle < 90 ? h : 0) + 1, as, left,
+                  mini(h, j.max_y - j.y + 1) + (pangle > 180 ? w : 0) + 1, ls, tmp, lane);
       ua = upsample_sel(w, h, j.filter_type, pangle - 90);
-      if (ua) edge_upsample(above, w + (pangle < 90 ? h : 0), j.maxv, tmp, lane);
+      if (ua) edge_upsample(above, w + (pangle < 90 ? h : 0), j.maxv, lane);
       ul = upsample_sel(w, h, j.filter_type, pangle - 180);
-      if (ul) edge_upsample(left, h + (pangle > 180 ? w : 0), j.maxv, tmp, lane);
+      if (ul) edge_upsample(left, h + (pangle > 180 ? w : 0), j.maxv, lane);
     }
     int dx = 0, dy = 0;
     if (pangle < 90) dx = kDrDeriv[pangle];
     else if (pangle > 90 && pangle < 180) dx = kDrDeriv[180 - pangle];
     if (pangle > 90 && pangle < 180) dy = kDrDeriv[pangle - 90];
     else if (pangle > 180) dy = kDrDeriv[270 - pangle];
-    for (int k = lane; k < n; k += 32) {
-      const int i = k >> lw, jj = k & (w - 1);
-      const int v = dir_sample(above, left, w, h, pangle, dx, dy, ua, ul, i, jj);
-      put(i, jj, clampi(v, 0, j.maxv));
-    }
-    return;
-  }
-  if (mode >= 9 && mode <= 11 && w >= 32) {
-    /* wide blocks: a lane keeps its column's above sample and weight and
-     * walks down the rows */
-    const int bl = left[h - 1], tr = above[w - 1];
-    for (int c = lane; c < w; c += 32) {
-      const int av = above[c], wx = sm_weight(w, c);
-      for (int i = 0; i < h; ++i) {
-        int pred;
-        if (mode == 9) {
-          const int wy = sm_weight(h, i);
-          pred = rnd2(wy * av + (256 - wy) * bl + wx * left[i] + (256 - wx) * tr, 9);
-        } else if (mode == 10) {
-          const int wy = sm_weight(h, i);
-          pred = rnd2(wy * av + (256 - wy) * bl, 8);
-        } else {
-          pred = rnd2(wx * left[i] + (256 - wx) * tr, 8);
-        }
-        put(i, c, clampi(pred, 0, j.maxv));
-      }
-    }
+    each([&](int i, int jj) {
+      return clampi(dir_sample(above, left, w, h, pangle, dx, dy, ua, ul, i, jj), 0, j.maxv);
+    });
     return;
   }
   if (mode >= 9 && mode <= 11) {
-    for (int k = lane; k < n; k += 32) {
-      const int i = k >> lw, jj = k & (w - 1);
+    const int bl = left[h - 1], tr = above[w - 1];
+    each([&](int i, int jj) {
       int pred;
       if (mode == 9) {
         const int wy = sm_weight(h, i), wx = sm_weight(w, jj);
-        pred = rnd2(wy * above[jj] + (256 - wy) * left[h - 1] + wx * left[i] +
-                        (256 - wx) * above[w - 1], 9);
+        pred = rnd2(wy * above[jj] + (256 - wy) * bl + wx * left[i] + (256 - wx) * tr, 9);
       } else if (mode == 10) {
         const int wy = sm_weight(h, i);
-        pred = rnd2(wy * above[jj] + (256 - wy) * left[h - 1], 8);
+        pred = rnd2(wy * above[jj] + (256 - wy) * bl, 8);
       } else {
         const int wx = sm_weight(w, jj);
-        pred = rnd2(wx * left[i] + (256 - wx) * above[w - 1], 8);
+        pred = rnd2(wx * left[i] + (256 - wx) * tr, 8);
       }
-      put(i, jj, clampi(pred, 0, j.maxv));
-    }
+      return clampi(pred, 0, j.maxv);
+    });
     return;
   }
   if (mode == 12) {
     const int tl = above[-1];
-    for (int k = lane; k < n; k += 32) {
-      const int i = k >> lw, jj = k & (w - 1);
+    each([&](int i, int jj) {
       const int base = above[jj] + left[i] - tl;
       const int pl = absi(base - left[i]), pt = absi(base - above[jj]), ptl = absi(base - tl);
       const int v = (pl <= pt && pl <= ptl) ? left[i] : (pt <= ptl ? above[jj] : tl);
-      put(i, jj, clampi(v, 0, j.maxv));
-    }
+      return clampi(v, 0, j.maxv);
+    });
     return;
   }
   const int dc = clampi(intra_dc(j, above, left, lane), 0, j.maxv);
-  for (int k = lane; k < n; k += 32) {
-    const int i = k >> lw, jj = k & (w - 1);
-    put(i, jj, dc);
-  }
+  each([&](int, int) { return dc; });
 }
 
 }  // namespace av1b

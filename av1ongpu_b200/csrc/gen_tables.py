@@ -91,8 +91,6 @@ for n in (4, 8, 16, 32, 64):
     sm += numbers(tables_h, r'av1g_tbl_sm_w%d\[%d\]' % (n, n), n)
 w('/* Sm_Weights_Tx_4x4 .. 64x64 back to back: size n starts at n - 4 */')
 w(emit('kSmWeights', 'short', [124], sm))
-w('/* Intra_Edge_Kernel[strength - 1][tap] */')
-w(emit('kEdgeKernel', 'short', [15], numbers(tables_h, r'av1g_tbl_edge_kernel\[3\]\[5\]', 15), storage='AV1B_CTABLE'))
 w('/* Intra_Filter_Taps[mode][position 0..7][tap 0..6] */')
 w(emit('kFilterIntraTaps', 'signed char', [280],
        numbers(tables_h, r'av1g_tbl_filter_intra\[5\]\[8\]\[7\]', 280), per_line=14))

@@ -22,6 +22,7 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <utility>
 
 #include "dev_common.cuh"
@@ -866,6 +867,95 @@ __device__ void add_residual_cg(const FrameArgs& a, const BlockRec& b, const TxR
   __syncwarp();
 }
 
+/* Starts the copies of the residual of an intra block's `rows` rows from row0
+ * and `cols` columns from col0 on into `tmp` (row-major; asynchronous,
+ * committed). The common block has one transform of its size: runs of 16-byte
+ * copies, its place in the block's record. Only such a block comes in parts. */
+__device__ __forceinline__ void fetch_residual(const FrameArgs& a, const BlockRec& b, int* tmp, int row0, int rows,
+                                               int col0, int cols, int lane) {
+  const int* pool = b.residual_provided ? a.residual : a.pre_res;
+  const int w = b.w, n = rows * cols;
+  const int* src0 = pool + b.res_off + row0 * w + col0;
+  if (b.res_one && ((cols | w) & 3) == 0 && (reinterpret_cast<uintptr_t>(src0) & 15) == 0) {
+    const int lc = ilog2(cols);
+    for (int k = lane * 4; k < n; k += 128) {
+      const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(tmp + k));
+      const int* src = src0 + (k >> lc) * w + (k & (cols - 1));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    }
+  } else {
+    for (int k = lane; k < n; k += 32) tmp[k] = 0;
+    __syncwarp();
+    for (int t = 0; t < b.tx_count; ++t) {
+      const TxRec tx = a.txs[b.tx_first + t];
+      const int* src = pool + (b.residual_provided ? tx.coef_off : tx.pre_off);
+      for (int k = lane; k < tx.w * tx.h; k += 32) {
+        const int yy = k / tx.w, xx = k - yy * tx.w;
+        const int row = tx.y + yy - row0, col = tx.x + xx - col0;
+        if (row < 0 || row >= rows || col < 0 || col >= cols) continue;
+        const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(tmp + row * cols + col));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src + k) : "memory");
+      }
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+/* An intra block's prediction job and its tagged samples (`tagged`: at its
+ * top-left sample; `write`: its samples are final as they are predicted). */
+__device__ __forceinline__ IntraJob intra_job(const FrameArgs& a, const BlockRec& b) {
+  const PlaneGeom& g = a.L.p[b.plane];
+  IntraJob j;
+  j.x = b.x;
+  j.y = b.y;
+  j.w = b.w;
+  j.h = b.h;
+  j.mode = b.mode;
+  j.angle = b.angle_delta;
+  j.bitdepth = a.L.bit_depth;
+  j.maxv = a.maxv;
+  j.have_left = b.have_left;
+  j.have_above = b.have_above;
+  j.have_ar = b.have_ar;
+  j.have_bl = b.have_bl;
+  j.filter_type = b.filter_type;
+  j.filter_intra = b.fi_mode >= 0;
+  j.fi_mode = b.fi_mode >= 0 ? b.fi_mode : 0;
+  j.cfl_alpha = b.cfl_alpha;
+  j.max_x = g.grid_w - 1;
+  j.max_y = g.grid_h - 1;
+  j.ss_x = a.L.ss_x;
+  j.ss_y = a.L.ss_y;
+  j.palette = b.palette;
+  j.palette_off = b.palette_off;
+  j.palette_stride = b.palette_stride;
+  return j;
+}
+
+__device__ __forceinline__ TagIo tag_io(const FrameArgs& a, const BlockRec& b, unsigned* tagged, bool write) {
+  const int p = b.plane;
+  const PlaneGeom& g = a.L.p[p];
+  TagIo t;
+  t.write = write ? tagged : nullptr;
+  t.at = tagged;
+  t.stride = g.grid_w;
+  t.luma_at = a.tags ? a.tags + a.tag_off[0] : nullptr;
+  t.luma_stride = a.L.p[0].grid_w;
+  t.tag = a.tag;
+  t.wait = a.tags && (b.sync & AV1B_SYNC_TAGS);
+  t.luma = a.tags && (b.sync & AV1B_SYNC_LUMA);
+  t.corner = (b.sync & AV1B_SYNC_CORNER) != 0;
+  t.cell = p == 0 ? 2 : ((p == 1 ? a.L.ss_x : a.L.ss_y) ? 1 : 2);
+  t.above = b.wait_cells[0][0] | (static_cast<unsigned long long>(b.wait_cells[0][1]) << 32);
+  t.left = b.wait_cells[1][0] | (static_cast<unsigned long long>(b.wait_cells[1][1]) << 32);
+  t.clip_w = mini(b.w, g.grid_w - b.x);
+  t.clip_h = mini(b.h, g.grid_h - b.y);
+  t.status = a.status;
+  t.status_host = a.status_host;
+  t.limit_ns = a.wait_ns;
+  return t;
+}
+
 /* INTER: the frame has phase B inter blocks (inter-intra, intra block copy);
  * a frame of intra blocks only (every key frame) runs the instantiation
  * without the inter prediction code, a much smaller kernel. */
@@ -882,11 +972,9 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
      * the kernel with inter prediction, whose registers it would spill) */
     int bi_next = a.units[a.chains[c]];
     BlockRec b_next = a.blocks[bi_next];
-    TxRec tx_next = a.txs[b_next.tx_count ? b_next.tx_first : 0];
     for (int u = a.chains[c]; u < u_end; ++u) {
       const int bi = bi_next;
       const BlockRec b = INTER ? a.blocks[bi] : b_next;
-      const TxRec tx0 = INTER ? a.txs[b.tx_count ? b.tx_first : 0] : tx_next;
       if (u + 1 < u_end) {
         bi_next = a.units[u + 1];
         if (!INTER) b_next = a.blocks[bi_next];
@@ -896,37 +984,9 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
       const bool fused = b.kind == AV1B_U_INTRA && b.fuse_res;
 
       /* the residual image, copied asynchronously: it arrives while the
-       * block waits and reads its edges (intra_predict waits for it). The
-       * common block has one transform of its size: one run of 16-byte
-       * copies; its record was loaded during the block before, so the copies
-       * start at once (behind the record's own round trip they were the last
-       * thing a step waited for: a 4K key frame's phase 4.11 -> 3.91 ms). */
+       * block waits and reads its edges (intra_predict waits for it) */
       const bool has_res = fused && b.tx_count > 0;
-      if (has_res) {
-        const int n = b.w * b.h;
-        const int* src0 = b.residual_provided ? a.residual + tx0.coef_off : a.pre_res + tx0.pre_off;
-        if (b.tx_count == 1 && tx0.w == b.w && tx0.h == b.h && (n & 3) == 0 &&
-            (reinterpret_cast<uintptr_t>(src0) & 15) == 0) {
-          for (int k = lane * 4; k < n; k += 128) {
-            const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(tmp + k));
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src0 + k) : "memory");
-          }
-        } else {
-          for (int k = lane; k < n; k += 32) tmp[k] = 0;
-          __syncwarp();
-          for (int t = 0; t < b.tx_count; ++t) {
-            const TxRec tx = a.txs[b.tx_first + t];
-            const int* src = b.residual_provided ? a.residual + tx.coef_off : a.pre_res + tx.pre_off;
-            for (int k = lane; k < tx.w * tx.h; k += 32) {
-              const int yy = k / tx.w, xx = k - yy * tx.w;
-              const unsigned d =
-                  static_cast<unsigned>(__cvta_generic_to_shared(tmp + (tx.y + yy) * b.w + tx.x + xx));
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src + k) : "memory");
-            }
-          }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-      }
+      if (has_res) fetch_residual(a, b, tmp, 0, b.h, 0, b.w, lane);
 
       /* the blocks this one reads from: each lane's acquire load of a done flag
        * orders the samples that block published before that lane's later
@@ -975,55 +1035,19 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
       unsigned* tagged = a.tags ? a.tags + a.tag_off[p] + b.y * g.grid_w + b.x : nullptr;
       const bool tag_last = tagged && !(b.kind == AV1B_U_INTRA && fused);
       if (b.kind == AV1B_U_INTRA) {
-        TagIo t;
-        t.write = tag_last ? nullptr : tagged;
-        t.at = tagged;
-        t.stride = g.grid_w;
-        t.luma_at = a.tags ? a.tags + a.tag_off[0] : nullptr;
-        t.luma_stride = a.L.p[0].grid_w;
-        t.tag = a.tag;
-        t.wait = a.tags && (b.sync & AV1B_SYNC_TAGS);
-        t.luma = a.tags && (b.sync & AV1B_SYNC_LUMA);
-        t.corner = (b.sync & AV1B_SYNC_CORNER) != 0;
-        t.cell = p == 0 ? 2 : ((p == 1 ? a.L.ss_x : a.L.ss_y) ? 1 : 2);
-        t.above = b.wait_cells[0][0] | (static_cast<unsigned long long>(b.wait_cells[0][1]) << 32);
-        t.left = b.wait_cells[1][0] | (static_cast<unsigned long long>(b.wait_cells[1][1]) << 32);
-        t.clip_w = mini(b.w, g.grid_w - b.x);
-        t.clip_h = mini(b.h, g.grid_h - b.y);
-        t.status = a.status;
-        t.status_host = a.status_host;
-        t.limit_ns = a.wait_ns;
-        IntraJob j;
-        j.x = b.x;
-        j.y = b.y;
-        j.w = b.w;
-        j.h = b.h;
-        j.mode = b.mode;
-        j.angle = b.angle_delta;
-        j.bitdepth = a.L.bit_depth;
-        j.maxv = a.maxv;
-        j.have_left = b.have_left;
-        j.have_above = b.have_above;
-        j.have_ar = b.have_ar;
-        j.have_bl = b.have_bl;
-        j.filter_type = b.filter_type;
-        j.filter_intra = b.fi_mode >= 0;
-        j.fi_mode = b.fi_mode >= 0 ? b.fi_mode : 0;
-        j.cfl_alpha = b.cfl_alpha;
-        j.max_x = g.grid_w - 1;
-        j.max_y = g.grid_h - 1;
-        j.ss_x = a.L.ss_x;
-        j.ss_y = a.L.ss_y;
-        j.palette = b.palette;
-        j.palette_off = b.palette_off;
-        j.palette_stride = b.palette_stride;
+        TagIo t = tag_io(a, b, tagged, !tag_last);
+        t.tile = nullptr;
+        t.luma_tile = nullptr;
+        t.tile_x = t.tile_y = t.tile_w = t.tile_h = t.luma_tile_w = 0;
+        t.row0 = 0;
+        t.row1 = b.h;
+        t.col0 = 0;
+        t.cols = b.w;
         /* filter intra (at most 32x32) keeps its predictions after the
          * residual image: tmp[1024 ..] */
-        intra_predict(j, dst, g.stride, a.cur + a.L.p[0].off, a.L.p[0].stride, a.palette_map,
+        intra_predict(intra_job(a, b), dst, g.stride, a.cur + a.L.p[0].off, a.L.p[0].stride, a.palette_map,
                       a.palette_colors + 8 * b.palette_color_idx, edges, lane, t,
-                      has_res ? tmp : nullptr, tmp + 1024, has_res, [&] {
-                        if (!INTER && u + 1 < u_end) tx_next = a.txs[b_next.tx_count ? b_next.tx_first : 0];
-                      });
+                      has_res ? tmp : nullptr, reinterpret_cast<short*>(tmp + 1024), has_res, [] {});
       } else if constexpr (INTER) {
         InterJob j;
         make_inter_job(a, b, &j);
@@ -1061,7 +1085,8 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
   }
 }
 
-template <bool INTER>
+/* What k_regions does not take: frames with inter blocks in phase B or with
+ * blocks off the cell grid, and traced ones. */
 __global__ void __launch_bounds__(128, AV1B_UNIT_CTAS_PER_SM) k_units(const __grid_constant__ FrameArgs a) {
   extern __shared__ int smem[];
   deps_may_start();
@@ -1076,7 +1101,155 @@ __global__ void __launch_bounds__(128, AV1B_UNIT_CTAS_PER_SM) k_units(const __gr
     if (lane == 0) c = static_cast<int>(atomicAdd(a.queue, 1u) - a.queue_base);
     c = __shfl_sync(0xffffffffu, c, 0);
     if (c >= a.n_chains) break;
-    run_chain<INTER>(a, c, edges, tmp, lane);
+    run_chain<true>(a, c, edges, tmp, lane);
+  }
+}
+
+/* Phase B by regions: a CTA claims a region of 64x64 or 128x128 luma samples
+ * (in an order in which every region comes after those its blocks wait for)
+ * and its warps claim the region's items in order of dependency depth, so
+ * every wait is on an item claimed before and the earliest unfinished item
+ * always progresses. The path through a frame is a chain of small blocks, most
+ * of them neighbours: a step through the tagged words in L2 took a store and a
+ * polled load (about 1 us of the 2.0 us step of a 4x4 block) where two blocks
+ * of a region now hand their samples over in shared memory. A block of more
+ * than AV1B_ITEM_SAMPLES samples is several items of some rows each, and one
+ * that several regions share is items in each; they gather its edges each for
+ * themselves. (One warp alone took 21 us for a 64x64 block.) An item's record
+ * is loaded while the one before it is predicted. Key frames, a pass: 720p
+ * 1,128 -> 585 us, 1080p 2,170 -> 1,360, 4K 3,838 -> 2,455. */
+struct RegionSmem {
+  static constexpr int PER_WARP = 3 * AV1B_EDGE_LEN + AV1B_REGION_SCRATCH;   /* ints */
+  int warp[AV1B_REGION_WARPS][PER_WARP];
+  BlockRec rec[AV1B_REGION_WARPS];
+  int region, next, pad[2];
+};
+
+/* then the tiles, and the items */
+static size_t region_smem(const Layout& L, int log2) {
+  return sizeof(RegionSmem) + region_samples(L, log2) * sizeof(px_t) + region_items(L, log2) * sizeof(int);
+}
+
+/* Its CTAs: as many as an SM's shared memory holds, but one on one SM, where
+ * the grain templates' CTA runs beside them. */
+static int region_ctas(const FrameArgs& a, int n_sm) {
+  const int fit = 2 * (region_smem(a.L, a.region_log2) + 1024) <= 228 * 1024 ? 2 * n_sm - 1 : n_sm;
+  return a.n_regions < fit ? a.n_regions : fit;
+}
+unsigned unit_claims(const FrameArgs& a, int n_sm) {
+  return units_by_region(a) ? static_cast<unsigned>(a.n_regions + region_ctas(a, n_sm))
+                            : static_cast<unsigned>(a.n_chains) + 4u * AV1B_UNIT_CTAS_PER_SM * n_sm;
+}
+
+template <class Ahead>
+__device__ __forceinline__ void run_item(const FrameArgs& a, const BlockRec& b, int part, int bi, const int4& reg,
+                                         volatile unsigned short* tiles, int* edges, int* tmp, int lane,
+                                         Ahead&& ahead) {
+  const int p = b.plane;
+  const PlaneGeom& g = a.L.p[p];
+  const int ss_x = p ? a.L.ss_x : 0, ss_y = p ? a.L.ss_y : 0;
+  const int tile_w = (1 << a.region_log2) >> ss_x, tile_h = (1 << a.region_log2) >> ss_y;
+  /* the part: a column of regions' width of the block, and some of its rows */
+  const int cols = mini(b.w, tile_w), across = b.parts > 1 ? b.w / cols : 1;
+  const int rows = b.h / (b.parts / across);
+  /* the scratch holds a residual of 1024 samples */
+  const bool fused = b.fuse_res && (b.tx_count == 0 || rows * cols <= 1024);
+  const bool has_res = fused && b.tx_count > 0;
+  const int row0 = part / across * rows, col0 = part % across * cols;
+  if (has_res) fetch_residual(a, b, tmp, row0, rows, col0, cols, lane);
+  /* a block that does not wait on samples: the done flags of the list */
+  if (!(b.sync & AV1B_SYNC_TAGS)) {
+    for (int k = lane; k < b.dep_count; k += 32) wait_block(a, a.deps[b.dep_first + k]);
+    __syncwarp();
+  }
+  px_t* dst = a.cur + g.off + b.y * g.stride + b.x;
+  unsigned* tagged = a.tags + a.tag_off[p] + b.y * g.grid_w + b.x;
+  TagIo t = tag_io(a, b, tagged, fused);
+  t.tile_w = tile_w;
+  t.tile_h = tile_h;
+  t.tile_x = b.x - reg.z * tile_w;
+  t.tile_y = b.y - reg.w * tile_h;
+  t.tile = tiles + (p == 0 ? 0 : (1 << (2 * a.region_log2)) + (p - 1) * t.tile_w * t.tile_h);
+  t.luma_tile_w = 1 << a.region_log2;
+  t.luma_tile = tiles + (t.tile_y << a.L.ss_y) * t.luma_tile_w + (t.tile_x << a.L.ss_x);
+  t.row0 = row0;
+  t.row1 = row0 + rows;
+  t.col0 = col0;
+  t.cols = cols;
+  intra_predict(intra_job(a, b), dst, g.stride, a.cur + a.L.p[0].off, a.L.p[0].stride, a.palette_map,
+                a.palette_colors + 8 * b.palette_color_idx, edges, lane, t, has_res ? tmp : nullptr,
+                reinterpret_cast<short*>(tmp + 1024), has_res, ahead);
+  __syncwarp();
+  if (!fused) {
+    for (int k = 0; k < b.tx_count; ++k) add_residual_cg(a, b, a.txs[b.tx_first + k], lane);
+    __syncwarp();
+    for (int y = 0; y < t.clip_h; ++y)
+      for (int x = lane; x < t.clip_w; x += 32) {
+        const unsigned v = static_cast<unsigned>(ldpx(dst + y * g.stride + x));
+        t.tile[(t.tile_y + y) * t.tile_w + t.tile_x + x] = static_cast<unsigned short>(v);
+        if (t.tile_y + y == t.tile_h - 1 || t.tile_x + x == t.tile_w - 1)
+          st_tag(tagged + y * g.grid_w + x, a.tag | v);
+      }
+  }
+  __syncwarp();
+  if (lane == 0 && (b.sync & AV1B_SYNC_FLAG)) st_release(a.done + (size_t)bi * AV1B_FLAG_STRIDE, a.epoch);
+  __syncwarp();   /* the caller replaces the record */
+}
+
+__global__ void __launch_bounds__(32 * AV1B_REGION_WARPS, 1) k_regions(const __grid_constant__ FrameArgs a) {
+  extern __shared__ __align__(16) unsigned char region_mem[];
+  RegionSmem& m = *reinterpret_cast<RegionSmem*>(region_mem);
+  const int n_samples = region_samples(a.L, a.region_log2);
+  volatile unsigned short* tiles = reinterpret_cast<volatile unsigned short*>(&m + 1);
+  int* items = reinterpret_cast<int*>(&m + 1) + n_samples / 2;
+  deps_may_start();
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* edges = m.warp[wib];
+  int* tmp = edges + 3 * AV1B_EDGE_LEN;
+  BlockRec& b = m.rec[wib];
+  constexpr int kBlockMask = (1 << AV1B_ITEM_SHIFT) - 1;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      /* every CTA makes one claim past the last region and ends */
+      m.region = static_cast<int>(atomicAdd(a.queue, 1u) - a.queue_base);
+      m.next = 0;
+    }
+    uint4* clear = reinterpret_cast<uint4*>(region_mem + sizeof(RegionSmem));
+    for (int k = threadIdx.x; k < n_samples / 8; k += blockDim.x)
+      clear[k] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    __syncthreads();
+    const int r = m.region;
+    if (r >= a.n_regions) break;
+    const int4 reg = a.regions[r];
+    for (int k = threadIdx.x; k < reg.y; k += blockDim.x) items[k] = a.items[reg.x + k];
+    __syncthreads();
+    auto claim = [&] {
+      int u = 0;
+      if (lane == 0) u = atomicAdd(&m.next, 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
+      return u < reg.y ? items[u] : -1;
+    };
+    /* a record, a word a lane */
+    constexpr int kWords = sizeof(BlockRec) / sizeof(int);
+    static_assert(kWords <= 32 && sizeof(BlockRec) % sizeof(int) == 0, "a record is a word a lane");
+    auto record = [&](int item) {
+      return lane < kWords ? reinterpret_cast<const int*>(a.blocks + (item & kBlockMask))[lane] : 0;
+    };
+    int item = claim();
+    int word = item >= 0 ? record(item) : 0;
+    while (item >= 0) {
+      if (lane < kWords) reinterpret_cast<int*>(&b)[lane] = word;
+      __syncwarp();
+      /* the next item is claimed once this one's edges are there */
+      int next = -1;
+      run_item(a, b, item >> AV1B_ITEM_SHIFT, item & kBlockMask, reg, tiles, edges, tmp, lane, [&] {
+        next = claim();
+        if (next >= 0) word = record(next);
+      });
+      item = next;
+    }
+    /* the tiles and the items are read until every warp is through */
+    __syncthreads();
   }
 }
 
@@ -2617,10 +2790,12 @@ cudaError_t launch_recon_stage(int stage, const FrameArgs& a, int n_sm, cudaStre
       break;
     default:
       if (a.n_units > 0) {
-        const size_t smem = 4 * (3 * AV1B_EDGE_LEN + AV1B_UNIT_SCRATCH) * sizeof(int);
-        const int grid = AV1B_UNIT_CTAS_PER_SM * n_sm;
-        if (a.units_inter) k_units<true><<<grid, 128, smem, s>>>(a);
-        else k_units<false><<<grid, 128, smem, s>>>(a);
+        if (units_by_region(a)) {
+          k_regions<<<region_ctas(a, n_sm), 32 * AV1B_REGION_WARPS, region_smem(a.L, a.region_log2), s>>>(a);
+        } else {
+          const size_t smem = 4 * (3 * AV1B_EDGE_LEN + AV1B_UNIT_SCRATCH) * sizeof(int);
+          k_units<<<AV1B_UNIT_CTAS_PER_SM * n_sm, 128, smem, s>>>(a);
+        }
       }
       break;
   }
@@ -2817,7 +2992,7 @@ static cudaError_t load_all_kernels() {
       (e = load_kernel(k_itx<2>)) != cudaSuccess || (e = load_kernel(k_itx<3>)) != cudaSuccess ||
       (e = load_kernel(k_itx<4>)) != cudaSuccess || (e = load_kernel(k_itx<5>)) != cudaSuccess ||
       (e = load_kernel(k_itx<6>)) != cudaSuccess || (e = load_kernel(k_itx<7>)) != cudaSuccess ||
-      (e = load_kernel(k_units<true>)) != cudaSuccess || (e = load_kernel(k_units<false>)) != cudaSuccess ||
+      (e = load_kernel(k_units)) != cudaSuccess || (e = load_kernel(k_regions)) != cudaSuccess ||
       (e = load_kernel(k_selftest_wait)) != cudaSuccess || (e = load_kernel(k_deblock<AV1B_DB_PLAIN>)) != cudaSuccess ||
       (e = load_kernel(k_cdef_search)) != cudaSuccess || (e = load_kernel(k_cdef)) != cudaSuccess ||
       (e = load_kernel(k_cdef_tile)) != cudaSuccess ||
@@ -2835,17 +3010,20 @@ cudaError_t set_kernel_attributes() {
     const cudaError_t e = load_all_kernels();
     if (e != cudaSuccess) return e;
   }
-  cudaError_t e = cudaFuncSetAttribute(k_units<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(k_units, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        4 * (3 * AV1B_EDGE_LEN + AV1B_UNIT_SCRATCH) * (int)sizeof(int));
   if (e != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(k_units<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                4 * (3 * AV1B_EDGE_LEN + AV1B_UNIT_SCRATCH) * (int)sizeof(int))) != cudaSuccess)
+  Layout full{}, half{};   /* the largest tiles: 64x64 in 4:4:4, 128x128 in 4:2:0 */
+  half.ss_x = half.ss_y = 1;
+  const size_t most = std::max(region_smem(full, 6), region_smem(half, 7));
+  if ((e = cudaFuncSetAttribute(k_regions, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(most))) != cudaSuccess)
     return e;
   /* phase B's picture reads bypass L1: the SM's memory goes to shared memory,
-   * so AV1B_UNIT_CTAS_PER_SM CTAs fit */
-  if ((e = cudaFuncSetAttribute(k_units<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+   * so two CTAs fit */
+  if ((e = cudaFuncSetAttribute(k_units, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_units<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
+      (e = cudaFuncSetAttribute(k_regions, cudaFuncAttributePreferredSharedMemoryCarveout,
                                 cudaSharedmemCarveoutMaxShared)) != cudaSuccess)
     return e;
   return cudaSuccess;

@@ -29,6 +29,19 @@ namespace av1b {
  * microseconds on the dependency path, more than the halved residency (two
  * CTAs a SM instead of four) costs. */
 #define AV1B_UNIT_SCRATCH 4096
+/* Phase B by regions: squares of 64 luma samples - or of 128, in a frame with
+ * a block that no 64x64 square holds and that cannot be predicted in parts - a
+ * CTA a region. Its warps, its scratch a warp (ints: a residual of up to 1024
+ * samples, and 1024 16-bit predictions), and the samples of an item (a larger block
+ * is several, each some of its rows). A region's time falls with its warps:
+ * most of them wait, holding the next blocks in order of depth while others
+ * become ready (a 4K key frame alone 8.26, 5.72, 4.73, 3.83 and 3.64 ms a pass
+ * at 4, 6, 8, 12 and 16 warps; more do not fit the SM's registers). */
+#define AV1B_REGION_WARPS 16
+#define AV1B_REGION_SCRATCH 1536
+#define AV1B_ITEM_SAMPLES 512
+/* an item: the block's index, from bit AV1B_ITEM_SHIFT on which of its parts */
+#define AV1B_ITEM_SHIFT 27
 /* superres: output samples of a row a CTA writes; loop restoration: the
  * columns of a tile */
 #define AV1B_UP_OUT 512
@@ -77,10 +90,16 @@ struct FrameArgs {
   const int* units;             /* phase B block indices, chain after chain */
   const int* chains;            /* chain c is units[chains[c] .. chains[c + 1]) */
   int n_chains;
+  /* phase B by regions (n_regions 0: by chains): region r's items are
+   * items[regions[r].x] on, regions[r].y of them; z and w: its place, in
+   * regions */
+  const int4* regions;
+  const int* items;
+  int n_regions, region_log2;
   const int* deps;              /* the phase B blocks each phase B block waits for */
   int units_inter;              /* some phase B block is an inter kind */
   int n_units;
-  unsigned* queue;              /* counts every claim: chain = count - queue_base */
+  unsigned* queue;              /* counts every claim: chain (or region) = count - queue_base */
   unsigned queue_base;
   const int2* inter_tiles;      /* phase A: (block, x0 | y0 << 16) */
   int n_inter_tiles;
@@ -142,6 +161,14 @@ inline bool inter_one_launch(const FrameArgs& a, int n_sm) {
 inline bool itx_one_launch(const FrameArgs& a, int n_sm) {
   return !a.itx_overlap && a.n_itx_batches <= 4 * AV1B_ITX_ALL_CTAS * n_sm;
 }
+/* The samples of a region's planes; the items it may have (blocks of 4x4). */
+AV1B_HD int region_samples(const Layout& L, int log2) {
+  return (1 << (2 * log2)) + 2 * (1 << (2 * log2 - L.ss_x - L.ss_y));
+}
+AV1B_HD int region_items(const Layout& L, int log2) { return region_samples(L, log2) / 16; }
+/* Stage 3 by regions, and the claims it makes of the queue. */
+inline bool units_by_region(const FrameArgs& a) { return a.tags && a.n_regions > 0; }
+unsigned unit_claims(const FrameArgs& a, int n_sm);
 /* stage 1: phase A prediction; 2: the inverse transforms (phase A residual
  * added, phase B residual computed ahead); 3: the dependency-scheduled
  * phase B. */
