@@ -176,8 +176,8 @@ cudaError_t launch_recon_stage(int stage, const FrameArgs& a, int n_sm, cudaStre
 /* `early` (here and below): the kernel starts as the one launched before it
  * drains, and waits for it to end before it reads anything. Only for a kernel
  * that follows one which waited itself, or was launched without: the kernels
- * before that one are then complete too. (The grain templates' kernel does not
- * wait: it reads nothing a kernel of the frame writes.) */
+ * before that one are then complete too. (The grain templates' kernel reads
+ * nothing a kernel of the frame writes: it waits as it ends.) */
 cudaError_t launch_prep_filters(const av1b_deblock_edge* edges, int n_edges, const av1b_cdef_block* cdef,
                                 int n_cdef, const Layout& L, int grid_w, int grid_n, DeblockRec* v,
                                 DeblockRec* h, CdefRec* cdef_out, unsigned* cells, unsigned* extra,
