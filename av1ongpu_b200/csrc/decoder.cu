@@ -943,8 +943,9 @@ inline size_t piece_begin(size_t n, int pieces, int i) { return n * i / pieces; 
  * of some rows each, and items in each region where several share it. Returns
  * false, and the frame runs by larger regions or by chains, where a block that
  * cannot be does not lie in one region, or is off the cell grid (no tagged
- * samples), regions wait on each other in a circle, inter blocks are among
- * them, or a palette colour could be the tiles' empty mark. */
+ * samples), one waits for samples inside another region (only a region's last
+ * row and column are tagged), regions wait on each other in a circle, inter
+ * blocks are among them, or a palette colour could be the tiles' empty mark. */
 bool plan_regions(const PlanCtx& c, int log2, Plan* P, const std::vector<int>& U,
                   const std::vector<int>& first, const std::vector<int>& udeps, const std::vector<int>& depth) {
   PlanScratch& S = *c.scratch;
@@ -996,6 +997,22 @@ bool plan_regions(const PlanCtx& c, int log2, Plan* P, const std::vector<int>& U
     if (of[u] < 0 && (!apart || (across > 1 && b.x & ((1 << bx) - 1)) || b.y & (b.h / down - 1) ||
                       (across == 1 && rx1 != rx)))
       return false;
+    if (b.sync & AV1B_SYNC_TAGS) {
+      /* its edges' samples in other regions than its own (of a block that
+       * several share, all its samples: each part reads the edges): above,
+       * in a last row where the block starts a region's rows; left, in a last
+       * column likewise */
+      const bool row_off = b.y & ((1 << by) - 1), col_off = b.x & ((1 << bx) - 1), one = of[u] >= 0;
+      const int cell = b.plane == 0 ? 2 : ((b.plane == 1 ? L.ss_x : L.ss_y) ? 1 : 2);
+      auto outside = [&](const unsigned (&cells)[2], int own) {
+        const uint64_t m = cells[0] | (static_cast<uint64_t>(cells[1]) << 32);
+        return (one && own >= 64 ? 0 : m >> (one ? own : 0)) != 0;
+      };
+      if ((row_off && outside(b.wait_cells[0], (((rx + 1) << bx) - b.x) >> cell)) ||
+          (col_off && outside(b.wait_cells[1], (((ry + 1) << by) - b.y) >> cell)) ||
+          (!one && row_off && col_off && (b.sync & AV1B_SYNC_CORNER)))
+        return false;
+    }
     b.parts = static_cast<short>(down * across);
     bool full = false;
     each_part(u, [&](int r, int) { full |= ++count[r] > region_items(L, log2); });

@@ -2,7 +2,9 @@
 wait end (tests/cpp/regions.cu). On the GPU, the same frames decoded by regions
 and by chains (a traced frame runs by chains), which must give the same
 samples: regions cut by the picture's sides, regions of one block, blocks of
-several items, raw residuals, each bit depth and superblock size."""
+several items, raw residuals, each bit depth and superblock size; and layouts
+and coding orders that no partition tree gives (tests/cpp/layouts.hpp), in
+4:2:0, 4:2:2 and 4:4:4."""
 import os
 import subprocess
 
@@ -62,3 +64,26 @@ def test_regions_and_chains_agree(av1b, params):
     for k, (a, b) in enumerate(zip(_decode(av1b, prm, 3, False), _decode(av1b, prm, 3, True))):
         for p in range(3):
             assert np.array_equal(a[p], b[p]), 'frame %d plane %d' % (k, p)
+
+
+def build_layouts_client(tmp_path):
+    exe = str(tmp_path / 'layouts_client')
+    lib = os.path.join(tpi.ROOT, 'av1ongpu_b200')
+    cmd = ['/usr/bin/g++', '-std=c++17', '-O1', os.path.join(tpi.ROOT, 'tests', 'cpp', 'layouts_client.cpp'),
+           '-L', lib, '-lav1b', '-Wl,-rpath,' + lib, '-o', exe]
+    subprocess.run(cmd, check=True, capture_output=True)
+    return exe
+
+
+def test_layouts_client_builds(tmp_path):
+    from av1ongpu_b200 import build as b
+    b.build()
+    build_layouts_client(tmp_path)
+
+
+@pytest.mark.gpu
+def test_layouts_by_regions_and_by_chains(av1b, tmp_path):
+    if not av1b.cuda_available():
+        pytest.skip('no CUDA device')
+    r = subprocess.run([build_layouts_client(tmp_path)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith('ok'), r.stdout[-2000:] + r.stderr[-500:]
