@@ -1251,7 +1251,8 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
       }
       if (b.kind == AV1B_U_INTRA && b.mode == 13 && !b.palette) {
         /* by their tags only where every luma sample is of a block waited
-         * for: another's would never be tagged */
+         * for: another's would never be tagged. Chroma only: the mode on a
+         * luma block reads at twice its own place, outside its region's tile */
         const int lx1 = (b.x + b.w) << L.ss_x, ly1 = (b.y + b.h) << L.ss_y;
         bool all = lx1 <= L.p[0].grid_w && ly1 <= L.p[0].grid_h && b.w * b.h <= 1024;
         each_cell(0, b.x << L.ss_x, (b.x + b.w - 1) << L.ss_x, b.y << L.ss_y,
@@ -1261,7 +1262,7 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
             const int o = S.owner[0][static_cast<size_t>(cy) * cw[0] + cx];
             all = all && o >= 0 && o < bi && is_b[o];
           }
-        if (all && b.sync)
+        if (all && p > 0 && b.sync)
           b.sync |= AV1B_SYNC_LUMA;
         else
           b.sync = 0;

@@ -160,7 +160,7 @@ class LayoutBuilder {
   std::vector<uint8_t> done_[3];
 };
 
-static const int kHandLayouts = 6, kRandomLayouts = 60;
+static const int kHandLayouts = 7, kRandomLayouts = 60;
 inline int layout_count() { return kHandLayouts + kRandomLayouts; }
 
 inline LayoutFrame layout_frame(int i) {
@@ -226,6 +226,17 @@ inline LayoutFrame layout_frame(int i) {
         for (int x = 0; x < 64; x += 16)
           for (int k = 0; k < 64; k += 16) b.block(0, x, y + k, 16, 16, 7);
         b.chroma(0, y, 64, y + 64);
+      }
+      return b.take();
+    }
+    case 5: {  /* the mode of chroma from luma on a luma block, the samples at
+                  twice its place coded before it */
+      LayoutBuilder b("luma by the chroma from luma mode", 128, 128, 8, 1, 1, 6);
+      static const int kOrder[4][2] = {{64, 64}, {0, 0}, {64, 0}, {0, 64}};
+      for (const int* at : kOrder) {
+        if (at[0] + at[1] == 0) b.block(0, 48, 48, 16, 16, 13);
+        b.fill(0, at[0], at[1], at[0] + 64, at[1] + 64, 16, 16);
+        b.chroma(at[0], at[1], at[0] + 64, at[1] + 64);
       }
       return b.take();
     }

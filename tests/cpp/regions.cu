@@ -8,7 +8,8 @@
  * samples lie in, as items that are each of its parts once; every sample it
  * waits for is either of an item earlier in its own region, or of an item of a
  * region listed before and in that region's last row or column (the only
- * samples that are tagged); and a part's residual fits a warp's scratch.
+ * samples that are tagged); what a chroma-from-luma block waits for by tags
+ * lies in its region's luma tile; and a part's residual fits a warp's scratch.
  * A frame with inter blocks in phase B or a block off its cells has no
  * regions. Prints "ok" at the end; exits non-zero on a failure.
  */
@@ -114,6 +115,12 @@ void check_syntax(av1b_decoder* d, WorkPool* pool, const av1b_frame_syntax& s, c
         if (b.sync & AV1B_SYNC_CORNER) awaited(b.x - 1, b.y - 1);
       }
       CHECK(ok, "%s frame %d: block %d part %d waits for a sample nobody tags", name, k, bi, part);
+      if (b.sync & AV1B_SYNC_LUMA) {
+        const int side = 1 << P.region_log2;
+        const int lx = (b.x - r.z * tw) << L.ss_x, ly = (b.y - r.w * th) << L.ss_y;
+        CHECK(lx >= 0 && ly >= 0 && lx + (b.w << L.ss_x) <= side && ly + (b.h << L.ss_y) <= side,
+              "%s frame %d: block %d's luma is outside its region's tile", name, k, bi);
+      }
     }
   }
   CHECK(static_cast<size_t>(place) == lists.items.size(), "%s frame %d: items outside regions", name, k);
