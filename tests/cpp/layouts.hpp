@@ -118,10 +118,10 @@ class LayoutBuilder {
 
   /* The plane's samples not coded yet, in blocks of w x h from (x0, y0) on,
    * row by row. */
-  void fill(int plane, int x0, int y0, int x1, int y1, int w, int h) {
+  void fill(int plane, int x0, int y0, int x1, int y1, int w, int h, int mode = -1) {
     for (int y = y0; y < y1; y += h)
       for (int x = x0; x < x1; x += w)
-        if (!at(plane, x, y)) block(plane, x, y, w, h);
+        if (!at(plane, x, y)) block(plane, x, y, w, h, mode);
   }
   void chroma() { chroma(0, 0, f_.width, f_.height); }
   /* the chroma of [x0, x1) x [y0, y1) of luma */
@@ -235,7 +235,7 @@ inline LayoutFrame layout_frame(int i) {
       static const int kOrder[4][2] = {{64, 64}, {0, 0}, {64, 0}, {0, 64}};
       for (const int* at : kOrder) {
         if (at[0] + at[1] == 0) b.block(0, 48, 48, 16, 16, 13);
-        b.fill(0, at[0], at[1], at[0] + 64, at[1] + 64, 16, 16);
+        b.fill(0, at[0], at[1], at[0] + 64, at[1] + 64, 16, 16, 0);
         b.chroma(at[0], at[1], at[0] + 64, at[1] + 64);
       }
       return b.take();
