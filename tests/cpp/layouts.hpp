@@ -125,9 +125,10 @@ class LayoutBuilder {
   }
   void chroma() { chroma(0, 0, f_.width, f_.height); }
   /* the chroma of [x0, x1) x [y0, y1) of luma */
-  void chroma(int x0, int y0, int x1, int y1) {
+  void chroma(int x0, int y0, int x1, int y1, int mode = -1) {
     for (int p = 1; p < 3; ++p)
-      fill(p, x0 >> f_.ss_x, y0 >> f_.ss_y, std::min(gw_[p], x1 >> f_.ss_x), std::min(gh_[p], y1 >> f_.ss_y), 16, 16);
+      fill(p, x0 >> f_.ss_x, y0 >> f_.ss_y, std::min(gw_[p], x1 >> f_.ss_x), std::min(gh_[p], y1 >> f_.ss_y), 16, 16,
+           mode);
   }
 
   /* A random tiling of [x, x + w) x [y, y + h): split in two, in either
@@ -236,7 +237,7 @@ inline LayoutFrame layout_frame(int i) {
       for (const int* at : kOrder) {
         if (at[0] + at[1] == 0) b.block(0, 48, 48, 16, 16, 13);
         b.fill(0, at[0], at[1], at[0] + 64, at[1] + 64, 16, 16, 0);
-        b.chroma(at[0], at[1], at[0] + 64, at[1] + 64);
+        b.chroma(at[0], at[1], at[0] + 64, at[1] + 64, 0);
       }
       return b.take();
     }
