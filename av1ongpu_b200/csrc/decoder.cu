@@ -179,6 +179,7 @@ struct av1b_decoder {
   /* chroma blocks of difference-weighted compounds read their luma block's
    * mask when it is the same prediction (av1b_set_shared_masks) */
   std::atomic<bool> share_masks{true};
+  std::atomic<bool> plan_regions{true};   /* its plans get regions (plan_without_regions) */
 
   /* optional trace of phase B (av1b_set_unit_trace): 4 uint64 per block */
   bool tracing = false;
@@ -503,6 +504,7 @@ struct PlanCtx {
   bool levels = false;
   size_t n_levels = 0, n_qm = 0;
   bool share_masks = true;        /* plan_shared_masks runs */
+  bool regions = true;            /* the plan may run by regions */
 };
 
 /* The first error one piece of the planner met. */
@@ -918,7 +920,9 @@ struct PlanScratch {
   std::vector<uint64_t> head_key;
   std::vector<int> units_coding, ui_of, udepth, udeps;
   std::vector<uint8_t> is_b;
-  std::vector<int> region_of, region_level, region_count, by_depth;
+  std::vector<int> region_count[2], region_level, region_at, region_first, region_heirs;
+  std::vector<uint64_t> region_waits[2], region_keys;
+  std::vector<int> unit_region;       /* per unit: its 64x64 region when it is one item; -1 */
   std::vector<uint8_t> flagged;       /* blocks some block waits on by done flag */
   bool on_grid = false;               /* every block lies on its plane's owner cells */
   std::vector<uint16_t> itx_key;
@@ -935,154 +939,242 @@ int pieces_for(size_t n, const PlanCtx& c, size_t min_piece) {
 inline size_t piece_begin(size_t n, int pieces, int i) { return n * i / pieces; }
 
 /* The phase B blocks by regions of 1 << log2 luma samples square, for the
- * kernel that runs a region a CTA: U, the blocks in coding order, with their dependency
- * lists (unit indices) and depths. Regions are listed by level - one more
- * than the deepest region a block of theirs waits for - so every region comes
- * after those it waits for, and a region's blocks by depth, for the same
- * reason. A large block whose samples can be predicted apart is several items
- * of some rows each, and items in each region where several share it. Returns
- * false, and the frame runs by larger regions or by chains, where a block that
- * cannot be does not lie in one region, or is off the cell grid (no tagged
- * samples), one waits for samples inside another region (only a region's last
- * row and column are tagged), regions wait on each other in a circle, inter
- * blocks are among them, or a palette colour could be the tiles' empty mark. */
-bool plan_regions(const PlanCtx& c, int log2, Plan* P, const std::vector<int>& U,
-                  const std::vector<int>& first, const std::vector<int>& udeps, const std::vector<int>& depth) {
-  PlanScratch& S = *c.scratch;
-  const Layout& L = c.L;
-  auto& B = P->R->blocks;
-  const size_t nu = U.size();
-  if (!S.on_grid || P->units_inter || B.size() >= (size_t(1) << AV1B_ITEM_SHIFT)) return false;
-  if (log2 > 6 && !(L.ss_x && L.ss_y)) return false;  /* the tiles would not fit an SM */
-  for (int v : P->R->palette_colors)
-    if (v < 0 || v > 4095) return false;
-  const int rw = (L.p[0].grid_w + (1 << log2) - 1) >> log2, rh = (L.p[0].grid_h + (1 << log2) - 1) >> log2;
-  std::vector<int>& of = S.region_of;  /* a block's region; -1: several */
-  std::vector<int>& level = S.region_level;
-  std::vector<int>& count = S.region_count;
-  of.resize(nu);
-  level.assign(static_cast<size_t>(rw) * rh, 0);
-  count.assign(static_cast<size_t>(rw) * rh, 0);
-  /* the regions of block u's parts, each `f(region, part)` */
-  auto each_part = [&](size_t u, auto&& f) {
-    const BlockRec& b = B[U[u]];
-    if (of[u] >= 0) {
-      for (int k = 0; k < b.parts; ++k) f(of[u], k);
-      return;
-    }
+ * kernel that runs a region a CTA. Regions are listed by level - one more
+ * than the deepest region whose samples a block of theirs waits for - so every
+ * region comes after those it waits for, and a region's items by their blocks'
+ * depth, for the same reason. A large block whose samples can be predicted
+ * apart is several items of some rows each, and items in each region where
+ * several share it. A frame cannot run by regions of a size, and runs by
+ * larger ones or by chains, where a block that cannot be in parts does not lie
+ * in one region, or is off the cell grid (no tagged samples), one waits for
+ * samples inside another region (only a region's last row and column are
+ * tagged), regions wait on each other in a circle, inter blocks are among
+ * them, or a palette colour could be the tiles' empty mark.
+ *
+ * What it costs is one look at each block for both sizes, which the pool's
+ * threads share and which goes with the pass that writes the block's
+ * dependency list (RegionScan::block), and placing and sorting the items,
+ * which go beside the chains; the graph has a node a region and a few edges
+ * each, and only a size whose graph has no circle gets lists. A key frame's
+ * plan on seven threads, without regions / with them: 720p 3.5 / 3.8 ms, 1080p
+ * 6.1 / 6.5, 4K with 128x128 superblocks 13.2 / 13.4. As one serial pass a
+ * size that swept the blocks' dependency lists until the levels stood: 5.7,
+ * 10.7 and 39 ms. */
+struct RegionScan {
+  Layout L;
+  const BlockRec* blocks = nullptr;
+  const int* deps = nullptr;      /* the blocks' dependency lists */
+  int log2 = 6, rw = 0, rh = 0;
+  int* count = nullptr;           /* items, by region */
+  uint64_t* waits = nullptr;      /* the regions each waits for: bit (dy + 3) * 8 + dx + 3 */
+  std::atomic<bool> refused{true};
+
+  void start(const Layout& layout, const PlanLists& R, int log2_side, std::vector<int>& counts,
+             std::vector<uint64_t>& masks) {
+    L = layout;
+    blocks = R.blocks.data();
+    deps = R.deps.data();
+    log2 = log2_side;
+    rw = (L.p[0].grid_w + (1 << log2) - 1) >> log2;
+    rh = (L.p[0].grid_h + (1 << log2) - 1) >> log2;
+    counts.assign(static_cast<size_t>(rw) * rh, 0);
+    masks.assign(static_cast<size_t>(rw) * rh, 0);
+    count = counts.data();
+    waits = masks.data();
+    refused = false;
+  }
+
+  /* The parts of block b, `across` side by side; 0: it is refused. */
+  int parts(const BlockRec& b, int* across) const {
     const int bx = log2 - (b.plane ? L.ss_x : 0), by = log2 - (b.plane ? L.ss_y : 0);
-    const int cols = std::min<int>(b.w, 1 << bx), across = b.w / cols, rows = b.h / (b.parts / across);
-    for (int k = 0; k < b.parts; ++k)
-      f(((b.y + k / across * rows) >> by) * rw + ((b.x + k % across * cols) >> bx), k);
-  };
-  for (size_t u = 0; u < nu; ++u) {
-    BlockRec& b = B[U[u]];
-    const int bx = log2 - (b.plane ? L.ss_x : 0), by = log2 - (b.plane ? L.ss_y : 0);
-    const int rx = b.x >> bx, ry = b.y >> by;
     const int n = b.w * b.h;
-    const int rx1 = (b.x + b.w - 1) >> bx, ry1 = (b.y + b.h - 1) >> by;
-    if (b.x < 0 || b.y < 0 || rx1 >= rw || ry1 >= rh || (b.fi_mode >= 0 && n > 1024)) return false;
-    of[u] = rx1 == rx && ry1 == ry ? ry * rw + rx : -1;
+    *across = 1;
+    const bool one = (b.x + b.w - 1) >> bx == b.x >> bx && (b.y + b.h - 1) >> by == b.y >> by;
+    if (one && n <= AV1B_ITEM_SAMPLES) return 1;
     /* in parts: not the recursive filter, nor chroma from luma (one average),
      * nor a block that others wait for as a whole */
-    const bool apart = pow2_in(b.w, 4, 64) && pow2_in(b.h, 4, 64) && b.fuse_res &&
-                       (b.tx_count == 0 || b.res_one) && (b.palette || (b.mode != 13 && b.fi_mode < 0)) &&
-                       !(b.sync & AV1B_SYNC_FLAG);
-    int down = 1, across = 1;
-    if (apart) {
-      const int cols = std::min<int>(b.w, 1 << bx);
-      across = b.w / cols;
-      while (b.h / down > (1 << by) || b.h / down * cols > AV1B_ITEM_SAMPLES) down *= 2;
-    }
-    if (of[u] < 0 && (!apart || (across > 1 && b.x & ((1 << bx) - 1)) || b.y & (b.h / down - 1) ||
-                      (across == 1 && rx1 != rx)))
-      return false;
-    if (b.sync & AV1B_SYNC_TAGS) {
-      /* its edges' samples in other regions than its own (of a block that
-       * several share, all its samples: each part reads the edges): above,
-       * in a last row where the block starts a region's rows; left, in a last
-       * column likewise */
-      const bool row_off = b.y & ((1 << by) - 1), col_off = b.x & ((1 << bx) - 1), one = of[u] >= 0;
-      const int cell = b.plane == 0 ? 2 : ((b.plane == 1 ? L.ss_x : L.ss_y) ? 1 : 2);
-      auto outside = [&](const unsigned (&cells)[2], int own) {
-        const uint64_t m = cells[0] | (static_cast<uint64_t>(cells[1]) << 32);
-        return (one && own >= 64 ? 0 : m >> (one ? own : 0)) != 0;
-      };
-      if ((row_off && outside(b.wait_cells[0], (((rx + 1) << bx) - b.x) >> cell)) ||
-          (col_off && outside(b.wait_cells[1], (((ry + 1) << by) - b.y) >> cell)) ||
-          (!one && row_off && col_off && (b.sync & AV1B_SYNC_CORNER)))
-        return false;
-    }
-    b.parts = static_cast<short>(down * across);
-    bool full = false;
-    each_part(u, [&](int r, int) { full |= ++count[r] > region_items(L, log2); });
-    if (full) return false;
+    const bool apart = pow2_in(b.w, 4, 64) && pow2_in(b.h, 4, 64) && b.fuse_res && (b.tx_count == 0 || b.res_one) &&
+                       (b.palette || (b.mode != 13 && b.fi_mode < 0)) && !(b.sync & AV1B_SYNC_FLAG);
+    if (!apart) return one ? 1 : 0;
+    int down = 1;
+    const int cols = std::min<int>(b.w, 1 << bx);
+    *across = b.w / cols;
+    while (b.h / down > (1 << by) || b.h / down * cols > AV1B_ITEM_SAMPLES) down *= 2;
+    if (!one && ((*across > 1 && b.x & ((1 << bx) - 1)) || b.y & (b.h / down - 1) ||
+                 (*across == 1 && (b.x + b.w - 1) >> bx != b.x >> bx)))
+      return 0;
+    return down * *across;
   }
-  /* one sweep in coding order gives the levels where regions are coded one
-   * after another; where they interleave, a few */
-  bool changed = true;
-  for (int sweep = 0; changed; ++sweep) {
-    if (sweep == 8) return false;
-    changed = false;
-    for (size_t u = 0; u < nu; ++u) {
-      auto raise = [&](int r, int) {
-        int l = level[r];
-        for (int j = first[u]; j < first[u + 1]; ++j) {
-          auto wait = [&](int o, int) {
-            if (o != r && level[o] >= l) l = level[o] + 1;
-          };
-          const int o = udeps[j];
-          if (of[o] >= 0) wait(of[o], 0);
-          else each_part(o, wait);
-        }
-        if (l > level[r]) {
-          level[r] = l;
-          changed = true;
-        }
-      };
-      if (of[u] >= 0) raise(of[u], 0);
-      else each_part(u, raise);
-    }
+  /* The region of part k of block b's n. */
+  int region(const BlockRec& b, int n, int across, int k) const {
+    const int bx = log2 - (b.plane ? L.ss_x : 0), by = log2 - (b.plane ? L.ss_y : 0);
+    return ((b.y + k / across * (b.h / (n / across))) >> by) * rw + ((b.x + k % across * (b.w / across)) >> bx);
   }
-  std::vector<int>& order = S.by_depth;
-  const size_t nr = level.size();
-  int most = 0;
-  size_t items = 0, used = 0;
+
+  /* The region that a region of the smaller size lies in. */
+  int larger(const RegionScan& small, int r) const { return r / small.rw / 2 * rw + r % small.rw / 2; }
+
+  /* What a thread has seen of the region its last block was in: blocks come
+   * region after region, so the shared words, whose cache lines the threads'
+   * regions share, are written once a run. */
+  struct Run {
+    int region = -1, count = 0;
+    uint64_t waits = 0;
+  };
+  void flush(Run& run) {
+    if (run.region >= 0) {
+      __atomic_fetch_add(count + run.region, run.count, __ATOMIC_RELAXED);
+      if (run.waits) __atomic_fetch_or(waits + run.region, run.waits, __ATOMIC_RELAXED);
+    }
+    run = Run();
+  }
+  void add(Run& run, int region, int items, uint64_t mask) {
+    if (run.region != region) {
+      flush(run);
+      run.region = region;
+    }
+    run.count += items;
+    run.waits |= mask;
+  }
+
+  /* One block (any thread): its parts, counted in their regions, and the
+   * regions they wait for. Its region when it is one item, else -1; `inner`:
+   * it is one, and waits for no other region. */
+  int block(const BlockRec& b, Run& run, bool* inner) {
+    *inner = false;
+    auto refuse = [&] {
+      refused.store(true, std::memory_order_relaxed);
+      return -1;
+    };
+    if (refused.load(std::memory_order_relaxed)) return -1;
+    const int bx = log2 - (b.plane ? L.ss_x : 0), by = log2 - (b.plane ? L.ss_y : 0);
+    const int rx = b.x >> bx, ry = b.y >> by;
+    const int rx1 = (b.x + b.w - 1) >> bx, ry1 = (b.y + b.h - 1) >> by;
+    const bool one = rx1 == rx && ry1 == ry;
+    int across = 1;
+    const int n = rx1 < rw && ry1 < rh && !(b.fi_mode >= 0 && b.w * b.h > 1024) ? parts(b, &across) : 0;
+    if (n == 0) return refuse();
+    const int own = n == 1 ? ry * rw + rx : -1;
+    for (int k = 0; k < n; ++k) add(run, n == 1 ? own : region(b, n, across, k), 1, 0);
+    /* every part waits for the regions (x0 .. x1, y0 .. y1) */
+    bool waits_any = false;
+    auto wait = [&](int x0, int x1, int y0, int y1) {
+      for (int py = ry; py <= ry1; ++py)
+        for (int px = rx; px <= rx1; ++px) {
+          uint64_t m = 0;
+          for (int y = y0; y <= y1; ++y)
+            for (int x = x0; x <= x1; ++x) {
+              if (x == px && y == py) continue;
+              if (x < px - 3 || x > px + 4 || y < py - 3 || y > py + 4) {
+                refuse();
+                return;
+              }
+              m |= 1ull << ((y - py + 3) * 8 + x - px + 3);
+            }
+          if (m) {
+            waits_any = true;
+            add(run, py * rw + px, 0, m);
+          }
+        }
+    };
+    if (!(b.sync & AV1B_SYNC_TAGS)) {
+      /* by the done flags of its list: blocks of one region each */
+      for (int j = 0; j < b.dep_count; ++j) {
+        const BlockRec& o = blocks[deps[b.dep_first + j]];
+        const int ox = o.x >> (log2 - (o.plane ? L.ss_x : 0)), oy = o.y >> (log2 - (o.plane ? L.ss_y : 0));
+        wait(ox, ox, oy, oy);
+      }
+      return own;
+    }
+    /* by the samples of its edges: those in other regions than its own (of a
+     * block that several share, all of them: each part reads the edges) lie
+     * above, in a last row where the block starts a region's rows, and left,
+     * in a last column likewise */
+    const int cell = b.plane == 0 ? 2 : ((b.plane == 1 ? L.ss_x : L.ss_y) ? 1 : 2);
+    const bool row_off = b.y & ((1 << by) - 1), col_off = b.x & ((1 << bx) - 1);
+    const uint64_t above = b.wait_cells[0][0] | (static_cast<uint64_t>(b.wait_cells[0][1]) << 32);
+    const uint64_t left = b.wait_cells[1][0] | (static_cast<uint64_t>(b.wait_cells[1][1]) << 32);
+    const int in_x = (((rx + 1) << bx) - b.x) >> cell, in_y = (((ry + 1) << by) - b.y) >> cell;
+    if ((row_off && (one ? in_x < 64 && above >> in_x : above != 0)) ||
+        (col_off && (one ? in_y < 64 && left >> in_y : left != 0)) ||
+        (!one && row_off && col_off && (b.sync & AV1B_SYNC_CORNER)))
+      return refuse();
+    auto first = [](uint64_t m) { return __builtin_ctzll(m); };
+    auto last = [](uint64_t m) { return 63 - __builtin_clzll(m); };
+    if (above && !row_off)
+      wait((b.x + (first(above) << cell)) >> bx, (b.x + (last(above) << cell)) >> bx, ry - 1, ry - 1);
+    if (left && !col_off)
+      wait(rx - 1, rx - 1, (b.y + (first(left) << cell)) >> by, (b.y + (last(left) << cell)) >> by);
+    if (b.sync & AV1B_SYNC_CORNER && !(row_off && col_off)) {
+      const int x = (b.x - 1) >> bx, y = (b.y - 1) >> by;
+      wait(x, x, y, y);
+    }
+    *inner = own >= 0 && !waits_any;
+    return own;
+  }
+};
+
+/* The regions of a size by level (P->R->regions, items still unplaced); false
+ * where they wait on each other in a circle, or one has more items than its
+ * samples hold (blocks that overlap). */
+bool order_regions(const RegionScan& g, PlanScratch& S, PlanLists& R) {
+  const size_t nr = static_cast<size_t>(g.rw) * g.rh;
+  /* what each region's end leaves to do: its heirs, as lists back to back */
+  std::vector<int>& first = S.region_first;
+  std::vector<int>& heirs = S.region_heirs;
+  std::vector<int>& left = S.region_at;   /* regions still waited for */
+  std::vector<int>& level = S.region_level;
+  first.assign(nr + 1, 0);
+  left.assign(nr, 0);
+  level.assign(nr, 0);
+  auto each_wait = [&](size_t r, auto&& f) {
+    for (uint64_t m = g.waits[r]; m; m &= m - 1) {
+      const int bit = __builtin_ctzll(m);
+      f(static_cast<size_t>(static_cast<long long>(r) + (bit / 8 - 3) * g.rw + bit % 8 - 3));
+    }
+  };
+  for (size_t r = 0; r < nr; ++r)
+    each_wait(r, [&](size_t o) {
+      ++first[o + 1];
+      ++left[r];
+    });
+  for (size_t r = 0; r < nr; ++r) first[r + 1] += first[r];
+  heirs.resize(first[nr]);
+  std::vector<int> at(first.begin(), first.end() - 1), ready;
+  for (size_t r = 0; r < nr; ++r) each_wait(r, [&](size_t o) { heirs[at[o]++] = static_cast<int>(r); });
+  size_t used = 0, items = 0;
   for (size_t r = 0; r < nr; ++r) {
+    if (g.count[r] == 0) continue;
+    if (g.count[r] > region_items(g.L, g.log2)) return false;
+    ++used;
+    items += static_cast<size_t>(g.count[r]);
+    if (left[r] == 0) ready.push_back(static_cast<int>(r));
+  }
+  int most = 0;
+  for (size_t k = 0; k < ready.size(); ++k) {
+    const int r = ready[k];
     most = std::max(most, level[r]);
-    items += static_cast<size_t>(count[r]);
-    used += count[r] > 0;
+    for (int h = first[r]; h < first[r + 1]; ++h) {
+      level[heirs[h]] = std::max(level[heirs[h]], level[r] + 1);
+      if (--left[heirs[h]] == 0) ready.push_back(heirs[h]);
+    }
   }
-  /* the regions by level (a counting sort), their items' places */
-  std::vector<int> at(most + 2, 0);
+  if (ready.size() != used) return false;
+  at.assign(most + 2, 0);
   for (size_t r = 0; r < nr; ++r)
-    if (count[r]) ++at[level[r] + 1];
+    if (g.count[r]) ++at[level[r] + 1];
   for (int k = 0; k <= most; ++k) at[k + 1] += at[k];
-  sized(P->R->regions, used);
-  sized(P->R->items, items);
+  sized(R.regions, used);
+  sized(R.items, items);
   for (size_t r = 0; r < nr; ++r)
-    if (count[r])
-      P->R->regions[at[level[r]]++] = make_int4(0, count[r], static_cast<int>(r % rw), static_cast<int>(r / rw));
+    if (g.count[r])
+      R.regions[at[level[r]]++] =
+          make_int4(0, g.count[r], static_cast<int>(r) % g.rw, static_cast<int>(r) / g.rw);
   int place = 0;
-  for (int4& g : P->R->regions) {
-    g.x = place;
-    level[static_cast<size_t>(g.w) * rw + g.z] = place;
-    place += g.y;
+  for (int4& r : R.regions) {
+    r.x = place;
+    place += r.y;
   }
-  /* the blocks by depth (a counting sort), into their regions */
-  int deep = 0;
-  for (size_t u = 0; u < nu; ++u) deep = std::max(deep, depth[u]);
-  at.assign(deep + 2, 0);
-  for (size_t u = 0; u < nu; ++u) ++at[depth[u] + 1];
-  for (int k = 0; k <= deep; ++k) at[k + 1] += at[k];
-  order.resize(nu);
-  for (size_t u = 0; u < nu; ++u) order[at[depth[u]]++] = static_cast<int>(u);
-  for (size_t k = 0; k < nu; ++k) {
-    const int bi = U[order[k]];
-    each_part(order[k],
-              [&](int r, int part) { P->R->items[level[r]++] = bi | part << AV1B_ITEM_SHIFT; });
-  }
-  P->region_log2 = log2;
   return true;
 }
 
@@ -1349,8 +1441,22 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
   sized(P->R->deps, first[nu]);
   std::vector<int>& udeps = S.udeps;
   udeps.resize(first[nu]);
+  P->units_inter = false;
+  for (int pi = 0; pi < pieces; ++pi)
+    if (inter_piece[pi]) P->units_inter = true;
+  /* by regions of 64x64 luma samples, or of 128x128 (whose tiles fit an SM
+   * where chroma is subsampled both ways), or not */
+  RegionScan scan[2];
+  if (c.regions && S.on_grid && !P->units_inter && nb < (size_t(1) << AV1B_ITEM_SHIFT) &&
+      std::all_of(P->R->palette_colors.begin(), P->R->palette_colors.end(), [](int v) { return v >= 0 && v <= 4095; })) {
+    scan[0].start(L, *P->R, 6, S.region_count[0], S.region_waits[0]);
+    if (L.ss_x && L.ss_y) scan[1].start(L, *P->R, 7, S.region_count[1], S.region_waits[1]);
+    S.unit_region.resize(nu);
+  }
+  const bool by_regions = !scan[0].refused;
   c.pool->run(pieces, [&](int pi) {
     const size_t u0 = piece_begin(nu, pieces, pi), u1 = piece_begin(nu, pieces, pi + 1);
+    RegionScan::Run run[2];
     std::copy(pdeps[pi].begin(), pdeps[pi].end(), P->R->deps.begin() + first[u0]);
     for (size_t k = first[u0]; k < first[u1]; ++k) udeps[k] = ui_of[pdeps[pi][k - first[u0]]];
     for (size_t ui = u0; ui < u1; ++ui) {
@@ -1358,8 +1464,21 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
       b.dep_first = static_cast<int>(first[ui]);
       b.dep_count = dep_count[ui];
       if (flagged[P->R->units[ui]]) b.sync |= AV1B_SYNC_FLAG;
+      if (by_regions) {
+        b.parts = 1;
+        bool inner, large;
+        S.unit_region[ui] = scan[0].block(b, run[0], &inner);
+        if (!inner)
+          scan[1].block(b, run[1], &large);
+        else if (!scan[1].refused.load(std::memory_order_relaxed))
+          scan[1].add(run[1], scan[1].larger(scan[0], S.unit_region[ui]), 1, 0);
+      }
     }
+    for (int k = 0; k < 2; ++k) scan[k].flush(run[k]);
   });
+  const RegionScan* regions = nullptr;
+  for (RegionScan& g : scan)
+    if (!regions && !g.refused && order_regions(g, S, *P->R)) regions = &g;
   /* chains: a warp claims a chain and runs its blocks in order, so a block
    * whose deepest dependency is the block before it in its chain waits on
    * its own warp's work instead of a flag published on another SM.
@@ -1399,61 +1518,123 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
     ud[u] = static_cast<int>(key >> 32) + 1;
     max_depth = std::max(max_depth, ud[u]);
   }
-  std::vector<int>& height = S.height;
-  std::vector<int>& best = S.best;
-  height.assign(nu, 0);
-  best.assign(nu, -1);
-  for (size_t k = nu; k-- > 0;) {
-    const int u = static_cast<int>(k);  /* every block waiting for u is done: its height is final */
-    for (size_t j = first[u]; j < first[u + 1]; ++j) {
-      const int o = udeps[j];
-      height[o] = std::max(height[o], height[u] + 1);
+  auto build_chains = [&] {
+    std::vector<int>& height = S.height;
+    std::vector<int>& best = S.best;
+    height.assign(nu, 0);
+    best.assign(nu, -1);
+    for (size_t k = nu; k-- > 0;) {
+      const int u = static_cast<int>(k);  /* every block waiting for u is done: its height is final */
+      for (size_t j = first[u]; j < first[u + 1]; ++j) {
+        const int o = udeps[j];
+        height[o] = std::max(height[o], height[u] + 1);
+      }
+      const int cr = critv[u];
+      if (cr >= 0) {
+        const int bu = best[cr];  /* later in coding order than u */
+        if (bu < 0 || height[u] > height[bu] || (height[u] == height[bu] && ud[u] <= ud[bu])) best[cr] = u;
+      }
     }
-    const int cr = critv[u];
-    if (cr >= 0) {
-      const int bu = best[cr];  /* later in coding order than u */
-      if (bu < 0 || height[u] > height[bu] || (height[u] == height[bu] && ud[u] <= ud[bu])) best[cr] = u;
+    /* each block's chain, as the (depth, unit) key of its first block */
+    std::vector<uint64_t>& hk = S.head_key;
+    hk.resize(nu);
+    std::vector<int> count(max_depth + 2, 0);
+    for (size_t u = 0; u < nu; ++u) {
+      const int cr = critv[u];
+      const uint64_t own = (static_cast<uint64_t>(ud[u]) << 32) | static_cast<uint32_t>(u);
+      uint64_t h = own;
+      if (cr >= 0 && best[cr] == static_cast<int>(u)) {
+        const uint64_t hc = hk[cr];
+        bool ok = true;
+        for (size_t j = first[u]; j < first[u + 1]; ++j) ok &= hk[udeps[j]] <= hc;
+        if (ok) h = hc;
+      }
+      hk[u] = h;
+      if (h == own) ++count[ud[u] + 1];
     }
-  }
-  /* each block's chain, as the (depth, unit) key of its first block */
-  std::vector<uint64_t>& hk = S.head_key;
-  hk.resize(nu);
-  std::vector<int> count(max_depth + 2, 0);
-  for (size_t u = 0; u < nu; ++u) {
-    const int cr = critv[u];
-    const uint64_t own = (static_cast<uint64_t>(ud[u]) << 32) | static_cast<uint32_t>(u);
-    uint64_t h = own;
-    if (cr >= 0 && best[cr] == static_cast<int>(u)) {
-      const uint64_t hc = hk[cr];
-      bool ok = true;
-      for (size_t j = first[u]; j < first[u + 1]; ++j) ok &= hk[udeps[j]] <= hc;
-      if (ok) h = hc;
+    for (int k = 0; k <= max_depth; ++k) count[k + 1] += count[k];
+    const size_t nch = static_cast<size_t>(count[max_depth + 1]);
+    P->depth_first.assign(count.begin(), count.end());
+    std::vector<int>& cid = S.chain_id;  /* each block's chain, in claim order */
+    std::vector<int>& clen = S.chain_len;
+    cid.resize(nu);
+    clen.assign(nch + 1, 0);
+    for (size_t u = 0; u < nu; ++u) {
+      const int hu = static_cast<int>(static_cast<uint32_t>(hk[u]));
+      cid[u] = hu == static_cast<int>(u) ? count[ud[u]]++ : cid[hu];
+      ++clen[cid[u] + 1];
     }
-    hk[u] = h;
-    if (h == own) ++count[ud[u] + 1];
+    sized(P->R->chains, nch + 1);
+    for (size_t k = 0; k < nch; ++k) clen[k + 1] += clen[k];
+    for (size_t k = 0; k <= nch; ++k) P->R->chains[k] = clen[k];
+    for (size_t u = 0; u < nu; ++u) P->R->units[clen[cid[u]]++] = U[u];
+    P->n_chains = nch;
+    P->unit_depth = max_depth;
+  };
+  if (!regions) {
+    build_chains();
+    return AV1B_OK;
   }
-  for (int k = 0; k <= max_depth; ++k) count[k + 1] += count[k];
-  const size_t nch = static_cast<size_t>(count[max_depth + 1]);
-  P->depth_first.assign(count.begin(), count.end());
-  std::vector<int>& cid = S.chain_id;  /* each block's chain, in claim order */
-  std::vector<int>& clen = S.chain_len;
-  cid.resize(nu);
-  clen.assign(nch + 1, 0);
-  for (size_t u = 0; u < nu; ++u) {
-    const int hu = static_cast<int>(static_cast<uint32_t>(hk[u]));
-    cid[u] = hu == static_cast<int>(u) ? count[ud[u]]++ : cid[hu];
-    ++clen[cid[u] + 1];
-  }
-  sized(P->R->chains, nch + 1);
-  for (size_t k = 0; k < nch; ++k) clen[k + 1] += clen[k];
-  for (size_t k = 0; k <= nch; ++k) P->R->chains[k] = clen[k];
-  for (size_t u = 0; u < nu; ++u) P->R->units[clen[cid[u]]++] = U[u];
-  P->n_chains = nch;
-  P->unit_depth = max_depth;
-  P->units_inter = false;
-  for (int pi = 0; pi < pieces; ++pi)
-    if (inter_piece[pi]) P->units_inter = true;
-  if (!plan_regions(c, 6, P, U, first, udeps, ud)) plan_regions(c, 7, P, U, first, udeps, ud);
+  /* beside the chains, on the pool's other threads: the items into their
+   * regions, then each region's in order of depth (those tasks are claimed
+   * after the ones that place the items, and wait for them) */
+  P->region_log2 = regions->log2;
+  std::vector<uint64_t>& keys = S.region_keys;
+  std::vector<int>& at = S.region_at;   /* where each region's next key goes */
+  keys.resize(P->R->items.size());
+  for (const int4& r : P->R->regions) at[static_cast<size_t>(r.w) * regions->rw + r.z] = r.x;
+  auto place = [&](int pi) {
+    auto key = [&](size_t u, int part) {
+      return (static_cast<uint64_t>(ud[u]) << 32) | static_cast<uint32_t>(U[u] << 4 | part);
+    };
+    const size_t end = piece_begin(nu, pieces, pi + 1);
+    for (size_t u = piece_begin(nu, pieces, pi); u < end;) {
+      const int r = S.unit_region[u];
+      if (r >= 0) {
+        /* the units of one region that follow each other take their places at once */
+        size_t v = u + 1;
+        while (v < end && S.unit_region[v] == r) ++v;
+        int k = __atomic_fetch_add(&at[regions->log2 == 6 ? r : regions->larger(scan[0], r)], static_cast<int>(v - u),
+                                   __ATOMIC_RELAXED);
+        for (; u < v; ++u) keys[k++] = key(u, 0);
+        continue;
+      }
+      BlockRec& b = P->R->blocks[U[u]];
+      int across;
+      b.parts = static_cast<short>(regions->parts(b, &across));
+      for (int k = 0; k < b.parts; ++k)
+        keys[__atomic_fetch_add(&at[regions->region(b, b.parts, across, k)], 1, __ATOMIC_RELAXED)] = key(u, k);
+      ++u;
+    }
+  };
+  const size_t nr = P->R->regions.size();
+  const int rpieces = pieces_for(nr, c, 16);
+  auto sort_regions = [&](int pi) {
+    for (size_t r = piece_begin(nr, rpieces, pi); r < piece_begin(nr, rpieces, pi + 1); ++r) {
+      const int4 g = P->R->regions[r];
+      std::sort(keys.begin() + g.x, keys.begin() + g.x + g.y);
+      for (int k = g.x; k < g.x + g.y; ++k) {
+        const uint32_t id = static_cast<uint32_t>(keys[k]);
+        P->R->items[k] = static_cast<int>((id >> 4) | (id & 15) << AV1B_ITEM_SHIFT);
+      }
+    }
+  };
+  std::atomic<int> placed{0};
+  auto run_task = [&](int task) {
+    if (task == 0) return build_chains();
+    if (task <= pieces) {
+      place(task - 1);
+      placed.fetch_add(1, std::memory_order_release);
+      return;
+    }
+    while (placed.load(std::memory_order_acquire) != pieces) AV1B_CPU_RELAX();
+    sort_regions(task - 1 - pieces);
+  };
+  /* few units are sooner done than the pool is woken */
+  if (pieces == 1)
+    for (int task = 0; task < 1 + pieces + rpieces; ++task) run_task(task);
+  else
+    c.pool->run(1 + pieces + rpieces, run_task);
   return AV1B_OK;
 }
 
@@ -2104,6 +2285,13 @@ struct av1b_plan {
 namespace av1b {
 namespace {
 
+}  // namespace
+
+/* A batched step runs phase B by chains. */
+void plan_without_regions(av1b_decoder* d) { d->plan_regions.store(false); }
+
+namespace {
+
 /* Plans `s` into `pl`: validation, records, and the upload of records and
  * coefficient pools into the plan's device memory, on the upload stream. It
  * takes neither the decoder's lock nor its stream, so a pipeline plans frame
@@ -2160,6 +2348,7 @@ int plan_frame(av1b_decoder* d, const av1b_frame_syntax& s, av1b_plan* pl) {
   c.n_levels = s.n_levels;
   c.n_qm = s.n_qm_pool;
   c.share_masks = d->share_masks.load();
+  c.regions = d->plan_regions.load();
   const size_t n_coef = c.levels ? 0 : s.n_coefficients;
   if (!pl->ready) {
     /* blocking-sync events: a waiting planner sleeps instead of spinning on

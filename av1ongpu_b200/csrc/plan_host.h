@@ -7,7 +7,13 @@
 
 #include <cstdint>
 
+struct av1b_decoder;
+
 namespace av1b {
+
+/* The decoder's plans from now on are for batched steps only, which run phase
+ * B by chains: no regions are planned or uploaded (decoder.cu). */
+void plan_without_regions(av1b_decoder* d);
 
 /* setup_shear (7.11.3.6): alpha..delta of a global warp model. Returns false
  * when the shear is too steep (warpValid = 0). */

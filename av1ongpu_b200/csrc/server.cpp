@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "../../include/av1b.h"
+#include "plan_host.h"
 
 namespace {
 
@@ -505,6 +506,7 @@ int av1b_server_open(av1b_server* s, const av1b_stream_desc* desc, int* stream_i
   st->plan_cost_ms = px * 1.6e-6 / std::min(threads, 4);
   av1b_decoder_options dopt{1, threads};
   int rc = av1b_decoder_create_ex(s->opt.device, need - kOutRing * nv12, &dopt, &st->dec);
+  if (rc == AV1B_OK) av1b::plan_without_regions(st->dec);   /* every frame runs in a batched step */
   for (int i = 0; rc == AV1B_OK && i < ring_n; ++i) rc = av1b_reserve_reference(st->dec, &st->ring[i]);
   if (rc == AV1B_OK && nv12) {
     st->nv12_bytes = nv12;

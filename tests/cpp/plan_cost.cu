@@ -1,0 +1,63 @@
+/*
+ * plan_cost.cu - what planning phase B's regions costs (test infrastructure;
+ * no GPU needed).
+ *
+ * Plans seeded key frames with the planner compiled here, in turn with
+ * regions and without, and compares the fastest plan of each: the regions of
+ * a frame are to take a small part of its plan, since a caller that plans and
+ * decodes a frame at once waits for both. Prints "ok" at the end; exits
+ * non-zero on a failure.
+ */
+#define main plan_invariants_main
+#include "plan_invariants.cu"
+#undef main
+
+int main() {
+  av1b_decoder* d = new av1b_decoder;
+  WorkPool pool(4);
+  struct Case {
+    const char* name;
+    int w, h, cw, bd, sb, tools;
+  };
+  const int all = (1 << 16) - 1 - (1 << 13) - (1 << 11) - (1 << 12) - (1 << 14);
+  const Case cases[] = {{"720p", 1280, 720, 0, 8, 64, 0},
+                        {"1080p", 1920, 1080, 0, 10, 64, all},
+                        {"4K superres, 128x128 superblocks", 3840, 2160, 2880, 10, 128, all}};
+  for (const Case& cs : cases) {
+    uint8_t* blob = nullptr;
+    size_t len = 0;
+    if (av1s_synth_frame_ex(cs.w, cs.h, cs.cw, cs.bd, cs.sb, cs.tools, 5, 0, 30, &blob, &len) != AV1B_OK) return 1;
+    av1b_frame_syntax s;
+    av1b_syntax_view(blob, len, &s);
+    PlanCtx c;
+    c.L = make_layout(s.width, s.height, s.coded_width > 0 ? s.coded_width : s.width, s.bit_depth, s.ss_x, s.ss_y);
+    PlanScratch scratch;
+    PlanLists lists;
+    c.pool = &pool;
+    c.scratch = &scratch;
+    Plan P;
+    P.R = &lists;
+    double best[2] = {1e9, 1e9};
+    for (int k = 0; k < 24; ++k) {
+      c.regions = k & 1;
+      const auto t0 = std::chrono::steady_clock::now();
+      const int rc = build_plan(d, c, s, &P);
+      const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+      if (rc || lists.regions.empty() == c.regions) {
+        std::printf("FAIL: %s: plan %d, %zu regions\n", cs.name, rc, lists.regions.size());
+        return 1;
+      }
+      best[k & 1] = std::min(best[k & 1], ms);
+    }
+    std::printf("%s: %.2f ms without regions, %.2f with\n", cs.name, best[0], best[1]);
+    /* measured 1.02 to 1.08; 1.5 to 2.7 when it was a serial pass a size */
+    if (best[1] > 1.35 * best[0]) {
+      std::printf("FAIL: %s\n", cs.name);
+      ++failures;
+    }
+    av1s_blob_free(blob);
+  }
+  if (failures) return 1;
+  std::printf("ok\n");
+  return 0;
+}

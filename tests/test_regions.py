@@ -15,20 +15,28 @@ import test_plan_invariants as tpi
 from test_plan_invariants import have_nvcc  # noqa: F401
 
 
-def test_regions_only_wait_on_earlier_items(tmp_path, have_nvcc):  # noqa: F811
+def _run_checker(tmp_path, name, opt='-O2'):
     from av1ongpu_b200 import build as b
     b.build()
     objs = [os.path.join(b.OUT, f) for f in ('kernels.cu.o', 'plan_host.cpp.o', 'synth.cpp.o', 'blob.cpp.o',
                                              'api.cpp.o', 'noalloc.cu.o')]
-    exe = str(tmp_path / 'regions')
-    cmd = [tpi.NVCC, '-gencode', 'arch=compute_100a,code=sm_100a', '-O2', '-std=c++17', '-diag-suppress', '68',
+    exe = str(tmp_path / name)
+    cmd = [tpi.NVCC, '-gencode', 'arch=compute_100a,code=sm_100a', opt, '-std=c++17', '-diag-suppress', '68',
            '-I', tpi.CSRC, '-I', os.path.join(tpi.ROOT, 'include'),
-           os.path.join(tpi.ROOT, 'tests', 'cpp', 'regions.cu')] + objs + ['-o', exe, '-lpthread']
+           os.path.join(tpi.ROOT, 'tests', 'cpp', name + '.cu')] + objs + ['-o', exe, '-lpthread']
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-2000:]
     assert r.stdout.strip().endswith('ok')
+
+
+def test_regions_only_wait_on_earlier_items(tmp_path, have_nvcc):  # noqa: F811
+    _run_checker(tmp_path, 'regions')
+
+
+def test_regions_cost_a_small_part_of_the_plan(tmp_path, have_nvcc):  # noqa: F811
+    _run_checker(tmp_path, 'plan_cost', '-O3')
 
 
 def _decode(av1b, params, frames, traced):
