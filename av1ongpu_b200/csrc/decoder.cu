@@ -921,8 +921,9 @@ struct PlanScratch {
   std::vector<int> units_coding, ui_of, udepth, udeps;
   std::vector<uint8_t> is_b;
   std::vector<int> region_count[2], region_level, region_at, region_first, region_heirs;
-  std::vector<uint64_t> region_waits[2], region_keys;
-  std::vector<int> unit_region;       /* per unit: its 64x64 region when it is one item; -1 */
+  std::vector<uint64_t> region_waits[2];
+  std::vector<int> unit_region[2];    /* per unit, by size: its region when it is one item, else -1 */
+  std::vector<int> by_depth[4];
   std::vector<uint8_t> flagged;       /* blocks some block waits on by done flag */
   bool on_grid = false;               /* every block lies on its plane's owner cells */
   std::vector<uint16_t> itx_key;
@@ -953,13 +954,16 @@ inline size_t piece_begin(size_t n, int pieces, int i) { return n * i / pieces; 
  *
  * What it costs is one look at each block for both sizes, which the pool's
  * threads share and which goes with the pass that writes the block's
- * dependency list (RegionScan::block), and placing and sorting the items,
- * which go beside the chains; the graph has a node a region and a few edges
- * each, and only a size whose graph has no circle gets lists. A key frame's
- * plan on seven threads, without regions / with them: 720p 3.5 / 3.8 ms, 1080p
- * 6.1 / 6.5, 4K with 128x128 superblocks 13.2 / 13.4. As one serial pass a
- * size that swept the blocks' dependency lists until the levels stood: 5.7,
- * 10.7 and 39 ms. */
+ * dependency list (RegionScan::block), and placing the items, which goes
+ * beside the chains; the graph has a node a region and a few edges each, and
+ * only a size whose graph has no circle gets lists. A key frame's plan on
+ * seven threads, without regions / with them: 720p 3.7 / 3.9 ms, 1080p 6.5 /
+ * 7.1, 4K with 128x128 superblocks 13.8 / 14.9. As one serial pass a size that
+ * swept the blocks' dependency lists until the levels stood: 5.7, 10.7 and 39
+ * ms. The placing takes no more tasks than that, and none that wait for
+ * others: three planners' threads share the cores, and tasks that sorted each
+ * region and spun until all items were placed cost an end-to-end 4K stream a
+ * quarter of its rate (400 of 540 frames/s). */
 struct RegionScan {
   Layout L;
   const BlockRec* blocks = nullptr;
@@ -1451,7 +1455,7 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
       std::all_of(P->R->palette_colors.begin(), P->R->palette_colors.end(), [](int v) { return v >= 0 && v <= 4095; })) {
     scan[0].start(L, *P->R, 6, S.region_count[0], S.region_waits[0]);
     if (L.ss_x && L.ss_y) scan[1].start(L, *P->R, 7, S.region_count[1], S.region_waits[1]);
-    S.unit_region.resize(nu);
+    for (auto& v : S.unit_region) v.resize(nu);
   }
   const bool by_regions = !scan[0].refused;
   c.pool->run(pieces, [&](int pi) {
@@ -1467,11 +1471,11 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
       if (by_regions) {
         b.parts = 1;
         bool inner, large;
-        S.unit_region[ui] = scan[0].block(b, run[0], &inner);
+        const int r = S.unit_region[0][ui] = scan[0].block(b, run[0], &inner);
         if (!inner)
-          scan[1].block(b, run[1], &large);
+          S.unit_region[1][ui] = scan[1].block(b, run[1], &large);
         else if (!scan[1].refused.load(std::memory_order_relaxed))
-          scan[1].add(run[1], scan[1].larger(scan[0], S.unit_region[ui]), 1, 0);
+          scan[1].add(run[1], S.unit_region[1][ui] = scan[1].larger(scan[0], r), 1, 0);
       }
     }
     for (int k = 0; k < 2; ++k) scan[k].flush(run[k]);
@@ -1575,66 +1579,43 @@ int plan_units(av1b_decoder* d, const PlanCtx& c, Plan* P) {
     build_chains();
     return AV1B_OK;
   }
-  /* beside the chains, on the pool's other threads: the items into their
-   * regions, then each region's in order of depth (those tasks are claimed
-   * after the ones that place the items, and wait for them) */
+  /* beside the chains: the units by depth, a counting sort, into their
+   * regions; of many units on a large pool, every fourth region a task */
   P->region_log2 = regions->log2;
-  std::vector<uint64_t>& keys = S.region_keys;
-  std::vector<int>& at = S.region_at;   /* where each region's next key goes */
-  keys.resize(P->R->items.size());
+  const std::vector<int>& region_of = S.unit_region[regions == &scan[1]];
+  const int tasks = nu < 16384 || c.pool->threads() < 5 ? 1 : 4;
+  std::vector<int>& at = S.region_at;   /* where each region's next item goes */
   for (const int4& r : P->R->regions) at[static_cast<size_t>(r.w) * regions->rw + r.z] = r.x;
-  auto place = [&](int pi) {
-    auto key = [&](size_t u, int part) {
-      return (static_cast<uint64_t>(ud[u]) << 32) | static_cast<uint32_t>(U[u] << 4 | part);
+  auto fill_regions = [&](int part) {
+    auto mine = [&](int region) { return (region & (tasks - 1)) == part; };
+    /* its units, and those of several items */
+    auto each = [&](auto&& f) {
+      for (size_t u = 0; u < nu; ++u)
+        if (region_of[u] < 0 || mine(region_of[u])) f(u);
     };
-    const size_t end = piece_begin(nu, pieces, pi + 1);
-    for (size_t u = piece_begin(nu, pieces, pi); u < end;) {
-      const int r = S.unit_region[u];
+    std::vector<int>& order = S.by_depth[part];
+    std::vector<int> depth_at(max_depth + 2, 0);
+    each([&](size_t u) { ++depth_at[ud[u] + 1]; });
+    for (int k = 0; k <= max_depth; ++k) depth_at[k + 1] += depth_at[k];
+    order.resize(depth_at[max_depth + 1]);
+    each([&](size_t u) { order[depth_at[ud[u]]++] = static_cast<int>(u); });
+    for (int u : order) {
+      const int r = region_of[u];
       if (r >= 0) {
-        /* the units of one region that follow each other take their places at once */
-        size_t v = u + 1;
-        while (v < end && S.unit_region[v] == r) ++v;
-        int k = __atomic_fetch_add(&at[regions->log2 == 6 ? r : regions->larger(scan[0], r)], static_cast<int>(v - u),
-                                   __ATOMIC_RELAXED);
-        for (; u < v; ++u) keys[k++] = key(u, 0);
+        P->R->items[at[r]++] = U[u];
         continue;
       }
       BlockRec& b = P->R->blocks[U[u]];
       int across;
-      b.parts = static_cast<short>(regions->parts(b, &across));
-      for (int k = 0; k < b.parts; ++k)
-        keys[__atomic_fetch_add(&at[regions->region(b, b.parts, across, k)], 1, __ATOMIC_RELAXED)] = key(u, k);
-      ++u;
-    }
-  };
-  const size_t nr = P->R->regions.size();
-  const int rpieces = pieces_for(nr, c, 16);
-  auto sort_regions = [&](int pi) {
-    for (size_t r = piece_begin(nr, rpieces, pi); r < piece_begin(nr, rpieces, pi + 1); ++r) {
-      const int4 g = P->R->regions[r];
-      std::sort(keys.begin() + g.x, keys.begin() + g.x + g.y);
-      for (int k = g.x; k < g.x + g.y; ++k) {
-        const uint32_t id = static_cast<uint32_t>(keys[k]);
-        P->R->items[k] = static_cast<int>((id >> 4) | (id & 15) << AV1B_ITEM_SHIFT);
+      const int n = regions->parts(b, &across);
+      if (part == 0) b.parts = static_cast<short>(n);
+      for (int k = 0; k < n; ++k) {
+        const int region = regions->region(b, n, across, k);
+        if (mine(region)) P->R->items[at[region]++] = U[u] | k << AV1B_ITEM_SHIFT;
       }
     }
   };
-  std::atomic<int> placed{0};
-  auto run_task = [&](int task) {
-    if (task == 0) return build_chains();
-    if (task <= pieces) {
-      place(task - 1);
-      placed.fetch_add(1, std::memory_order_release);
-      return;
-    }
-    while (placed.load(std::memory_order_acquire) != pieces) AV1B_CPU_RELAX();
-    sort_regions(task - 1 - pieces);
-  };
-  /* few units are sooner done than the pool is woken */
-  if (pieces == 1)
-    for (int task = 0; task < 1 + pieces + rpieces; ++task) run_task(task);
-  else
-    c.pool->run(1 + pieces + rpieces, run_task);
+  c.pool->run(1 + tasks, [&](int task) { task ? fill_regions(task - 1) : build_chains(); });
   return AV1B_OK;
 }
 
