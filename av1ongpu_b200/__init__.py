@@ -215,6 +215,9 @@ _SYNTH_SIGNATURES = {
                                              ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_uint64,
                                              ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_void_p),
                                              ctypes.POINTER(ctypes.c_size_t)]),
+    'av1s_synth_frame_format': (ctypes.c_int, [ctypes.c_int] * 9 + [ctypes.c_uint64, ctypes.c_int, ctypes.c_int,
+                                                                    ctypes.POINTER(ctypes.c_void_p),
+                                                                    ctypes.POINTER(ctypes.c_size_t)]),
     'av1s_blob_free': (None, [ctypes.c_void_p]),
 }
 _synth = None
@@ -345,6 +348,19 @@ def synth_frame_ex(width, height, coded_width, bit_depth, sb_size, tools, seed, 
                                                ctypes.byref(p), ctypes.byref(n))
     if rc:
         raise Av1bError(rc, 'synth_frame_ex')
+    return Blob(p.value, n.value, True)
+
+
+def synth_frame_format(width, height, coded_width, bit_depth, ss_x, ss_y, sb_size, tools, seed, index,
+                       key_interval=30, max_refs=3):
+    """synth_frame_ex in 4:2:0 (ss_x and ss_y 1), 4:2:2 (1, 0) or 4:4:4 (0, 0)."""
+    p = ctypes.c_void_p()
+    n = ctypes.c_size_t()
+    rc = synth_lib().av1s_synth_frame_format(width, height, coded_width, bit_depth, ss_x, ss_y, sb_size, tools,
+                                             max_refs, seed, index, key_interval, ctypes.byref(p),
+                                             ctypes.byref(n))
+    if rc:
+        raise Av1bError(rc, 'synth_frame_format')
     return Blob(p.value, n.value, True)
 
 

@@ -92,6 +92,7 @@ struct Params {
   int tools = 0;
   int key_interval = 30;
   int max_refs = 1;
+  int ss_x = 1, ss_y = 1;
 };
 
 struct Tile {
@@ -108,8 +109,8 @@ class Generator {
     cw = P.coded_width > 0 ? P.coded_width : P.width;
     grid_w[0] = (cw + 7) & ~7;
     grid_h[0] = (P.height + 7) & ~7;
-    grid_w[1] = grid_w[2] = grid_w[0] >> 1;
-    grid_h[1] = grid_h[2] = grid_h[0] >> 1;
+    grid_w[1] = grid_w[2] = grid_w[0] >> P.ss_x;
+    grid_h[1] = grid_h[2] = grid_h[0] >> P.ss_y;
     maxv = (1 << P.bit_depth) - 1;
     lossless = (P.tools & kToolLossless) != 0;
   }
@@ -145,8 +146,8 @@ class Generator {
     h.coded_width = P.coded_width > 0 && P.coded_width != P.width ? P.coded_width : 0;
     h.height = P.height;
     h.bit_depth = P.bit_depth;
-    h.ss_x = 1;
-    h.ss_y = 1;
+    h.ss_x = P.ss_x;
+    h.ss_y = P.ss_y;
     h.base_q_idx = rng.range(20, 200);
     h.sharpness = has(kToolEdgeVariants) ? rng.range(0, 7) : 0;
     h.enable_intra_edge_filter = 1;
@@ -335,8 +336,8 @@ class Generator {
     const bool filter_intra = !palette && has(kToolFilterIntra) && s <= 32 && rng.chance(1, 7);
     const int fi_mode = rng.range(0, 4);
     for (int plane = 0; plane < 3; ++plane) {
-      const int sub = plane ? 1 : 0;
-      const int px = x >> sub, py = y >> sub, ps = s >> sub;
+      const int sx = plane ? P.ss_x : 0, sy = plane ? P.ss_y : 0;
+      const int px = x >> sx, py = y >> sy, pw = s >> sx, ph = s >> sy;
       /* this plane's palette and colour map */
       int colors[8] = {0};
       int pal_size = 0;
@@ -346,21 +347,24 @@ class Generator {
         for (int i = 0; i < pal_size; ++i) colors[i] = rng.range(0, maxv);
         std::sort(colors, colors + pal_size);
         pal_base = f->palette_map.size();
-        f->palette_map.resize(pal_base + static_cast<size_t>(ps) * ps);
+        f->palette_map.resize(pal_base + static_cast<size_t>(pw) * ph);
         uint8_t* map = f->palette_map.data() + pal_base;
         int run = rng.range(0, pal_size - 1);
-        for (int i = 0; i < ps * ps; ++i) {
+        for (int i = 0; i < pw * ph; ++i) {
           if (rng.chance(1, 4)) run = rng.range(0, pal_size - 1);
           map[i] = static_cast<uint8_t>(run);
         }
       }
-      const bool cfl = plane > 0 && !palette && has(kToolCfl) && ps <= 32 && rng.chance(1, 4);
+      const bool cfl = plane > 0 && !palette && has(kToolCfl) && std::max(pw, ph) <= 32 && rng.chance(1, 4);
       const int cfl_alpha = rng.range(-16, 16);
       int tw, th;
-      pick_tx(ps, ps, &tw, &th);
-      if (cfl) tw = th = std::min(ps, 32);
-      for (int ty = 0; ty < ps; ty += th)
-        for (int tx = 0; tx < ps; tx += tw) {
+      pick_tx(pw, ph, &tw, &th);
+      if (cfl) {
+        tw = std::min(pw, 32);
+        th = std::min(ph, 32);
+      }
+      for (int ty = 0; ty < ph; ty += th)
+        for (int tx = 0; tx < pw; tx += tw) {
           av1b_block b = new_block(plane, px + tx, py + ty, tw, th);
           b.is_intra = 1;
           b.mode = rng.range(0, 12);
@@ -380,8 +384,8 @@ class Generator {
             b.mode = 0;
             b.palette_size = pal_size;
             for (int i = 0; i < 8; ++i) b.palette[i] = colors[i];
-            b.palette_off = static_cast<int32_t>(pal_base + static_cast<size_t>(ty) * ps + tx);
-            b.palette_stride = ps;
+            b.palette_off = static_cast<int32_t>(pal_base + static_cast<size_t>(ty) * pw + tx);
+            b.palette_stride = pw;
           }
           const bool residual = rng.chance(4, 5);
           add_transforms(&b, plane, tw, th, residual, true, tw, th);
@@ -404,8 +408,8 @@ class Generator {
     const int sx = std::max(0, std::min(grid_w[0] - s, x + rng.range(-8, 8) * 8));
     const int mvx = (sx - x) * 8, mvy = (sy - y) * 8;
     for (int plane = 0; plane < 3; ++plane) {
-      const int sub = plane ? 1 : 0;
-      av1b_block b = new_block(plane, x >> sub, y >> sub, s >> sub, s >> sub);
+      const int sx = plane ? P.ss_x : 0, sy = plane ? P.ss_y : 0;
+      av1b_block b = new_block(plane, x >> sx, y >> sy, s >> sx, s >> sy);
       b.is_intra = 0;
       b.intrabc = 1;
       b.mv[0][0] = mvx;
@@ -472,8 +476,8 @@ class Generator {
     int tw = 0, th = 0;
     pick_tx(std::min(s, 64), std::min(s, 64), &tw, &th);
     for (int plane = 0; plane < 3; ++plane) {
-      const int sub = plane ? 1 : 0;
-      av1b_block b = new_block(plane, x >> sub, y >> sub, s >> sub, s >> sub);
+      const int sx = plane ? P.ss_x : 0, sy = plane ? P.ss_y : 0;
+      av1b_block b = new_block(plane, x >> sx, y >> sy, s >> sx, s >> sy);
       b.is_intra = 0;
       b.ref[0] = ref0;
       b.ref[1] = ref1;
@@ -514,10 +518,10 @@ class Generator {
       for (const Strip& st : strips) {
         av1b_obmc o;
         o.pass = st.pass;
-        o.x = st.x >> sub;
-        o.y = st.y >> sub;
-        o.w = st.w >> sub;
-        o.h = st.h >> sub;
+        o.x = st.x >> sx;
+        o.y = st.y >> sy;
+        o.w = st.w >> sx;
+        o.h = st.h >> sy;
         o.mv[0] = st.mvx;
         o.mv[1] = st.mvy;
         o.filter = st.filt;
@@ -532,10 +536,11 @@ class Generator {
         add_residual(&b);
       } else if (skip) {
         /* a skipped block still has its prediction edges deblocked */
-        const int e = std::min(b.w, 64 >> sub);
-        add_transforms(&b, plane, b.w, b.h, false, true, e, std::min(b.h, 64 >> sub));
+        const int e = std::min(b.w, 64 >> sx);
+        add_transforms(&b, plane, b.w, b.h, false, true, e, std::min(b.h, 64 >> sy));
       } else {
-        const int ptw = std::max(4, tw >> sub), pth = std::max(4, th >> sub);
+        int ptw = std::max(4, tw >> sx), pth = std::max(4, th >> sy);
+        while (pth > 4 * ptw) pth >>= 1; /* 4:2:2 of a 1:4 tile */
         add_transforms(&b, plane, b.w, b.h, true, true, std::min(ptw, b.w), std::min(pth, b.h));
       }
       f->blocks.push_back(b);
@@ -630,7 +635,7 @@ class Generator {
             f->cdef.push_back(av1b_cdef_block{0, x, y, preset[idx][0], preset[idx][1], damping, -1});
             for (int p = 1; p < 3; ++p)
               f->cdef.push_back(
-                  av1b_cdef_block{p, x >> 1, y >> 1, preset[idx][2], preset[idx][3], damping, -1});
+                  av1b_cdef_block{p, x >> P.ss_x, y >> P.ss_y, preset[idx][2], preset[idx][3], damping, -1});
           }
       }
   }
@@ -638,8 +643,8 @@ class Generator {
   /* ---- loop restoration ---------------------------------------------------- */
   void restoration() {
     for (int p = 0; p < 3; ++p) {
-      const int sub = p ? 1 : 0;
-      const int pw = (P.width + sub) >> sub, ph = (P.height + sub) >> sub;
+      const int sx = p ? P.ss_x : 0, sy = p ? P.ss_y : 0;
+      const int pw = (P.width + sx) >> sx, ph = (P.height + sy) >> sy;
       const int cols = std::max((pw + 32) >> 6, 1), rows = std::max((ph + 32) >> 6, 1);
       f->hdr.restoration_type[p] = 1; /* switchable: every unit picks */
       f->hdr.restoration_unit_log2[p] = 6;
@@ -789,21 +794,31 @@ int av1s_synth_frame(int config, int scale, uint64_t seed, int frame_index, uint
   return synth_to_blob(p, seed, frame_index, blob, len);
 }
 
-int av1s_synth_frame_refs(int width, int height, int coded_width, int bit_depth, int sb_size,
-                          int tools, int max_refs, uint64_t seed, int frame_index, int key_interval,
-                          uint8_t** blob, size_t* len) {
+int av1s_synth_frame_format(int width, int height, int coded_width, int bit_depth, int ss_x, int ss_y,
+                            int sb_size, int tools, int max_refs, uint64_t seed, int frame_index,
+                            int key_interval, uint8_t** blob, size_t* len) {
   av1b::Params p;
   p.width = width;
   p.height = height;
   p.coded_width = coded_width;
   p.bit_depth = bit_depth;
+  p.ss_x = ss_x;
+  p.ss_y = ss_y;
   p.sb = sb_size == 128 ? 128 : 64;
   p.tools = tools;
   p.key_interval = key_interval > 0 ? key_interval : (1 << 30);
   p.max_refs = max_refs;
   if (bit_depth != 8 && bit_depth != 10 && bit_depth != 12) return AV1B_ERR_ARG;
   if (max_refs < 1 || max_refs > 3) return AV1B_ERR_ARG;
+  if (ss_x < 0 || ss_x > 1 || ss_y < 0 || ss_y > ss_x) return AV1B_ERR_ARG;
   return synth_to_blob(p, seed, frame_index, blob, len);
+}
+
+int av1s_synth_frame_refs(int width, int height, int coded_width, int bit_depth, int sb_size,
+                          int tools, int max_refs, uint64_t seed, int frame_index, int key_interval,
+                          uint8_t** blob, size_t* len) {
+  return av1s_synth_frame_format(width, height, coded_width, bit_depth, 1, 1, sb_size, tools, max_refs,
+                                 seed, frame_index, key_interval, blob, len);
 }
 
 int av1s_synth_frame_ex(int width, int height, int coded_width, int bit_depth, int sb_size,

@@ -49,6 +49,10 @@ AV1S_API int av1s_synth_frame_ex(int width, int height, int coded_width, int bit
 AV1S_API int av1s_synth_frame_refs(int width, int height, int coded_width, int bit_depth,
                                    int sb_size, int tools, int max_refs, uint64_t seed,
                                    int frame_index, int key_interval, uint8_t** blob, size_t* len);
+/* The same in 4:2:0 (ss_x and ss_y 1), 4:2:2 (ss_x 1, ss_y 0) or 4:4:4. */
+AV1S_API int av1s_synth_frame_format(int width, int height, int coded_width, int bit_depth, int ss_x,
+                                     int ss_y, int sb_size, int tools, int max_refs, uint64_t seed,
+                                     int frame_index, int key_interval, uint8_t** blob, size_t* len);
 AV1S_API void av1s_blob_free(uint8_t* blob);
 
 #ifdef __cplusplus
