@@ -33,6 +33,7 @@ TOOL_FILTER_INTRA, TOOL_COMPOUND, TOOL_MASKS, TOOL_OBMC = 16, 32, 64, 128
 TOOL_WARP, TOOL_LR, TOOL_GRAIN, TOOL_INTERINTRA = 256, 512, 1024, 2048
 TOOL_INTRABC, TOOL_LOSSLESS, TOOL_RESIDUAL, TOOL_EDGE_VARIANTS = 4096, 8192, 16384, 32768
 TOOL_NO_DEBLOCK, TOOL_NO_CDEF = 1 << 16, 1 << 17
+TOOL_422, TOOL_444 = 1 << 18, 1 << 19
 TOOLS_ALL = (TOOL_TX64 | TOOL_ALLTYPES | TOOL_CFL | TOOL_PALETTE | TOOL_FILTER_INTRA |
              TOOL_COMPOUND | TOOL_MASKS | TOOL_OBMC | TOOL_WARP | TOOL_LR | TOOL_GRAIN |
              TOOL_EDGE_VARIANTS)
@@ -215,9 +216,6 @@ _SYNTH_SIGNATURES = {
                                              ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_uint64,
                                              ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_void_p),
                                              ctypes.POINTER(ctypes.c_size_t)]),
-    'av1s_synth_frame_format': (ctypes.c_int, [ctypes.c_int] * 9 + [ctypes.c_uint64, ctypes.c_int, ctypes.c_int,
-                                                                    ctypes.POINTER(ctypes.c_void_p),
-                                                                    ctypes.POINTER(ctypes.c_size_t)]),
     'av1s_blob_free': (None, [ctypes.c_void_p]),
 }
 _synth = None
@@ -348,19 +346,6 @@ def synth_frame_ex(width, height, coded_width, bit_depth, sb_size, tools, seed, 
                                                ctypes.byref(p), ctypes.byref(n))
     if rc:
         raise Av1bError(rc, 'synth_frame_ex')
-    return Blob(p.value, n.value, True)
-
-
-def synth_frame_format(width, height, coded_width, bit_depth, ss_x, ss_y, sb_size, tools, seed, index,
-                       key_interval=30, max_refs=3):
-    """synth_frame_ex in 4:2:0 (ss_x and ss_y 1), 4:2:2 (1, 0) or 4:4:4 (0, 0)."""
-    p = ctypes.c_void_p()
-    n = ctypes.c_size_t()
-    rc = synth_lib().av1s_synth_frame_format(width, height, coded_width, bit_depth, ss_x, ss_y, sb_size, tools,
-                                             max_refs, seed, index, key_interval, ctypes.byref(p),
-                                             ctypes.byref(n))
-    if rc:
-        raise Av1bError(rc, 'synth_frame_format')
     return Blob(p.value, n.value, True)
 
 

@@ -64,6 +64,8 @@ enum Tool : int {
   kToolEdgeVariants = 1 << 15, /* filter_type and sharpness variations    */
   kToolNoDeblock = 1 << 16,  /* leave the deblocking edge list empty      */
   kToolNoCdef = 1 << 17,     /* leave the CDEF block list empty           */
+  kTool422 = 1 << 18,        /* 4:2:2, not 4:2:0                          */
+  kTool444 = 1 << 19,        /* 4:4:4, not 4:2:0                          */
 };
 
 constexpr int kToolsAll = kToolTx64 | kToolAllTypes | kToolCfl | kToolPalette |
@@ -794,31 +796,23 @@ int av1s_synth_frame(int config, int scale, uint64_t seed, int frame_index, uint
   return synth_to_blob(p, seed, frame_index, blob, len);
 }
 
-int av1s_synth_frame_format(int width, int height, int coded_width, int bit_depth, int ss_x, int ss_y,
-                            int sb_size, int tools, int max_refs, uint64_t seed, int frame_index,
-                            int key_interval, uint8_t** blob, size_t* len) {
+int av1s_synth_frame_refs(int width, int height, int coded_width, int bit_depth, int sb_size,
+                          int tools, int max_refs, uint64_t seed, int frame_index, int key_interval,
+                          uint8_t** blob, size_t* len) {
   av1b::Params p;
   p.width = width;
   p.height = height;
   p.coded_width = coded_width;
   p.bit_depth = bit_depth;
-  p.ss_x = ss_x;
-  p.ss_y = ss_y;
+  p.ss_x = tools & av1b::kTool444 ? 0 : 1;
+  p.ss_y = tools & (av1b::kTool422 | av1b::kTool444) ? 0 : 1;
   p.sb = sb_size == 128 ? 128 : 64;
   p.tools = tools;
   p.key_interval = key_interval > 0 ? key_interval : (1 << 30);
   p.max_refs = max_refs;
   if (bit_depth != 8 && bit_depth != 10 && bit_depth != 12) return AV1B_ERR_ARG;
   if (max_refs < 1 || max_refs > 3) return AV1B_ERR_ARG;
-  if (ss_x < 0 || ss_x > 1 || ss_y < 0 || ss_y > ss_x) return AV1B_ERR_ARG;
   return synth_to_blob(p, seed, frame_index, blob, len);
-}
-
-int av1s_synth_frame_refs(int width, int height, int coded_width, int bit_depth, int sb_size,
-                          int tools, int max_refs, uint64_t seed, int frame_index, int key_interval,
-                          uint8_t** blob, size_t* len) {
-  return av1s_synth_frame_format(width, height, coded_width, bit_depth, 1, 1, sb_size, tools, max_refs,
-                                 seed, frame_index, key_interval, blob, len);
 }
 
 int av1s_synth_frame_ex(int width, int height, int coded_width, int bit_depth, int sb_size,

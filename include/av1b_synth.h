@@ -38,7 +38,8 @@ extern "C" {
  * size divided by `scale` (1 = full size). */
 AV1S_API int av1s_synth_frame(int config, int scale, uint64_t seed, int frame_index, uint8_t** blob,
                               size_t* len);
-/* A frame of any geometry: `tools` is a mask of the generator's tool bits
+/* A frame of any geometry: `tools` is a mask of the generator's tool bits,
+ * the chroma formats 4:2:2 (bit 18) and 4:4:4 (bit 19) among them
  * (compound prediction among them selects up to three references), a key
  * frame every `key_interval` frames (0: only the first). */
 AV1S_API int av1s_synth_frame_ex(int width, int height, int coded_width, int bit_depth, int sb_size,
@@ -49,10 +50,6 @@ AV1S_API int av1s_synth_frame_ex(int width, int height, int coded_width, int bit
 AV1S_API int av1s_synth_frame_refs(int width, int height, int coded_width, int bit_depth,
                                    int sb_size, int tools, int max_refs, uint64_t seed,
                                    int frame_index, int key_interval, uint8_t** blob, size_t* len);
-/* The same in 4:2:0 (ss_x and ss_y 1), 4:2:2 (ss_x 1, ss_y 0) or 4:4:4. */
-AV1S_API int av1s_synth_frame_format(int width, int height, int coded_width, int bit_depth, int ss_x,
-                                     int ss_y, int sb_size, int tools, int max_refs, uint64_t seed,
-                                     int frame_index, int key_interval, uint8_t** blob, size_t* len);
 AV1S_API void av1s_blob_free(uint8_t* blob);
 
 #ifdef __cplusplus

@@ -146,26 +146,24 @@ int main() {
   WorkPool pool(3);
   struct Case {
     const char* name;
-    int w, h, cw, bd, sb, tools, frames, ss_x, ss_y;
+    int w, h, cw, bd, sb, tools, frames;
   };
   const int all = (1 << 16) - 1 - (1 << 13) - (1 << 11) - (1 << 12);
   const Case cases[] = {
-      {"720p basic", 1280, 720, 0, 8, 64, 0, 2, 1, 1},
-      {"odd size", 998, 514, 750, 12, 128, all & ~(1 << 14), 3, 1, 1},
-      {"tiny", 16, 16, 0, 8, 64, all, 2, 1, 1},
-      {"raw residuals", 240, 136, 0, 10, 64, all, 3, 1, 1},
-      {"4K superres", 3840, 2160, 2880, 10, 128, all & ~(1 << 14), 2, 1, 1},
-      {"inter blocks in phase B", 640, 360, 0, 8, 64, (1 << 16) - 1 - (1 << 13), 2, 1, 1},
-      {"4:2:2", 338, 206, 0, 8, 64, all, 3, 1, 0},
-      {"4:4:4", 338, 206, 0, 10, 64, all, 3, 0, 0},
+      {"720p basic", 1280, 720, 0, 8, 64, 0, 2},
+      {"odd size", 998, 514, 750, 12, 128, all & ~(1 << 14), 3},
+      {"tiny", 16, 16, 0, 8, 64, all, 2},
+      {"raw residuals", 240, 136, 0, 10, 64, all, 3},
+      {"4K superres", 3840, 2160, 2880, 10, 128, all & ~(1 << 14), 2},
+      {"inter blocks in phase B", 640, 360, 0, 8, 64, (1 << 16) - 1 - (1 << 13), 2},
+      {"4:2:2", 338, 206, 0, 8, 64, all | (1 << 18), 3},
+      {"4:4:4", 338, 206, 0, 10, 64, all | (1 << 19), 3},
   };
   for (const Case& cs : cases)
     for (int k = 0; k < cs.frames; ++k) {
       uint8_t* blob = nullptr;
       size_t len = 0;
-      if (av1s_synth_frame_format(cs.w, cs.h, cs.cw, cs.bd, cs.ss_x, cs.ss_y, cs.sb, cs.tools, cs.tools & (1 << 5) ? 3 : 1,
-                                  5, k, 30, &blob, &len) != AV1B_OK)
-        return 1;
+      if (av1s_synth_frame_ex(cs.w, cs.h, cs.cw, cs.bd, cs.sb, cs.tools, 5, k, 30, &blob, &len) != AV1B_OK) return 1;
       check_frame(d, &pool, blob, len, cs.name, k, kSome);
       av1s_blob_free(blob);
     }

@@ -18,18 +18,18 @@ FORMATS = os.path.join(os.path.dirname(os.path.abspath(__file__)), 'golden', 'fo
 
 def cases(A):
     ext = A.TOOLS_ALL | A.TOOL_INTERINTRA | A.TOOL_INTRABC | A.TOOL_RESIDUAL
-    # name: (width, height, coded_width, bit_depth, ss_x, ss_y, superblock, tools), frames
+    # name: (width, height, coded_width, bit_depth, superblock, tools), frames
     return {
-        '422': ((338, 206, 0, 8, 1, 0, 64, ext), 3),
-        '444': ((338, 206, 0, 10, 0, 0, 64, ext), 3),
-        '422_superres': ((360, 200, 270, 12, 1, 0, 128, A.TOOLS_ALL), 3),
-        '444_superres': ((320, 182, 200, 8, 0, 0, 128, A.TOOLS_ALL), 3),
-        '422_larger': ((1416, 798, 0, 10, 1, 0, 128, A.TOOLS_ALL), 2),
-        '444_larger': ((1416, 798, 0, 8, 0, 0, 64, A.TOOLS_ALL), 2),
-        'grain_alone': ((200, 120, 0, 10, 1, 1, 64,
+        '422': ((338, 206, 0, 8, 64, ext | A.TOOL_422), 3),
+        '444': ((338, 206, 0, 10, 64, ext | A.TOOL_444), 3),
+        '422_superres': ((360, 200, 270, 12, 128, A.TOOLS_ALL | A.TOOL_422), 3),
+        '444_superres': ((320, 182, 200, 8, 128, A.TOOLS_ALL | A.TOOL_444), 3),
+        '422_larger': ((1416, 798, 0, 10, 128, A.TOOLS_ALL | A.TOOL_422), 2),
+        '444_larger': ((1416, 798, 0, 8, 64, A.TOOLS_ALL | A.TOOL_444), 2),
+        'grain_alone': ((200, 120, 0, 10, 64,
                          (A.TOOLS_ALL & ~A.TOOL_LR) | A.TOOL_NO_DEBLOCK | A.TOOL_NO_CDEF), 4),
-        'few_blocks': ((32, 24, 0, 8, 1, 1, 64, A.TOOLS_ALL), 12),
-        'few_blocks_unfiltered': ((40, 24, 0, 10, 1, 1, 64,
+        'few_blocks': ((32, 24, 0, 8, 64, A.TOOLS_ALL), 12),
+        'few_blocks_unfiltered': ((40, 24, 0, 10, 64,
                                    (A.TOOLS_ALL & ~A.TOOL_LR) | A.TOOL_NO_DEBLOCK | A.TOOL_NO_CDEF), 12),
     }
 
@@ -42,7 +42,7 @@ def frames(dec, av1b, params, n):
     """Hashes of each frame's planes."""
     slots, out = [], []
     for k in range(n):
-        b = av1b.synth_frame_format(*params, 515, k)
+        b = av1b.synth_frame_ex(*params, 515, k, 30)
         b.set_refs([slots[k - x] for x in b.get_refs()])
         slot, planes = dec.decode(b)
         slots.append(slot)
@@ -76,13 +76,14 @@ def test_planned_frames_of_a_format(av1b, name):
     if not av1b.cuda_available():
         pytest.skip('no CUDA device')
     params, n = cases(av1b)[name]
-    w, h, _cw, _bd, ss_x, ss_y = params[:6]
+    w, h, tools = params[0], params[1], params[5]
+    ss_x, ss_y = int(not tools & av1b.TOOL_444), int(not tools & (av1b.TOOL_422 | av1b.TOOL_444))
     dec = av1b.Decoder(0)
     slots = [dec.reserve_reference() for _ in range(4)]
     plans, none = [], 0
     # enough plans ahead that a frame is queued while the one before it runs
     for k in range(n):
-        b = av1b.synth_frame_format(*params, 515, k)
+        b = av1b.synth_frame_ex(*params, 515, k, 30)
         b.set_refs([slots[(k - x) % 4] for x in b.get_refs()])
         plans.append(dec.plan(b))
         none += k > 0 and dec.plan_stats(plans[-1])['phase_b_blocks'] == 0
