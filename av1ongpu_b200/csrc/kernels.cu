@@ -2405,7 +2405,6 @@ __global__ void __launch_bounds__(256) k_grain_template(GrainState* gs, const in
                                                         const uint16_t* orbit, const uint16_t* pos) {
   __shared__ GrainTemplateSmem sm;
   grain_template_body(gs, gs_src, prm, orbit, pos, sm);
-  ends_after_deps();
 }
 
 /* The stripe values of plane `p` (7.18.3.5, the horizontal half: the grain
@@ -2950,8 +2949,9 @@ cudaError_t launch_lr(const px_t* cdef, const px_t* curr, px_t* dst, const Layou
 }
 
 cudaError_t launch_grain_template(GrainState* gs, const int* gs_src, const GrainParamsDev& prm,
-                                  const uint16_t* orbit, const uint16_t* pos, bool early, cudaStream_t s) {
-  return launch_chained(early, k_grain_template, 1, 256, 0, s, gs, gs_src, prm, orbit, pos);
+                                  const uint16_t* orbit, const uint16_t* pos, cudaStream_t s) {
+  k_grain_template<<<1, 256, 0, s>>>(gs, gs_src, prm, orbit, pos);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_grain_blend(const px_t* src, px_t* dst, const Layout& L, const GrainState* gs,

@@ -176,8 +176,7 @@ cudaError_t launch_recon_stage(int stage, const FrameArgs& a, int n_sm, cudaStre
 /* `early` (here and below): the kernel starts as the one launched before it
  * drains, and waits for it to end before it reads anything. Only for a kernel
  * that follows one which waited itself, or was launched without: the kernels
- * before that one are then complete too. (The grain templates' kernel reads
- * nothing a kernel of the frame writes: it waits as it ends.) */
+ * before that one are then complete too. */
 cudaError_t launch_prep_filters(const av1b_deblock_edge* edges, int n_edges, const av1b_cdef_block* cdef,
                                 int n_cdef, const Layout& L, int grid_w, int grid_n, DeblockRec* v,
                                 DeblockRec* h, CdefRec* cdef_out, unsigned* cells, unsigned* extra,
@@ -216,7 +215,7 @@ cudaError_t launch_lr(const px_t* cdef, const px_t* curr, px_t* dst, const Layou
 /* gs_src: the frame's grain constants (GrainState from `lut` on), copied into
  * `gs` beside the templates; null: `gs` holds them. */
 cudaError_t launch_grain_template(GrainState* gs, const int* gs_src, const GrainParamsDev& prm,
-                                  const uint16_t* orbit, const uint16_t* pos, bool early, cudaStream_t s);
+                                  const uint16_t* orbit, const uint16_t* pos, cudaStream_t s);
 cudaError_t launch_grain_blend(const px_t* src, px_t* dst, const Layout& L, const GrainState* gs,
                                const uint16_t* orbit, const uint16_t* pos, cudaStream_t s);
 cudaError_t launch_nv12(const px_t* pic, uint8_t* out, const Layout& L, int pitch, cudaStream_t s);

@@ -302,7 +302,7 @@ extern "C" int av1b_apply_film_grain_noalloc(const av1b_frame_syntax* s, const u
     g.ar_cb[i] = f.ar_coeffs_cb[i];
     g.ar_cr[i] = f.ar_coeffs_cr[i];
   }
-  if (launch_grain_template(gs, nullptr, g, orbit, pos, false, st) != cudaSuccess) return AV1B_ERR_CUDA;
+  if (launch_grain_template(gs, nullptr, g, orbit, pos, st) != cudaSuccess) return AV1B_ERR_CUDA;
   const dim3 grid((a.w[0] + 127) / 128, a.h[0], 3);
   k_grain_blend_planes<<<grid, 128, 0, st>>>(a, gs, orbit, pos);
   return cudaGetLastError() == cudaSuccess ? AV1B_OK : AV1B_ERR_CUDA;

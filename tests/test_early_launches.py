@@ -38,7 +38,7 @@ def _function(src, name):
 
 def _early_kernels(src):
     names = set(re.findall(r'launch_chained\([^,;]*,\s*(k_\w+)', src))
-    assert names >= {'k_itx', 'k_inter_simple', 'k_grain_template', 'k_deblock', 'k_cdef_search', 'k_cdef_tile',
+    assert names >= {'k_itx', 'k_inter_simple', 'k_deblock', 'k_cdef_search', 'k_cdef_tile',
                      'k_upscale', 'k_lr_tile'}
     return sorted(names)
 
@@ -69,3 +69,16 @@ def test_early_kernels_read_plainly():
         fixed = set(re.findall(r'const\s+\w+\s*\*\s*__restrict__\s+(\w+)', params))
         assert fixed <= PLANNED, (name, fixed - PLANNED)
         assert '__ldg' not in body, name
+
+
+def test_grain_templates_run_beside_the_frame():
+    """The templates depend on the frame's parameters only: forked off before the
+    reconstruction, joined behind the filters."""
+    src = re.sub(r'/\*.*?\*/|//[^\n]*', '', open(os.path.join(CSRC, 'decoder.cu')).read(), flags=re.S)
+    body = _function(src, 'launch_step_plain')[1]
+    order = ['cudaEventRecord(d->ev_fork, st)', 'cudaStreamWaitEvent(d->aux, d->ev_fork', 'launch_grain_template(',
+             'cudaEventRecord(d->ev_join, d->aux)', 'launch_recon_stage(', 'launch_lr(',
+             'cudaStreamWaitEvent(st, d->ev_join', 'launch_grain_blend(']
+    at = [body.index(o) for o in order]
+    assert at == sorted(at)
+    assert re.search(r'launch_grain_template\([^;]*, d->aux\);', body)
