@@ -24,7 +24,8 @@ namespace av1b {
 
 #define AV1B_BATCH_MAX 64
 
-/* The stages of a batched step, in launch order. */
+/* The stages of a batched step, in launch order. (kBCopyPost is none any more:
+ * its place keeps the numbers of the launch configuration.) */
 enum BatchStage {
   kBInterSimple, kBInterLeanMask, kBInter, kBInterMask,
   kBItx2, kBItx3, kBItx4, kBItx5, kBItx6, kBItx7,
@@ -57,10 +58,10 @@ struct FilterArgs {
   const unsigned* cdef_extra;
   int* cdef_search;
   /* copies: the snapshot before CDEF, the one after it, the reference store */
-  const px_t* copy_src[3];
-  px_t* copy_dst[3];
-  long long copy_items[3];        /* AV1B_COPY_ITEM pieces (the bytes are a multiple of 16) */
-  long long copy_bytes[3];
+  const px_t* copy_src[2];        /* kBCopySnap, kBCopyRef */
+  px_t* copy_dst[2];
+  long long copy_items[2];        /* AV1B_COPY_ITEM pieces (the bytes are a multiple of 16) */
+  long long copy_bytes[2];
   /* superres: up to two passes (the rows loop restoration reads from the
    * pre-CDEF picture, then the picture) */
   const px_t* up_src[2];

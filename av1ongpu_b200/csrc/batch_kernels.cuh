@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(256) kb_deblock(const StreamStep* __restrict__
 /* A picture copy, AV1B_COPY_ITEM bytes a CTA item, 16 bytes a thread. */
 __global__ void __launch_bounds__(256) kb_copy(const StreamStep* __restrict__ st,
                                                const BatchHeader* __restrict__ h, int which) {
-  const int stage = which == 0 ? kBCopySnap : (which == 1 ? kBCopyPost : kBCopyRef);
+  const int stage = which == 0 ? kBCopySnap : kBCopyRef;
   const int* pfx = h->pfx[stage];
   const int n = h->n, total = pfx[n];
   int s = 0;
@@ -385,14 +385,13 @@ cudaError_t launch_batch_step(const StreamStep* steps, BatchHeader* hdr, const B
   kb_cdef_search<<<batch_grid(t, kBCdefSearch, n_sm), 128, 0, s>>>(steps, hdr);
   mark(kBCdef);
   kb_cdef<<<batch_grid(t, kBCdef, n_sm), 256, 0, s>>>(steps, hdr);
-  mark(kBCopyPost);
-  kb_copy<<<batch_grid(t, kBCopyPost, n_sm), 256, 0, s>>>(steps, hdr, 1);
+  mark(kBCopyPost);   /* nothing: the filters write out of place */
   mark(kBUpscale);
   kb_upscale<<<batch_grid(t, kBUpscale, n_sm), 128, 0, s>>>(steps, hdr);
   mark(kBLr);
   kb_lr<<<batch_grid(t, kBLr, n_sm), 256, 0, s>>>(steps, hdr);
   mark(kBCopyRef);
-  kb_copy<<<batch_grid(t, kBCopyRef, n_sm), 256, 0, s>>>(steps, hdr, 2);
+  kb_copy<<<batch_grid(t, kBCopyRef, n_sm), 256, 0, s>>>(steps, hdr, 1);
   if ((e = cudaStreamWaitEvent(s, join, 0)) != cudaSuccess) return e;
   mark(kBGrain);
   kb_grain_blend<<<batch_grid(t, kBGrain, n_sm), 128, 0, s>>>(steps, hdr);

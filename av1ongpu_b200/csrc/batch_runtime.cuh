@@ -92,7 +92,7 @@ int fill_filter_args(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
                           2 * ((L.p[1].out_w + AV1B_LR_TW - 1) / AV1B_LR_TW));
     f.lr_stripes = (L.p[0].out_h + 8 + 63) / 64;
   }
-  if (sp->store) set_copy(2, sp->out, static_cast<px_t*>(d->slot_buf[sp->slot].p));
+  if (sp->store) set_copy(1, sp->out, static_cast<px_t*>(d->slot_buf[sp->slot].p));
   d->disp_is_cur = true;
   d->disp_pending = false;
   if (P.grain) {
@@ -329,8 +329,7 @@ int batch_step(av1b_batch* b, int n, av1b_decoder* const* decs, av1b_plan* const
     items[kBDeblockV] = (f.n_dbv + AV1B_DB_GROUP - 1) / AV1B_DB_GROUP;
     items[kBDeblockH] = (f.n_dbh + AV1B_DB_GROUP - 1) / AV1B_DB_GROUP;
     items[kBCopySnap] = f.copy_items[0];
-    items[kBCopyPost] = f.copy_items[1];
-    items[kBCopyRef] = f.copy_items[2];
+    items[kBCopyRef] = f.copy_items[1];
     items[kBCdefSearch] = f.n_cdef > 0 ? (f.cdef_n_grid + f.n_cdef_extra + 127) / 128 : 0;
     items[kBCdef] = f.cdef_cells ? static_cast<long long>(f.cdef_tx) * f.cdef_ty * f.cdef_tz : (f.n_cdef + 15) / 16;
     items[kBUpscale] = f.up_items[0] + f.up_items[1];
@@ -717,7 +716,7 @@ int av1b_batch_autotune(av1b_batch* b, int n, av1b_decoder* const* decoders,
       {kBUnits},
       {kBDeblockV, kBDeblockH},
       {kBCdefSearch, kBCdef},
-      {kBCopySnap, kBCopyPost, kBCopyRef},
+      {kBCopySnap, kBCopyRef},
       {kBUpscale, kBLr},
       {kBGrainTemplate, kBGrain, kBNv12}};
   const int values[] = {1, 2, 4, 8, 16};

@@ -2638,12 +2638,10 @@ struct StepPrep {
 int fill_filter_args(av1b_decoder* d, av1b_plan* pl, StepPrep* sp);
 
 /* The host side of a frame step before anything is launched: the
- * destination slot, the buffers the frame needs, the done flags, claim
- * counter and status word (reset on the decoder's stream), the slot table,
- * and the arguments. In a batched step (`batched`) the film grain constants
- * are uploaded on the decoder's stream as well, and the filter chain's
- * arguments are filled for the batched kernels. Called with the decoder's
- * lock held. */
+ * destination slot, the buffers the frame needs, the done flags' epoch
+ * and the samples' tag (their buffers reset on the stream when they grow or
+ * wrap), the slot table, and the arguments; in a batched step (`batched`) the
+ * filter chain's as well. Called with the decoder's lock held. */
 int prepare_step(av1b_decoder* d, av1b_plan* pl, int keep, int forced_slot, bool batched,
                  StepPrep* sp, cudaStream_t st) {
   int rc;
@@ -2997,14 +2995,14 @@ int launch_step_plain(av1b_decoder* d, av1b_plan* pl, StepPrep* sp) {
   return AV1B_OK;
 }
 
-/* After the launches of a frame step: the read back into `out`, the status
- * word's copy, the stats, the plan's done event and the slot bookkeeping, on
+/* After the launches of a frame step: the read back into `out`, the stats,
+ * the plan's done event and the slot bookkeeping, on
  * the decoder's stream - which first waits for `after` when the step ran on
  * another stream (a batched step). Called with the decoder's lock held. */
 int commit_step(av1b_decoder* d, av1b_plan* pl, StepPrep* sp, const av1b_planes* out, int* out_slot,
                 bool sync, cudaStream_t batch_stream) {
   const Layout& L = d->L;
-  /* a batched step's status copy and plan event go on the batch's stream */
+  /* a batched step's plan event goes on the batch's stream */
   cudaStream_t st = batch_stream ? batch_stream : d->stream;
   const int keep = sp->keep, slot = sp->slot;
   const int launches = sp->launches;
@@ -3666,8 +3664,7 @@ int av1b_poll_status(av1b_decoder* d, int* status) {
   std::lock_guard<std::mutex> lk(d->mu);
   join_batch(d);
   cudaSetDevice(d->device);
-  /* the status word of the frames whose work has finished: its copy into
-   * page-locked memory is queued after each frame */
+  /* the status word, which a wait that gives up sets in page-locked memory */
   const cudaError_t q = cudaStreamQuery(d->stream);
   if (q != cudaSuccess && q != cudaErrorNotReady) return cuda_fail(d, q, "status poll");
   *status = *static_cast<volatile int*>(d->status_host);

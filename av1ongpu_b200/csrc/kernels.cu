@@ -966,10 +966,13 @@ __device__ __forceinline__ TagIo tag_io(const FrameArgs& a, const BlockRec& b, u
   return t;
 }
 
-/* INTER: the frame has phase B inter blocks (inter-intra, intra block copy);
- * a frame of intra blocks only (every key frame) runs the instantiation
- * without the inter prediction code, a much smaller kernel. */
-/* Runs chain `c` of the frame: its blocks one after another, each after the
+/* INTER: some frame of the launch has phase B inter blocks (inter-intra, intra
+ * block copy); a batched step of intra blocks only runs the instantiation
+ * without the inter prediction code. A single frame by chains has one build:
+ * a key frame takes as long with it as without that code (720p 1.86 ms, 1080p
+ * 2.55).
+ *
+ * Runs chain `c` of the frame: its blocks one after another, each after the
  * blocks it waits for. `edges` and `tmp` are the warp's shared memory. */
 template <bool INTER>
 __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges, int* tmp,

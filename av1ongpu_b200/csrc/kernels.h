@@ -50,8 +50,9 @@ namespace av1b {
 #define AV1B_CDEF_TW 64
 #define AV1B_CDEF_TH 32
 #define AV1B_UNIT_CTAS_PER_SM 2
-/* prediction: up to this many tiles an SM, unmasked and masked ones go in one
- * launch (16 warps an SM run at once) */
+/* prediction: up to this many tiles an SM, a warp each, unmasked and masked
+ * ones go in one launch: all its warps are resident at once (five CTAs of
+ * four) */
 #define AV1B_LEAN_ONE_LAUNCH 20
 /* the inverse transforms' one-launch kernel: CTAs of four warps an SM */
 #define AV1B_ITX_ALL_CTAS 3
