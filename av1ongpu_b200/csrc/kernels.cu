@@ -384,7 +384,6 @@ __global__ void __launch_bounds__(128, 5) k_inter_simple(const __grid_constant__
 __global__ void __launch_bounds__(128, 5) k_inter_lean(const __grid_constant__ FrameArgs a, int n_unmasked,
                                                        int end) {
   __shared__ McTileBuf buf[4][2];
-  deps_may_start();
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warp = blockIdx.x * 4 + wib;
   if (warp >= end) return;
@@ -718,7 +717,6 @@ __global__ void __launch_bounds__(128, kItxCtas[CLS]) k_itx(const __grid_constan
  * (1080p 65 -> 37 us, 4K 100 -> 64). */
 __global__ void __launch_bounds__(128, AV1B_ITX_ALL_CTAS) k_itx_all(const __grid_constant__ FrameArgs a, int n) {
   extern __shared__ int smem[];
-  deps_may_start();
   const int wib = threadIdx.x >> 5;
   const int bi = blockIdx.x * 4 + wib;
   const int lane = threadIdx.x & 31;
@@ -1102,7 +1100,6 @@ __device__ __forceinline__ void run_chain(const FrameArgs& a, int c, int* edges,
  * blocks off the cell grid, and traced ones. */
 __global__ void __launch_bounds__(128, AV1B_UNIT_CTAS_PER_SM) k_units(const __grid_constant__ FrameArgs a) {
   extern __shared__ int smem[];
-  deps_may_start();
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int* edges = smem + wib * (3 * AV1B_EDGE_LEN + AV1B_UNIT_SCRATCH);
@@ -1215,7 +1212,6 @@ __global__ void __launch_bounds__(32 * AV1B_REGION_WARPS, 1) k_regions(const __g
   const int n_samples = region_samples(a.L, a.region_log2);
   volatile unsigned short* tiles = reinterpret_cast<volatile unsigned short*>(&m + 1);
   int* items = reinterpret_cast<int*>(&m + 1) + n_samples / 2;
-  deps_may_start();
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* edges = m.warp[wib];
   int* tmp = edges + 3 * AV1B_EDGE_LEN;
